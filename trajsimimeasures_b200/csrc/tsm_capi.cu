@@ -11,6 +11,7 @@
 #include <string>
 
 #include "tsm.h"
+#include "tsm_haus.cuh"
 #include "tsm_kernels.h"
 #include "tsm_sched.cuh"
 #include "tsm_tile.cuh"
@@ -53,6 +54,15 @@ constexpr int kMaxLen = 32768;
 // non-empty pair runs one warp each on the wave kernels instead, with 4 rows
 // per lane unless rows_per_thread says otherwise.
 constexpr int kSmallBatchPerSm = 64;
+// Longest side of a pair in the two launches of the pruned Hausdorff pairs
+// kernel: 23 KB of shared memory per warp (eight warps per SM) and 181 KB (one).
+constexpr int kHausPrunedShort = 512;
+constexpr int kHausPrunedMax = 4096;
+static_assert(8 * tsm::haus_floats(kHausPrunedMax) <= 227 * 1024, "one staged pair fits a CTA");
+// Matrix launches of at most kHausThreadLen points on both sides and at least
+// kHausThreadPairs pairs (512 threads per SM) run one thread per pair.
+constexpr int kHausThreadLen = 64;
+constexpr int64_t kHausThreadPairs = 148 * 512;
 // Shared memory one CTA may use, leaving room for two CTAs per SM at cap 200.
 constexpr int kSmemPerCta = 113 * 1024;
 constexpr int kSmemMax = 227 * 1024;
@@ -155,23 +165,22 @@ int persistent_grid(const char* who, const void* fn, int threads, int smem, int6
     return TSM_OK;
 }
 
-// tsm_pairs' two kernels, which write disjoint outputs: `main` (the short
-// pairs, as a callable taking the stream) on the caller's stream and the
-// long-pair kernel on the calling thread's side stream, forked from and
-// joined back to the caller's; on the caller's stream one after the other
-// when there is no side stream.
-template <class Main>
-int launch_with_side(Main main, const void* wfn, dim3 w_grid, dim3 w_block, int w_smem, void** w_args,
-                     cudaStream_t s, int dev) {
+// tsm_pairs' short and long pairs, which write disjoint outputs: `main` (the
+// short pairs, as a callable taking the stream) on the caller's stream and
+// `longs` on the calling thread's side stream, forked from and joined back to
+// the caller's; on the caller's stream one after the other when there is no
+// side stream.
+template <class Main, class Longs>
+int launch_with_side(Main main, Longs longs, cudaStream_t s, int dev) {
     SideStream* side = side_stream(dev, s);
     if (!side) {
         const int rc = main(s);
-        return rc != TSM_OK ? rc : launch(wfn, w_grid, w_block, w_smem, w_args, s);
+        return rc != TSM_OK ? rc : longs(s);
     }
     cudaError_t e;
     if ((e = cudaEventRecord(side->fork, s)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
     if ((e = cudaStreamWaitEvent(side->st, side->fork, 0)) != cudaSuccess) return cuda_fail(e, "cudaStreamWaitEvent");
-    const int rc = launch(wfn, w_grid, w_block, w_smem, w_args, side->st);
+    const int rc = longs(side->st);
     const int rc_main = main(s);
     // join even after a failed launch, so that the side stream is not left forked from a capture
     if ((e = cudaEventRecord(side->join, side->st)) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
@@ -230,19 +239,39 @@ int tsm_pairs(int measure, const float* pts, const int64_t* off_a, const int32_t
         int64_t warp_cells = small ? 0 : tsm::kHausWarpCells;
         void* args[] = {&p2, &off_a, &len_a, &off_b, &len_b, &order, &n, &ml, &warp_cells, &out};
         if ((int64_t)max_len * max_len <= warp_cells) return launch(fn, grid, dim3(threads), 0, args, s);
-        // long pairs (small batch: every non-empty pair): one warp each, persistent
-        const void* wfn = tsm_k::haus_wave(R, exact);
-        dim3 w_grid;
-        int rc = persistent_grid("tsm_pairs", wfn, threads, 0, (n + 3) / 4, w_grid, dev);
-        if (rc != TSM_OK) return rc;
-        void* w_args[] = {&p2, &off_a, &len_a, &off_b, &len_b, &order, &n, &ml, &warp_cells, &out};
-        if (small) {  // the pairs kernel only flags bad lengths and empty pairs: one stream, in order
-            rc = launch(fn, grid, dim3(threads), 0, args, s);
-            return rc != TSM_OK ? rc : launch(wfn, w_grid, dim3(threads), 0, w_args, s);
-        }
-        // on the side stream, overlapping the one-thread-per-pair kernel
-        return launch_with_side([&](cudaStream_t st) { return launch(fn, grid, dim3(threads), 0, args, st); }, wfn,
-                                w_grid, dim3(threads), 0, w_args, s, dev);
+        // longer pairs (small batch: every non-empty pair), one warp each: pruned up to kHausPrunedShort points
+        // with many warps per SM, pruned up to kHausPrunedMax with the few that then fit, unpruned above
+        const void* pfn = tsm_k::haus_pruned_pairs(exact);
+        int lo[2] = {0, kHausPrunedShort};
+        int cap[2] = {max_len < kHausPrunedShort ? max_len : kHausPrunedShort,
+                      max_len < kHausPrunedMax ? max_len : kHausPrunedMax};
+        auto pruned = [&](int c, cudaStream_t st) {
+            const int pair_bytes = 8 * tsm::haus_floats(cap[c]);
+            int pw = 8;
+            while (pw > 1 && pw * pair_bytes > kSmemPerCta) pw >>= 1;
+            dim3 p_grid;
+            const int r = persistent_grid("tsm_pairs", pfn, 32 * pw, pw * pair_bytes, (n + pw - 1) / pw, p_grid, dev);
+            if (r != TSM_OK) return r;
+            void* p_args[] = {&p2, &off_a, &len_a, &off_b, &len_b, &order, &n, &lo[c], &cap[c], &warp_cells, &out};
+            return launch(pfn, p_grid, dim3(32 * pw), pw * pair_bytes, p_args, st);
+        };
+        auto main_side = [&](cudaStream_t st) {
+            const int r = launch(fn, grid, dim3(threads), 0, args, st);
+            return r != TSM_OK ? r : pruned(0, st);
+        };
+        auto long_side = [&](cudaStream_t st) {
+            const int r = pruned(1, st);
+            if (r != TSM_OK || max_len <= kHausPrunedMax) return r;
+            const void* wfn = tsm_k::haus_wave(R, exact);
+            dim3 w_grid;
+            const int r2 = persistent_grid("tsm_pairs", wfn, threads, 0, (n + 3) / 4, w_grid, dev);
+            if (r2 != TSM_OK) return r2;
+            void* w_args[] = {&p2, &off_a, &len_a, &off_b, &len_b, &order, &n, &ml, &cap[1], &warp_cells, &out};
+            return launch(wfn, w_grid, dim3(threads), 0, w_args, st);
+        };
+        if (max_len <= kHausPrunedShort) return main_side(s);
+        // the long pairs on the side stream, overlapping the shorter ones
+        return launch_with_side(main_side, long_side, s, dev);
     }
     const void* fn = tsm_k::dp_pairs(measure, R, exact);
     if (!fn) return fail(TSM_EINVAL, "tsm_pairs: rows_per_thread must be 4, 8 or 16");
@@ -275,7 +304,7 @@ int tsm_pairs(int measure, const float* pts, const int64_t* off_a, const int32_t
     // the wave kernel (few warps with long, uneven loops) on the side stream:
     // the tile kernel's blocks fill the SMs its warps leave idle
     return launch_with_side([&](cudaStream_t st) { return launch(fn, t_grid, dim3(32 * tW), t_smem, t_args, st); },
-                            wfn, w_grid, dim3(32 * W), w_smem, w_args, s, dev);
+                            [&](cudaStream_t st) { return launch(wfn, w_grid, dim3(32 * W), w_smem, w_args, st); }, s, dev);
 }
 
 namespace {
@@ -300,6 +329,30 @@ int matrix_launch(const char* who, int measure, const float* q_pts, const int64_
     if (measure == TSM_HAUSDORFF) {
         const void* fn = tsm_k::haus(true, R, exact);
         if (!fn) return fail(TSM_EINVAL, "%s: rows_per_thread must be 4, 8 or 16", who);
+        // One warp per pair with pruning, as many warps per CTA as fit (two CTAs per SM while they do), unless the
+        // trajectories are short and there are threads enough for a pair each.  Measured, 2000 x 2000 random walks,
+        // pruned / one thread per pair, ms: lengths 2..32 3.4 / 1.4, 2..64 4.7 / 4.2, 20..64 5.3 / 6.3, 2..96 5.7 /
+        // 8.7, 20..200 9.1 / 39.9; 1 x 2000 pairs of 20..200: 0.04 / 0.96.  (Points without any spatial order,
+        // where no box helps: 1000 x 1000 of 20..200 uniform random points 12.7 / 11.1.)
+        int dcap = d_max_len < 1 ? 1 : d_max_len;
+        const int64_t q_bytes = 4 * (int64_t)tsm::haus_floats(qcap), d_bytes = 4 * (int64_t)tsm::haus_floats(dcap);
+        int qb = sym == 2 ? 1 : 4, hw = 8;
+        while (hw > qb && qb * q_bytes + hw * d_bytes > kSmemPerCta) hw >>= 1;
+        if (qb * q_bytes + hw * d_bytes > kSmemPerCta) qb = 1;
+        while (hw > 1 && qb * q_bytes + hw * d_bytes > kSmemPerCta) hw >>= 1;
+        const bool by_thread = qcap <= kHausThreadLen && dcap <= kHausThreadLen && nq * nd >= kHausThreadPairs;
+        if (!by_thread && qb * q_bytes + hw * d_bytes <= kSmemPerCta) {
+            const int64_t qt = (nq + qb - 1) / qb;
+            int per_cta = 64;  // database slots per CTA: fewer when that leaves SMs without a few CTAs each
+            while (per_cta > hw && (nd + per_cta - 1) / per_cta * qt < 148 * 16) per_cta >>= 1;
+            const int64_t chunks64 = (nd + per_cta - 1) / per_cta;
+            if (chunks64 * qt > 0x7fffffffLL) return fail(TSM_EINVAL, "%s: grid too large", who);
+            int chunks = (int)chunks64;
+            void* args[] = {&q2,   &q_off, &q_len,  &q_order, &nq,  &d2,   &d_off, &d_len, &d_order,
+                            &ndd,  &dtot,  &chunks, &per_cta, &sym, &qcap, &dcap,  &out,   &ld};
+            return launch(tsm_k::haus_pruned_matrix(qb, exact), dim3((unsigned)(chunks * qt)), dim3(32 * hw),
+                          (int)(qb * q_bytes + hw * d_bytes), args, s);
+        }
         const int smem = ((qcap + 1) / 2) * 40;  // staged segment pairs
         if (smem > kSmemMax) return fail(TSM_ETOOLONG, "%s: query length %d too long", who, q_max_len);
         const int threads = 128;

@@ -1,5 +1,5 @@
 // Hausdorff kernels, both modes (table: tsm_kernels.h).
-#include "tsm_tile.cuh"
+#include "tsm_haus.cuh"
 #include "tsm_pick.cuh"
 
 namespace tsm_k {
@@ -30,5 +30,22 @@ const void* haus(bool matrix, int R, bool exact) {
 }
 
 const void* haus_wave(int R, bool exact) { return exact ? haus_wave_of<true>(R) : haus_wave_of<false>(R); }
+
+const void* haus_pruned_pairs(bool exact) {
+    return exact ? (const void*)&tsm::hausdorff_pruned_pairs_kernel<true>
+                 : (const void*)&tsm::hausdorff_pruned_pairs_kernel<false>;
+}
+
+const void* haus_pruned_matrix(int QB, bool exact) {
+    switch (QB) {
+        case 1:
+            return exact ? (const void*)&tsm::hausdorff_pruned_matrix_kernel<1, true>
+                         : (const void*)&tsm::hausdorff_pruned_matrix_kernel<1, false>;
+        case 4:
+            return exact ? (const void*)&tsm::hausdorff_pruned_matrix_kernel<4, true>
+                         : (const void*)&tsm::hausdorff_pruned_matrix_kernel<4, false>;
+        default: return nullptr;
+    }
+}
 
 }  // namespace tsm_k

@@ -16,6 +16,9 @@ const void* dp_wave(int measure, int R, bool exact);
 // hausdorff_matrix_kernel (matrix) or hausdorff_pairs_kernel, and hausdorff_wave_kernel <R, EXACT>
 const void* haus(bool matrix, int R, bool exact);
 const void* haus_wave(int R, bool exact);
+// hausdorff_pruned_matrix_kernel<QB, EXACT>, QB = 1 or 4, and hausdorff_pruned_pairs_kernel<EXACT>
+const void* haus_pruned_matrix(int QB, bool exact);
+const void* haus_pruned_pairs(bool exact);
 // dp_sched_kernel<R, EXACT>
 const void* sched(int R, bool exact);
 

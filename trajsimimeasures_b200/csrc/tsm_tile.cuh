@@ -1010,14 +1010,14 @@ __global__ void __launch_bounds__(128) hausdorff_matrix_kernel(
 }
 
 // Pairs mode: a pair with more than kHausWarpCells point products (na * nb)
-// runs one warp per pair (hausdorff_wave_kernel): on one thread, a pair of
-// two 2000-point trajectories is 8M evaluations and would hold a launch's
-// tail for tens of milliseconds.
-constexpr int64_t kHausWarpCells = 1 << 17;
+// runs one warp per pair (hausdorff_pruned_pairs_kernel, or above
+// kHausPrunedMax points hausdorff_wave_kernel): below that line one thread
+// per pair costs less than staging a pair (see matrix_launch for both sides).
+constexpr int64_t kHausWarpCells = 2048;
 
 // Pairs kernel: one thread per pair, both trajectories from global memory
 // (the pairs up to warp_cells point products -- kHausWarpCells, or 0 when a
-// small batch runs every non-empty pair on the warp kernel; it also flags
+// small batch runs every non-empty pair on the warp kernels; it also flags
 // bad lengths).
 template <int R, bool EXACT>
 __global__ void __launch_bounds__(128) hausdorff_pairs_kernel(
@@ -1040,8 +1040,8 @@ __global__ void __launch_bounds__(128) hausdorff_pairs_kernel(
     out[k] = __fsqrt_rn(fmaxf(m1, m2));
 }
 
-// Long pairs (more than warp_cells point products), one warp each.
-// Persistent, with the pair assignment of dp_wave_kernel (rounds of nw
+// Long pairs (more than warp_cells point products and a side of more than
+// min_side points), one warp each.  Persistent, with the pair assignment of dp_wave_kernel (rounds of nw
 // pairs in snake order, a ballot over 32 pairs at a time).  Lane l takes
 // point blocks l, l+32, ... of both directions; the lanes' maxima are
 // reduced with one warp max (exact), so the result is the one-thread
@@ -1050,7 +1050,7 @@ template <int R, bool EXACT>
 __global__ void __launch_bounds__(128) hausdorff_wave_kernel(
     const float2* __restrict__ pts, const int64_t* __restrict__ off_a, const int32_t* __restrict__ len_a,
     const int64_t* __restrict__ off_b, const int32_t* __restrict__ len_b, const int32_t* __restrict__ order,
-    int64_t n, int max_len, int64_t warp_cells, float* __restrict__ out) {
+    int64_t n, int max_len, int min_side, int64_t warp_cells, float* __restrict__ out) {
     const int lane = threadIdx.x & 31;
     const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -1062,7 +1062,8 @@ __global__ void __launch_bounds__(128) hausdorff_wave_kernel(
         if (t < n) {
             k = order ? (int64_t)order[t] : t;
             const int na = len_a[k], nb = len_b[k];
-            mine = na >= 0 && nb >= 0 && na <= max_len && nb <= max_len && (int64_t)na * nb > warp_cells;
+            mine = na >= 0 && nb >= 0 && na <= max_len && nb <= max_len && max(na, nb) > min_side &&
+                   (int64_t)na * nb > warp_cells;
         }
         unsigned todo = __ballot_sync(0xffffffffu, mine);
         while (todo) {
