@@ -6,11 +6,13 @@
 // and joined back to it).  No device allocation happens here.
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <string>
 
 #include "tsm.h"
+#include "tsm_bits.cuh"
 #include "tsm_haus.cuh"
 #include "tsm_kernels.h"
 #include "tsm_sched.cuh"
@@ -72,6 +74,8 @@ tsm::KParams make_kparams(const tsm_params* p) {
     const double eps = p ? p->eps : 0.0;
     const double gx = p ? p->gx : 0.0, gy = p ? p->gy : 0.0;
     k.eps2 = (float)(eps * eps);
+    k.epsr = sqrtf(k.eps2);
+    while (k.epsr * k.epsr < k.eps2) k.epsr = nextafterf(k.epsr, INFINITY);
     k.ghx = (float)gx;
     k.glx = (float)(gx - (double)k.ghx);
     k.ghy = (float)gy;
@@ -278,8 +282,9 @@ int tsm_pairs(int measure, const float* pts, const int64_t* off_a, const int32_t
     // small batch: tile capacity 0, so the tile kernel keeps only empty and
     // bad-length pairs and the wave kernel takes every other pair
     int cap = small ? 0 : (max_len < 1 ? 1 : (max_len < kTileCap ? max_len : kTileCap));
-    const int tW = warps_for(cap, 0);
-    const int t_smem = tW * 32 * cap * 4;
+    const bool bits = measure == TSM_EDR || measure == TSM_LCSS;
+    const int tW = bits ? 4 : warps_for(cap, 0);
+    const int t_smem = tW * 32 * (bits ? tsm::bits_words(cap) : cap) * 4;
     const dim3 t_grid((unsigned)((n + 32 * tW - 1) / (32 * tW)));
     void* t_args[] = {&p2, &off_a, &len_a, &off_b, &len_b, &order, &n, &cap, &ml, (void*)&kp, &out, &out_counts};
     // (a tile-heavy pair has a side longer than kHeavyRows >= kTileCap)
@@ -365,8 +370,21 @@ int matrix_launch(const char* who, int measure, const float* q_pts, const int64_
     }
     if (q_max_len > kMatrixQueryMax)
         return fail(TSM_ETOOLONG, "%s: q_max_len %d > %d (use the pairs form)", who, q_max_len, kMatrixQueryMax);
+    if (R != 4 && R != 8 && R != 16) return fail(TSM_EINVAL, "%s: rows_per_thread must be 4, 8 or 16", who);
+    if (measure == TSM_EDR || measure == TSM_LCSS) {
+        // queries per CTA: as many as share the database boxes within half an SM's shared memory, fewer when
+        // that leaves SMs without a few CTAs each
+        const int threads = tsm::kBitsThreads, carry_bytes = threads * tsm::bits_words(qcap) * 4;
+        int chunks = (int)((nd + threads - 1) / threads);
+        int qg = sym == 2 ? 1 : tsm::kBitsQueries;
+        while (qg > 1 && (qg * qcap * 8 + carry_bytes > kSmemPerCta || (nq + qg - 1) / qg * chunks < 148 * 8)) qg >>= 1;
+        const int64_t ctas = (nq + qg - 1) / qg * chunks;
+        if (ctas > 0x7fffffffLL) return fail(TSM_EINVAL, "%s: grid too large", who);
+        void* args[] = {&q2,   &q_off,  &q_len, &q_order, &nq,   &d2,  &d_off,      &d_len, &d_order, &ndd,
+                        &dtot, &chunks, &qg,    &sym,     &qcap, &dml, (void*)&kp, &out,   &ld,      &out_counts};
+        return launch(tsm_k::bits_matrix(measure), dim3((unsigned)ctas), dim3(threads), qg * qcap * 8 + carry_bytes, args, s);
+    }
     const void* fn = tsm_k::dp_matrix(measure, R, exact);
-    if (!fn) return fail(TSM_EINVAL, "%s: rows_per_thread must be 4, 8 or 16", who);
     const int W = warps_for(qcap, qcap * 16);
     const int threads = 32 * W;
     const int smem = qcap * 16 + W * 32 * qcap * 4;
@@ -374,8 +392,8 @@ int matrix_launch(const char* who, int measure, const float* q_pts, const int64_
     int chunks = (int)((nd + threads - 1) / threads);
     if ((int64_t)chunks * nq > 0x7fffffffLL) return fail(TSM_EINVAL, "%s: grid too large", who);
     dim3 grid((unsigned)(chunks * nq));
-    void* args[] = {&q2,     &q_off, &q_len, &q_order, &d2,        &d_off, &d_len, &d_order, &ndd,
-                    &dtot,   &chunks, &sym,  &qcap,    &dml,       (void*)&kp, &out, &ld,     &out_counts};
+    void* args[] = {&q2,   &q_off,  &q_len, &q_order, &d2,  &d_off,     &d_len, &d_order, &ndd,
+                    &dtot, &chunks, &sym,   &qcap,    &dml, (void*)&kp, &out,   &ld};
     return launch(fn, grid, dim3(threads), smem, args, s);
 }
 
@@ -499,7 +517,7 @@ int tsm_pairs_sched(const float* pts, const int64_t* off_a, const int32_t* len_a
     const void* fn = tsm_k::sched(R, exact);
     if (!fn) return fail(TSM_EINVAL, "tsm_pairs_sched: rows_per_thread must be 4 or 8");
     const int W = 4;
-    const int smem = W * warp_smem_floats * 4;
+    const int smem = W * tsm::sched_warp_floats(warp_smem_floats) * 4;
     if (smem > kSmemMax) return fail(TSM_ETOOLONG, "tsm_pairs_sched: %d bytes of shared memory per CTA", smem);
     cudaError_t e = set_smem(fn, smem);
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");

@@ -7,7 +7,11 @@ namespace tsm_k {
 
 const void* dp_matrix(int measure, int R, bool exact) {
     if (!exact) return dp_matrix_fast(measure, R);
-    TSM_DP_TABLE(tsm::dp_matrix_kernel, true, measure, R)
+    TSM_DP_MATRIX_TABLE(tsm::dp_matrix_kernel, true, measure, R)
+}
+
+const void* bits_matrix(int measure) {
+    return measure == TSM_EDR ? (const void*)&tsm::bits_matrix_kernel<tsm::EDR> : (const void*)&tsm::bits_matrix_kernel<tsm::LCSS>;
 }
 
 }  // namespace tsm_k

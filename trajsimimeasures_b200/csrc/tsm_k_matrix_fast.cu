@@ -6,7 +6,7 @@
 namespace tsm_k {
 
 const void* dp_matrix_fast(int measure, int R) {
-    TSM_DP_TABLE(tsm::dp_matrix_kernel, false, measure, R)
+    TSM_DP_MATRIX_TABLE(tsm::dp_matrix_kernel, false, measure, R)
 }
 
 }  // namespace tsm_k

@@ -10,9 +10,12 @@
 namespace tsm_k {
 
 // dp_pairs_kernel / dp_matrix_kernel / dp_wave_kernel<M, R, EXACT>, M = TSM_DTW .. TSM_DFRECHET
+// (dp_matrix: not EDR and LCSS)
 const void* dp_pairs(int measure, int R, bool exact);
 const void* dp_matrix(int measure, int R, bool exact);
 const void* dp_wave(int measure, int R, bool exact);
+// bits_matrix_kernel<M>, M = TSM_EDR or TSM_LCSS
+const void* bits_matrix(int measure);
 // hausdorff_matrix_kernel (matrix) or hausdorff_pairs_kernel, and hausdorff_wave_kernel <R, EXACT>
 const void* haus(bool matrix, int R, bool exact);
 const void* haus_wave(int R, bool exact);

@@ -19,3 +19,12 @@
         case TSM_DFRECHET: return TSM_BY_R(KER, tsm::DFRECHET, E, R);              \
         default: return nullptr;                                                   \
     }
+
+// the instantiation of KER<measure, R, E> for the measures whose matrix form is dp_matrix_kernel
+#define TSM_DP_MATRIX_TABLE(KER, E, measure, R)                                    \
+    switch (measure) {                                                             \
+        case TSM_DTW: return TSM_BY_R(KER, tsm::DTW, E, R);                        \
+        case TSM_ERP: return TSM_BY_R(KER, tsm::ERP, E, R);                        \
+        case TSM_DFRECHET: return TSM_BY_R(KER, tsm::DFRECHET, E, R);              \
+        default: return nullptr;                                                   \
+    }

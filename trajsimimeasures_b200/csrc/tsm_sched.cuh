@@ -56,6 +56,10 @@ struct PairsArgs {
     int64_t out_stride;  // out[measure * out_stride + pair]
 };
 
+// Shared memory per warp, in floats: the caller's, but two words per lane at
+// least (bits_words of one column).
+__host__ __device__ constexpr int sched_warp_floats(int warp_floats) { return warp_floats < 64 ? 64 : warp_floats; }
+
 // Group tasks stage their column points in shared memory when they fit.
 constexpr bool kGroupStageCols = true;
 
@@ -239,17 +243,36 @@ __device__ __forceinline__ void group_task(const PairsArgs& A, int first, int co
     __syncwarp();
 }
 
-// One pair per lane (the tile kernel's per-thread DP).
+// One pair per lane (the tile kernel's per-thread DP; EDR and LCSS: 32 rows
+// per word, tsm_bits.cuh, whose carries need fewer words than a boundary row).
 template <int M, int R, bool EXACT>
 __device__ __forceinline__ void tile_task(const PairsArgs& A, int first, int count, float* wsm, int cap) {
     const int lane = threadIdx.x & 31;
+    if constexpr (M == EDR || M == LCSS) {
+        const int64_t k = lane < count ? (int64_t)A.order[first + lane] : 0;
+        int na = -1, nb = -1;
+        bool bad = false;
+        if (lane < count) {
+            na = A.len_a[k];
+            nb = A.len_b[k];
+            bad = na < 0 || nb < 0 || na > A.max_len || nb > A.max_len || min(na, nb) > cap;
+        }
+        const bool mine = lane < count && !bad;
+        int c = lane_count<M>(mine ? A.pts + A.off_a[k] : A.pts, mine ? na : -1, mine ? A.pts + A.off_b[k] : A.pts,
+                              mine ? nb : -1, reinterpret_cast<uint32_t*>(wsm) + lane, A.p, lane);
+        if (bad) c = -1;
+        if (lane < count) {
+            A.out[M * A.out_stride + k] = bad ? CUDART_NAN_F : count_value<M>(c, na, nb);
+            if (A.counts) A.counts[M * A.out_stride + k] = c;
+        }
+        __syncwarp();
+        return;
+    }
     if (lane < count) {
         const int64_t k = A.order[first + lane];
         const int na = A.len_a[k], nb = A.len_b[k];
-        const bool cnt = (M == EDR || M == LCSS) && A.counts;
         if (na < 0 || nb < 0 || na > A.max_len || nb > A.max_len || min(na, nb) > cap) {
             A.out[M * A.out_stride + k] = CUDART_NAN_F;
-            if (cnt) A.counts[M * A.out_stride + k] = -1;
         } else {
             const bool a_rows = na >= nb;
             const float2* rowp = A.pts + (a_rows ? A.off_a[k] : A.off_b[k]);
@@ -265,7 +288,6 @@ __device__ __forceinline__ void tile_task(const PairsArgs& A, int first, int cou
             int c;
             finalize<M>(dl, na, nb, o, c);
             A.out[M * A.out_stride + k] = o;
-            if (cnt) A.counts[M * A.out_stride + k] = c;
         }
     }
     __syncwarp();
@@ -345,14 +367,14 @@ __device__ __forceinline__ void run_task(const int4 task, const PairsArgs& A, fl
 }
 
 // Persistent kernel.  grid = resident CTAs; block = 32*W; dynamic shared
-// memory = W * warp_floats floats.  queue: int[2] in global memory, zero
+// memory = W * sched_warp_floats(warp_floats) floats.  queue: int[2] in global memory, zero
 // before the first launch (self-resetting afterwards).
 template <int R, bool EXACT>
 __global__ void __launch_bounds__(128) dp_sched_kernel(PairsArgs A, const int4* __restrict__ tasks, int n_tasks,
                                                        int* __restrict__ queue, int total_warps, int warp_floats) {
     extern __shared__ float smem[];
     const int lane = threadIdx.x & 31;
-    float* wsm = smem + (threadIdx.x >> 5) * warp_floats;
+    float* wsm = smem + (threadIdx.x >> 5) * sched_warp_floats(warp_floats);
     for (;;) {
         int t = 0;
         if (lane == 0) t = atomicAdd(queue, 1);

@@ -24,6 +24,7 @@
 
 #include <type_traits>
 
+#include "tsm_bits.cuh"
 #include "tsm_device.cuh"
 
 namespace tsm {
@@ -109,29 +110,6 @@ struct RowBlock {
         return up;
     }
 
-    // The local terms of the R cells at column point c (C::term: the square
-    // root of the squared distance, or the match value), for step2t.
-    __device__ __forceinline__ void terms(const float4& c, float (&T)[R], float eps2) const {
-#pragma unroll
-        for (int r = 0; r < R; ++r) T[r] = C::term(d2nr<PACKED>(n[r], make_float2(c.x, c.y)), eps2);
-    }
-
-    // step2 with the local terms computed beforehand (by terms(), a step
-    // ahead): the same cells in the same order, so the same values.
-    __device__ __forceinline__ float step2t(const float (&Din)[R], float (&Dout)[R], const float (&T)[R], float gcol,
-                                            float top, float diag) const {
-        float up = top, dg = diag;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const float left = Din[r];
-            const float nv = C::comb(dg, up, left, T[r], g[r], gcol);
-            Dout[r] = nv;
-            dg = left;
-            up = nv;
-        }
-        return up;
-    }
-
     __device__ __forceinline__ float pick(int rr) const {
         float v = 0.f;
 #pragma unroll
@@ -147,116 +125,6 @@ template <class C, class Cols>
 constexpr bool kPacked() {
     return std::is_same<Cols, SmemCols>::value ? C::kPackedSmem : true;
 }
-
-// Lower-block-first form of the two-block pass (used by dp_pair for EDR and
-// LCSS with shared-memory columns, where it was measured 3-5 % faster; the
-// sqrt measures lose with it, since their first cells then wait on the
-// column load).  At step j the column point and top value of column j are
-// loaded first, the lower block computes column j-1 from operands already in
-// registers while the load is in flight, then the upper block computes column
-// j.  Every carried value then rotates through two registers only, which
-// the two-column unrolled loop renames away.
-template <int M, int R, bool EXACT, class Cols>
-__device__ __forceinline__ float dp_pair_lower_first(const float2* __restrict__ rowp, int nr, const Cols& cols,
-                                                     int nc, float* buf, const KParams& p, float srow, float scol) {
-    using C = typename CellOf<M, EXACT>::type;
-    for (int j = 0; j < nc; ++j) buf[32 * j] = C::topb(scol, j);
-    float dlast = 0.f;
-    int rb = 0;
-    for (; nr - rb > R; rb += 2 * R) {
-        RowBlock<C, R, EXACT, kPacked<C, Cols>()> hi, lo;
-        hi.load(rowp, rb, nr, srow, p);
-        lo.load(rowp, rb + R, nr, srow, p);
-        float HA[R], HB[R], LA[R], LB[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            HA[r] = hi.D[r];
-            LA[r] = lo.D[r];
-        }
-        float4 cp = col4<EXACT>(cols, 0, p, C::kGap);  // the lower block's column
-        float udiag = buf[0];                          // the upper block's diagonal
-        float hb1 = hi.step2(HA, HB, cp, udiag, (rb == 0) ? C::corner() : C::rowb(srow, rb - 1), p.eps2);
-        float hb2 = C::rowb(srow, rb + R - 1);  // upper block's bottom values at columns j-1, j-2
-        auto st = [&](const float (&Hi)[R], float (&Ho)[R], const float (&Li)[R], float (&Lo)[R], int j) {
-            const float4 cj = col4<EXACT>(cols, j, p, C::kGap);
-            const float tj = buf[32 * j];
-            buf[32 * (j - 1)] = lo.step2(Li, Lo, cp, hb1, hb2, p.eps2);
-            const float nb = hi.step2(Hi, Ho, cj, tj, udiag, p.eps2);
-            hb2 = hb1;
-            hb1 = nb;
-            udiag = tj;
-            cp = cj;
-        };
-        int j = 1;
-        for (; j + 1 < nc; j += 2) {
-            st(HB, HA, LA, LB, j);
-            st(HA, HB, LB, LA, j + 1);
-        }
-        float lb;
-        const int rr = nr - 1 - (rb + R);
-        if (j < nc) {
-            st(HB, HA, LA, LB, j);
-            lb = lo.step2(LB, LA, cp, hb1, hb2, p.eps2);
-            if (rb + 2 * R >= nr) {
-#pragma unroll
-                for (int r = 0; r < R; ++r)
-                    if (r == rr) dlast = LA[r];
-            }
-        } else {
-            lb = lo.step2(LA, LB, cp, hb1, hb2, p.eps2);
-            if (rb + 2 * R >= nr) {
-#pragma unroll
-                for (int r = 0; r < R; ++r)
-                    if (r == rr) dlast = LB[r];
-            }
-        }
-        buf[32 * (nc - 1)] = lb;
-    }
-    if (rb < nr) {  // last rows (at most R): one block, ping-pong over column pairs
-        RowBlock<C, R, EXACT, kPacked<C, Cols>()> blk;
-        blk.load(rowp, rb, nr, srow, p);
-        float DA[R], DB[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) DA[r] = blk.D[r];
-        float diag = (rb == 0) ? C::corner() : C::rowb(srow, rb - 1);
-        int j = 0;
-        for (; j + 1 < nc; j += 2) {
-            const float4 c0 = col4<EXACT>(cols, j, p, C::kGap);
-            const float t0 = buf[32 * j];
-            const float4 c1 = col4<EXACT>(cols, j + 1, p, C::kGap);
-            const float t1 = buf[32 * (j + 1)];
-            blk.step2(DA, DB, c0, t0, diag, p.eps2);
-            blk.step2(DB, DA, c1, t1, t0, p.eps2);
-            diag = t1;
-        }
-        const int rr = nr - 1 - rb;
-        if (j < nc) {
-            const float4 c0 = col4<EXACT>(cols, j, p, C::kGap);
-            blk.step2(DA, DB, c0, buf[32 * j], diag, p.eps2);
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                if (r == rr) dlast = DB[r];
-        } else {
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                if (r == rr) dlast = DA[r];
-        }
-    }
-    return dlast;
-}
-
-template <int M, class Cols>
-struct LowerFirst {
-    static constexpr bool value = false;
-};
-template <>
-struct LowerFirst<EDR, SmemCols> {
-    static constexpr bool value = true;
-};
-template <>
-struct LowerFirst<LCSS, SmemCols> {
-    static constexpr bool value = true;
-};
 
 // The DP of one pair, prefetching form (dp_pair's default).  rowp/nr: row
 // trajectory; cols/nc: column trajectory; buf: this thread's boundary row
@@ -363,130 +231,6 @@ __device__ __forceinline__ float dp_pair_prefetch(const float2* __restrict__ row
             diag = top;
         }
         dlast = blk.pick(nr - 1 - rb);
-    }
-    return dlast;
-}
-
-// The prefetching two-block pass with each cell's local term (C::term: for
-// DTW and ERP the MUFU square root of the squared distance) computed one
-// column step before the recurrence needs it.  At step j the upper block
-// computes column j and the lower block column j - 1 from terms made at step
-// j - 1; then the terms of step j + 1 are made: the lower block's at column j
-// (point already in registers), the upper block's at column j + 1 (point
-// loaded at the start of step j).  A cell's recurrence then no longer waits
-// on its own square root.  Term arrays alternate between two per block like
-// the value arrays.  The cells and their order along each dependency chain
-// are those of dp_pair_prefetch, so the values are identical.
-template <int M, int R, bool EXACT, class Cols>
-__device__ __forceinline__ float dp_pair_ahead(const float2* __restrict__ rowp, int nr, const Cols& cols, int nc,
-                                               float* buf, const KParams& p, float srow, float scol) {
-    using C = typename CellOf<M, EXACT>::type;
-    constexpr bool PK = kPacked<C, Cols>();
-    const float e2 = p.eps2;
-    for (int j = 0; j < nc; ++j) buf[32 * j] = C::topb(scol, j);
-    float dlast = 0.f;
-    int rb = 0;
-    for (; nr - rb > R; rb += 2 * R) {
-        RowBlock<C, R, EXACT, PK> hi, lo;
-        hi.load(rowp, rb, nr, srow, p);
-        lo.load(rowp, rb + R, nr, srow, p);
-        float HA[R], HB[R], LA[R], LB[R], THA[R], THB[R], TLA[R], TLB[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            HA[r] = hi.D[r];
-            LA[r] = lo.D[r];
-        }
-        float4 c = col4<EXACT>(cols, 0, p, C::kGap);
-        float top = buf[0];
-        const int j1 = min(1, nc - 1);
-        float4 cn = col4<EXACT>(cols, j1, p, C::kGap);
-        float tn = buf[32 * j1];
-        // step 0: the upper block's column 0; then the terms of step 1
-        hi.terms(c, THA, e2);
-        float ub1 = hi.step2t(HA, HB, THA, c.z, top, (rb == 0) ? C::corner() : C::rowb(srow, rb - 1));
-        lo.terms(c, TLA, e2);
-        hi.terms(cn, THA, e2);
-        float ub2 = C::rowb(srow, rb + R - 1), udiag = top, gprev = c.z;
-        // steps 1 .. nc-1: upper column j, lower column j-1, then the next step's terms
-        auto pair_step = [&](const float (&Hi)[R], float (&Ho)[R], const float (&Li)[R], float (&Lo)[R],
-                             const float (&THi)[R], float (&THo)[R], const float (&TLi)[R], float (&TLo)[R],
-                             int j) {
-            c = cn;
-            top = tn;
-            const int jn = min(j + 1, nc - 1);
-            cn = col4<EXACT>(cols, jn, p, C::kGap);
-            tn = buf[32 * jn];
-            const float nb = hi.step2t(Hi, Ho, THi, c.z, top, udiag);
-            const float lb = lo.step2t(Li, Lo, TLi, gprev, ub1, ub2);
-            buf[32 * (j - 1)] = lb;
-            lo.terms(c, TLo, e2);
-            hi.terms(cn, THo, e2);
-            udiag = top;
-            ub2 = ub1;
-            ub1 = nb;
-            gprev = c.z;
-        };
-        int j = 1;
-        for (; j + 1 < nc; j += 2) {
-            pair_step(HB, HA, LA, LB, THA, THB, TLA, TLB, j);
-            pair_step(HA, HB, LB, LA, THB, THA, TLB, TLA, j + 1);
-        }
-        float lb;
-        const int rr = nr - 1 - (rb + R);
-        if (j < nc) {
-            pair_step(HB, HA, LA, LB, THA, THB, TLA, TLB, j);
-            lb = lo.step2t(LB, LA, TLB, gprev, ub1, ub2);
-            if (rb + 2 * R >= nr) {
-#pragma unroll
-                for (int r = 0; r < R; ++r)
-                    if (r == rr) dlast = LA[r];
-            }
-        } else {
-            lb = lo.step2t(LA, LB, TLA, gprev, ub1, ub2);
-            if (rb + 2 * R >= nr) {
-#pragma unroll
-                for (int r = 0; r < R; ++r)
-                    if (r == rr) dlast = LB[r];
-            }
-        }
-        buf[32 * (nc - 1)] = lb;
-    }
-    if (rb < nr) {  // last rows (at most R): one block, its terms a step ahead too
-        RowBlock<C, R, EXACT, PK> blk;
-        blk.load(rowp, rb, nr, srow, p);
-        float DA[R], DB[R], TA[R], TB[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) DA[r] = blk.D[r];
-        float diag = (rb == 0) ? C::corner() : C::rowb(srow, rb - 1);
-        float4 c = col4<EXACT>(cols, 0, p, C::kGap);
-        float top = buf[0];
-        blk.terms(c, TA, e2);
-        auto st = [&](const float (&Di)[R], float (&Do)[R], const float (&Ti)[R], float (&To)[R], int j) {
-            const int jn = min(j + 1, nc - 1);
-            const float4 cn = col4<EXACT>(cols, jn, p, C::kGap);
-            const float tn = buf[32 * jn];
-            blk.step2t(Di, Do, Ti, c.z, top, diag);
-            blk.terms(cn, To, e2);
-            diag = top;
-            top = tn;
-            c = cn;
-        };
-        int j = 0;
-        for (; j + 1 < nc; j += 2) {
-            st(DA, DB, TA, TB, j);
-            st(DB, DA, TB, TA, j + 1);
-        }
-        const int rr = nr - 1 - rb;
-        if (j < nc) {
-            st(DA, DB, TA, TB, j);
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                if (r == rr) dlast = DB[r];
-        } else {
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                if (r == rr) dlast = DA[r];
-        }
     }
     return dlast;
 }
@@ -634,38 +378,28 @@ __device__ __forceinline__ float dp_pair_quad(const float2* __restrict__ rowp, i
     return dp_pair_prefetch<M, R, EXACT>(rowp, nr, cols, nc, buf, p, srow, scol, rb);
 }
 
-// The DP of one pair, with shared-memory columns (the matrix kernels): the
-// terms-ahead pass for EDR (kAheadMask), the lower-block-first pass for LCSS,
-// the four-block pass for ERP (kQuadPass), else the prefetching one; with
-// per-lane global columns (paired and scheduled kernels) the prefetching one.
-// Measured on B200, all-pairs 2000 x 2000: ERP 18.84 -> 18.05 ms with four
-// blocks of 8 rows; DTW 15.29 -> 15.69 ms (four blocks of 8) and 16.17 ms (of
-// 4), so DTW keeps two blocks.  The four-block pass stays out of the scheduled
-// kernel: compiled into its ERP tile tasks it raised the whole kernel from 127
-// to 190 registers, and the 500k-pair uneven batch from 5.1 to 6.5 ms.
+// The DP of one pair (DTW, ERP, discrete Frechet): with shared-memory columns
+// (the matrix kernels) the four-block pass for ERP (kQuadPass), else the
+// prefetching one.  Measured on B200, all-pairs 2000 x 2000: ERP 18.84 ->
+// 18.05 ms with four blocks of 8 rows; DTW 15.29 -> 15.69 ms (four blocks of
+// 8) and 16.17 ms (of 4), so DTW keeps two blocks.  The four-block pass stays
+// out of the scheduled kernel: compiled into its ERP tile tasks it raised the
+// whole kernel from 127 to 190 registers, and the 500k-pair uneven batch from
+// 5.1 to 6.5 ms.  Also measured slower, bit-identical: the square roots one
+// column ahead of the recurrence (DTW 15.17 -> 16.02, ERP 18.05 -> 19.84,
+// Frechet 12.33 -> 12.94), the lower block first (DTW and ERP 25-30 %), and
+// the squared distances of two rows packed in f32x2 (DTW 15.2 -> 19.0, ERP
+// 18.1 -> 20.5, Frechet 12.35 -> 15.6: an f32x2 instruction holds the pipe and
+// the issue port as long as two scalar ones).
 #ifndef TSM_QUAD_PASS
 #define TSM_QUAD_PASS 1
 #endif
 constexpr bool kQuadPass = TSM_QUAD_PASS != 0;
-// Measures (bit M) whose matrix kernels run dp_pair_ahead.  Measured on B200,
-// all-pairs 2000 x 2000, every measure bit-identical to its default pass:
-// EDR 14.79 -> 13.91 ms (its match terms a step ahead beat the lower-first
-// pass); slower for the others: DTW 15.17 -> 16.02, LCSS 12.49 -> 12.87, ERP
-// 18.05 -> 19.84 (against the four-block pass), Frechet 12.33 -> 12.94 ms,
-// and slower still with blocks of 16 rows.
-#ifndef TSM_AHEAD_MASK
-#define TSM_AHEAD_MASK (1 << EDR)
-#endif
-constexpr int kAheadMask = TSM_AHEAD_MASK;
 template <int M, int R, bool EXACT, class Cols>
 __device__ __forceinline__ float dp_pair(const float2* __restrict__ rowp, int nr, const Cols& cols,
                                          int nc, float* buf, const KParams& p, float srow, float scol) {
     if (nr <= 0 || nc <= 0) return 0.f;
-    if constexpr (kAheadMask & (1 << M) && std::is_same<Cols, SmemCols>::value) {
-        return dp_pair_ahead<M, R, EXACT>(rowp, nr, cols, nc, buf, p, srow, scol);
-    } else if constexpr (LowerFirst<M, Cols>::value) {
-        return dp_pair_lower_first<M, R, EXACT>(rowp, nr, cols, nc, buf, p, srow, scol);
-    } else if constexpr (kQuadPass && M == ERP && R <= 8 && std::is_same<Cols, SmemCols>::value) {
+    if constexpr (kQuadPass && M == ERP && R <= 8 && std::is_same<Cols, SmemCols>::value) {
         // (16 rows: four blocks spill)
         return dp_pair_quad<M, R, EXACT>(rowp, nr, cols, nc, buf, p, srow, scol);
     } else {
@@ -673,25 +407,61 @@ __device__ __forceinline__ float dp_pair(const float2* __restrict__ rowp, int nr
     }
 }
 
+// The EDR or LCSS count of one pair per lane (na, nb < 0: none), the whole
+// warp together; a count of 0 for an empty trajectory.
+template <int M>
+__device__ __forceinline__ int lane_count(const float2* a, int na, const float2* b, int nb, uint32_t* carry,
+                                          const KParams& p, int lane) {
+    const bool a_rows = na >= nb;
+    const float2* rowp = a_rows ? a : b;
+    const float2* colp = a_rows ? b : a;
+    const int nr = a_rows ? na : nb, nc = a_rows ? nb : na;
+    // the columns' boxes cost the warp about 1,400 instructions: for sweeps much longer than that (26 a word and
+    // column) only.  200,000 pairs of 2..32 points without this line 0.062 ms, with it 0.043
+    const int sweep = __reduce_max_sync(0xffffffffu, nc > 0 ? (nr + 31) / 32 * nc : 0);
+    const float4 all = make_float4(-CUDART_INF_F, CUDART_INF_F, -CUDART_INF_F, CUDART_INF_F);
+    const float4 cbox = sweep > 128 ? lane_boxes(colp, nc, lane) : all;
+    return nc > 0 ? bits_count<M>(rowp, nr, GlobalCols{colp}, nc, carry, p.eps2, p.epsr, cbox) : 0;
+}
 
 // Pairs mode ------------------------------------------------------------------
 
-// Block = 32*W threads, dynamic shared memory = W*32*cap floats.
+// Block = 32*W threads, dynamic shared memory = W*32*cap floats (EDR, LCSS:
+// W*32*bits_words(cap) words, tsm_bits.cuh).
 template <int M, int R, bool EXACT>
 __global__ void __launch_bounds__(128) dp_pairs_kernel(
     const float2* __restrict__ pts, const int64_t* __restrict__ off_a, const int32_t* __restrict__ len_a,
     const int64_t* __restrict__ off_b, const int32_t* __restrict__ len_b, const int32_t* __restrict__ order,
     int64_t n, int cap, int max_len, KParams p, float* __restrict__ out, int32_t* __restrict__ counts) {
     extern __shared__ float smem[];
-    float* buf = smem + (threadIdx.x >> 5) * (32 * cap) + (threadIdx.x & 31);
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if constexpr (M == EDR || M == LCSS) {
+        const int lane = threadIdx.x & 31;
+        uint32_t* carry = reinterpret_cast<uint32_t*>(smem) + (threadIdx.x >> 5) * 32 * bits_words(cap) + lane;
+        const int64_t k = t < n ? (order ? (int64_t)order[t] : t) : 0;
+        int na = -1, nb = -1;
+        bool bad = false;
+        if (t < n) {
+            na = len_a[k];
+            nb = len_b[k];
+            bad = na < 0 || nb < 0 || na > max_len || nb > max_len;
+        }
+        // (the wave kernel's pairs are left to it)
+        const bool mine = t < n && !bad && min(na, nb) <= cap && !tile_heavy<R>(max(na, nb), min(na, nb));
+        int c = lane_count<M>(mine ? pts + off_a[k] : pts, mine ? na : -1, mine ? pts + off_b[k] : pts, mine ? nb : -1,
+                              carry, p, lane);
+        if (bad) c = -1;
+        if (!mine && !bad) return;
+        out[k] = bad ? CUDART_NAN_F : count_value<M>(c, na, nb);
+        if (counts) counts[k] = c;
+        return;
+    }
+    float* buf = smem + (threadIdx.x >> 5) * (32 * cap) + (threadIdx.x & 31);
     if (t >= n) return;
     const int64_t k = order ? (int64_t)order[t] : t;
     const int na = len_a[k], nb = len_b[k];
-    const bool count = (M == EDR || M == LCSS) && counts != nullptr;
     if (na < 0 || nb < 0 || na > max_len || nb > max_len) {
         out[k] = CUDART_NAN_F;
-        if (count) counts[k] = -1;
         return;
     }
     const float2* a = pts + off_a[k];
@@ -711,7 +481,6 @@ __global__ void __launch_bounds__(128) dp_pairs_kernel(
     int c;
     finalize<M>(dl, na, nb, o, c);
     out[k] = o;
-    if (count) counts[k] = c;
 }
 
 // Matrix mode -----------------------------------------------------------------
@@ -723,8 +492,8 @@ __global__ void __launch_bounds__(128) dp_pairs_kernel(
 // out[i, j] and out[j, i]; CTAs wholly below the diagonal exit at once.
 // Gather mode (sym == 2): d_order holds one row of nd database indices per
 // query i (row i, whatever the processing order q_order), and slot t of query i
-// goes to out[i, t].  A database index outside
-// 0..d_total-1 gives NaN (count -1).
+// goes to out[i, t].  A database index outside 0..d_total-1 gives NaN.
+// (EDR and LCSS: bits_matrix_kernel, tsm_bits.cuh.)
 // Dynamic shared memory = cap float4 columns + W*32*cap floats.
 
 template <int M, int R, bool EXACT>
@@ -732,7 +501,7 @@ __global__ void __launch_bounds__(128) dp_matrix_kernel(
     const float2* __restrict__ q_pts, const int64_t* __restrict__ q_off, const int32_t* __restrict__ q_len,
     const int32_t* __restrict__ q_order, const float2* __restrict__ d_pts, const int64_t* __restrict__ d_off,
     const int32_t* __restrict__ d_len, const int32_t* __restrict__ d_order, int64_t nd, int64_t d_total, int chunks,
-    int sym, int cap, int d_max_len, KParams p, float* __restrict__ out, int64_t ld, int32_t* __restrict__ counts) {
+    int sym, int cap, int d_max_len, KParams p, float* __restrict__ out, int64_t ld) {
     extern __shared__ float smem[];
     __shared__ float s_scol;
     float4* cols = reinterpret_cast<float4*>(smem);
@@ -764,16 +533,11 @@ __global__ void __launch_bounds__(128) dp_matrix_kernel(
     const int64_t dj = d_order ? (int64_t)d_order[(sym == 2 ? qi * nd : 0) + slot] : slot;
     const bool dbad = dj < 0 || dj >= d_total;
     const int ndl = dbad ? -1 : d_len[dj];
-    const bool count = (M == EDR || M == LCSS) && counts != nullptr;
     const int64_t o_idx = qi * ld + (sym == 2 ? slot : dj), t_idx = dj * ld + qi;
     const bool mirror = sym == 1 && dj != qi;
     if (qbad || dbad || ndl < 0 || ndl > d_max_len) {
         out[o_idx] = CUDART_NAN_F;
-        if (count) counts[o_idx] = -1;
-        if (mirror) {
-            out[t_idx] = CUDART_NAN_F;
-            if (count) counts[t_idx] = -1;
-        }
+        if (mirror) out[t_idx] = CUDART_NAN_F;
         return;
     }
     const float2* dp = d_pts + d_off[dj];
@@ -787,11 +551,7 @@ __global__ void __launch_bounds__(128) dp_matrix_kernel(
     int c;
     finalize<M>(dl, nq, ndl, o, c);
     out[o_idx] = o;
-    if (count) counts[o_idx] = c;
-    if (mirror) {
-        out[t_idx] = o;
-        if (count) counts[t_idx] = c;
-    }
+    if (mirror) out[t_idx] = o;
 }
 
 // Hausdorff -------------------------------------------------------------------
