@@ -17,25 +17,18 @@
 // The reference trains its learned measures the same way (MSE on
 // distance / max distance, nn/MLP_trajsimi_train.py:74-84,197-200).
 //
-// Training recurrences (hand-written, SIMT FP32 FMA): 16 trajectories per CTA,
-// the BF16 weights resident in shared memory for all time steps, time stepped
-// inside the kernel, FP32 activations, and the caches BPTT needs.  The weight
-// gradients of the GRU (reductions over every valid step of the batch) run on
-// the tensor cores (tsm_wgrad.cu, BF16 hi/lo split products).  Inference
-// (embedding a database or a query batch) runs on the tensor cores instead:
-// enc_gru_embed_tc takes 128 trajectories per CTA, so each step's products
-// (128 x 384 x 192) are tcgen05 MMA tiles with the accumulators in tensor
-// memory.
+// Training runs on the tensor cores with FP32-accurate activations (three BF16
+// parts, tsm_train.cu; weight gradients tsm_wgrad.cu).  Inference (embedding a
+// database or a query batch) takes a_t and h_t as BF16: enc_gru_embed_tc, 128
+// trajectories per CTA, each step's products (128 x 384 x 192) tcgen05 MMA
+// tiles with the accumulators in tensor memory.
 //
 //   enc_round_bf16    FP32 master -> BF16 weights
-//   enc_conv_fwd      conv + relu -> A [B][T][64]
-//   enc_gru_fwd       persistent GRU over T steps -> H [B][T+1][128] and gate caches
+//   train_forward     conv + GRU over time, with the values BPTT needs (tsm_train.cu)
 //   enc_head_fwd      e = [Wo h_last + bo | sc_k r_k]
 //   enc_pair_loss     distances, MSE loss, dL/de (atomic)
 //   enc_head_bwd      dWo, dbo, dh_last; enc_skip_bwd: d sc_k
-//   enc_gru_bwd       BPTT: gate gradients G [B][T][384] (input side), dA [B][T][64], bias gradients
-//   tsm_wgrad_tc      weight gradients dW_ih, dW_hh on the tensor cores (tsm_wgrad.cu)
-//   enc_conv_bwd      dW1, db1
+//   train_backward    BPTT, GRU and conv gradients (tsm_train.cu, tsm_wgrad.cu)
 //   enc_adam          Adam step on the FP32 master weights
 //   enc_conv_fwd_tc   conv + relu -> BF16 a_t operand images for the tensor-core GRU
 //   enc_gru_embed_tc  inference GRU on the tensor cores -> last hidden state
@@ -45,228 +38,20 @@
 #include <stdint.h>
 
 #include "tsm.h"
+#include "tsm_enc.cuh"
+#include "tsm_train.h"
 #include "tsm_umma.cuh"
-#include "tsm_wgrad.h"
 
 int tsm_internal_fail(int code, const char* msg);
 
 namespace enc {
 
-constexpr int C1 = 64;    // conv channels
-constexpr int KW = 5;     // conv width
-constexpr int HD = 128;   // hidden
-constexpr int G3 = 384;   // 3 gates
-constexpr int EO = 128;   // learned head outputs
-constexpr int NS = 16;    // resampled points of the geometric skip
-constexpr int SK = 2 * NS;  // skip features (x, y of each resampled point)
-constexpr int ED = EO + SK; // embedding: [head outputs | skip weights * resampled points]
 static_assert(SK == 32, "enc_skip_bwd maps one skip value per lane");
-constexpr int S = 16;     // trajectories per GRU CTA
-constexpr int GRU_THREADS = 384;
-constexpr int SP = S + 4;  // row stride of the backward's trajectory-minor gate gradients (16-byte groups of 4)
-constexpr int SPA = S + 4; // row stride of the forward's trajectory-minor h and a_t
-
-// parameter offsets in the flat FP32 master buffer
-constexpr int OFF_W1 = 0;                    // [64][2][5]
-constexpr int OFF_B1 = OFF_W1 + C1 * 2 * KW; // [64]
-constexpr int OFF_WIH = OFF_B1 + C1;         // [384][64]
-constexpr int OFF_BIH = OFF_WIH + G3 * C1;   // [384]
-constexpr int OFF_WHH = OFF_BIH + G3;        // [384][128]
-constexpr int OFF_BHH = OFF_WHH + G3 * HD;   // [384]
-constexpr int OFF_WO = OFF_BHH + G3;         // [128][128]
-constexpr int OFF_BO = OFF_WO + EO * HD;     // [128]
-constexpr int OFF_SC = OFF_BO + EO;          // [16] u_k: log-weights of the resampled points of the skip
-constexpr int N_PARAMS = OFF_SC + NS;
-
-__device__ __forceinline__ float sigm(float x) { return 1.f / (1.f + expf(-x)); }
 
 // FP32 master -> BF16 copies of the conv and GRU weights (head stays FP32).
 __global__ void enc_round_bf16(const float* __restrict__ p, __nv_bfloat16* __restrict__ q) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < OFF_WO) q[i] = __float2bfloat16_rn(p[i]);
-}
-
-// Normalised input coordinate i of point t of trajectory b (0 outside).
-__device__ __forceinline__ float xin(const float2* pts, int64_t off, int len, int t, int i, float4 nrm) {
-    if (t < 0 || t >= len) return 0.f;
-    const float2 v = pts[off + t];
-    return i == 0 ? (v.x - nrm.x) * nrm.z : (v.y - nrm.y) * nrm.w;
-}
-
-// A[b][t][c] = relu(conv), 0 for t >= len.  One thread per (b, t, c).
-__global__ void enc_conv_fwd(const float2* __restrict__ pts, const int64_t* __restrict__ off,
-                             const int32_t* __restrict__ len, int B, int T, float4 nrm,
-                             const __nv_bfloat16* __restrict__ wq, const float* __restrict__ p,
-                             float* __restrict__ A) {
-    const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= (int64_t)B * T * C1) return;
-    const int c = gid % C1;
-    const int t = (gid / C1) % T;
-    const int b = gid / ((int64_t)C1 * T);
-    const int n = len[b];
-    float a = 0.f;
-    if (t < n) {
-        float acc = p[OFF_B1 + c];
-#pragma unroll
-        for (int k = 0; k < KW; ++k)
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-                acc = fmaf(__bfloat162float(wq[OFF_W1 + (c * 2 + i) * KW + k]), xin(pts, off[b], n, t + k - 2, i, nrm), acc);
-        a = fmaxf(acc, 0.f);
-    }
-    A[gid] = a;
-}
-
-// Persistent GRU forward.  CTA = S trajectories, 384 threads (thread j: gate
-// rows j % 192 and j % 192 + 192 of trajectories 8 (j / 192) .. +7).  Shared
-// memory: Wih and Whh BF16, transposed into (k, k+1) pairs per gate row
-// ([k/2][384][2]: a thread reads one 4-byte pair per row, consecutive threads
-// consecutive words), h [S][128], a [S][64], gate pre-activations gi, gh
-// [S][384].
-// Caches for the backward pass (only steps t < len are written):
-//   H [B][T+1][128] (H[b][0] = 0), R, Z, N, GHN [B][T][128] with
-//   GHN = Whn h + bhn.  hl [B][128] = h after the last valid step.
-__global__ void __launch_bounds__(GRU_THREADS, 1) enc_gru_fwd(
-    const float* __restrict__ A, const int32_t* __restrict__ len, int B, int T, const __nv_bfloat16* __restrict__ wq,
-    const float* __restrict__ p, float* __restrict__ H, float* __restrict__ R, float* __restrict__ Z,
-    float* __restrict__ N, float* __restrict__ GHN, float* __restrict__ hl) {
-    extern __shared__ __align__(16) unsigned char smraw[];
-    __nv_bfloat16* wih = reinterpret_cast<__nv_bfloat16*>(smraw);        // [32][384][2]: (k, k+1) pairs per gate row
-    __nv_bfloat16* whh = wih + C1 * G3;                                   // [64][384][2]
-    float* hs = reinterpret_cast<float*>(whh + HD * G3);                  // [128][SPA]: h, trajectory-minor
-    float* as = hs + HD * SPA;                                            // [64][SPA]: a_t, trajectory-minor
-    float* gi = as + C1 * SPA;                                            // [S][384]
-    float* gh = gi + S * G3;                                              // [S][384]
-    __shared__ int lens[S];
-    const int j = threadIdx.x;
-    const int b0 = blockIdx.x * S;
-    for (int e = j; e < G3 * C1; e += GRU_THREADS) {  // transpose into k-pair-major [k/2][row][k%2]
-        const int row = e / C1, col = e % C1;
-        wih[((col >> 1) * G3 + row) * 2 + (col & 1)] = wq[OFF_WIH + e];
-    }
-    for (int e = j; e < G3 * HD; e += GRU_THREADS) {
-        const int row = e / HD, col = e % HD;
-        whh[((col >> 1) * G3 + row) * 2 + (col & 1)] = wq[OFF_WHH + e];
-    }
-    for (int e = j; e < HD * SPA; e += GRU_THREADS) hs[e] = 0.f;
-    if (j < S) lens[j] = (b0 + j < B) ? len[b0 + j] : 0;
-    // the products: thread j takes gate rows jr and jr + 192 for trajectories
-    // 8 sh .. 8 sh + 7 as four (s, s + 1) pairs, FP32x2 FMAs of one weight
-    // against two trajectories' activations: a 4-byte load of two weights
-    // feeds 16 FMAs, a broadcast 16-byte load of four activations 8
-    constexpr int SH = S / 2;
-    const int jr = j % (G3 / 2), sh = j / (G3 / 2);
-    const float bih0 = p[OFF_BIH + jr], bhh0 = p[OFF_BHH + jr];
-    const float bih1 = p[OFF_BIH + jr + G3 / 2], bhh1 = p[OFF_BHH + jr + G3 / 2];
-    const uint32_t* wih2 = reinterpret_cast<const uint32_t*>(wih);
-    const uint32_t* whh2 = reinterpret_cast<const uint32_t*>(whh);
-    __syncthreads();
-    int tmax = 0;
-    for (int s = 0; s < S; ++s) tmax = max(tmax, lens[s]);
-    // H[b][0] = 0, and rows past the trajectory's length are zero too (the
-    // weight-gradient reduction multiplies every row by a gate gradient, 0
-    // past the length; the rows must hold numbers, not stale memory)
-    for (int s = 0; s < S; ++s) {
-        if (b0 + s >= B) break;
-        float* hb = H + (int64_t)(b0 + s) * (T + 1) * HD;
-        for (int e = j; e < HD; e += GRU_THREADS) hb[e] = 0.f;
-        for (int64_t e = (int64_t)(lens[s] + 1) * HD + j; e < (int64_t)(T + 1) * HD; e += GRU_THREADS) hb[e] = 0.f;
-    }
-    // this thread's elements e = j + 384 i of a_t, loaded a step ahead (the
-    // loads of step t + 1 are in flight during step t's products)
-    constexpr int AN = (S * C1 + GRU_THREADS - 1) / GRU_THREADS;
-    float an[AN];
-    auto load_a = [&](int t) {
-#pragma unroll
-        for (int i = 0; i < AN; ++i) {
-            const int e = j + GRU_THREADS * i;
-            const int s = e / C1;
-            an[i] = (e < S * C1 && b0 + s < B && t < lens[s]) ? A[((int64_t)(b0 + s) * T + t) * C1 + e % C1] : 0.f;
-        }
-    };
-    // the two BF16 weights of a pair as floats (low half: even k)
-    auto lo = [](uint32_t u) { return __uint_as_float(u << 16); };
-    auto hi = [](uint32_t u) { return __uint_as_float(u & 0xffff0000u); };
-    if (tmax > 0) load_a(0);
-    for (int t = 0; t < tmax; ++t) {
-#pragma unroll
-        for (int i = 0; i < AN; ++i) {
-            const int e = j + GRU_THREADS * i;  // element (s, c) = (e / 64, e % 64)
-            if (e < S * C1) as[(e % C1) * SPA + e / C1] = an[i];
-        }
-        __syncthreads();
-        if (t + 1 < tmax) load_a(t + 1);
-        // accumulator pairs (trajectories 8 sh + 2 q, 8 sh + 2 q + 1) of rows jr and jr + 192
-        float2 ai0[SH / 2], ai1[SH / 2], ah0[SH / 2], ah1[SH / 2];
-#pragma unroll
-        for (int q = 0; q < SH / 2; ++q) {
-            ai0[q] = make_float2(bih0, bih0);
-            ai1[q] = make_float2(bih1, bih1);
-            ah0[q] = make_float2(bhh0, bhh0);
-            ah1[q] = make_float2(bhh1, bhh1);
-        }
-        // k + 3, k + 2, k + 1, k within each group of four: the order of a
-        // nested fmaf(w_k, v_k, fmaf(w_k+1, v_k+1, ...)) dot product
-        auto prods = [&](const uint32_t* w2, const float* v, int K, float2 (&acc0)[SH / 2], float2 (&acc1)[SH / 2]) {
-            for (int k = 0; k < K; k += 4) {
-                const uint32_t p01 = w2[(k / 2) * G3 + jr], p23 = w2[(k / 2 + 1) * G3 + jr];
-                const uint32_t q01 = w2[(k / 2) * G3 + jr + G3 / 2], q23 = w2[(k / 2 + 1) * G3 + jr + G3 / 2];
-                const float wr0[4] = {lo(p01), hi(p01), lo(p23), hi(p23)};
-                const float wr1[4] = {lo(q01), hi(q01), lo(q23), hi(q23)};
-#pragma unroll
-                for (int kk = 3; kk >= 0; --kk) {
-                    const float4 va = *reinterpret_cast<const float4*>(v + (k + kk) * SPA + SH * sh);
-                    const float4 vb = *reinterpret_cast<const float4*>(v + (k + kk) * SPA + SH * sh + 4);
-                    const float2 vv[4] = {make_float2(va.x, va.y), make_float2(va.z, va.w),
-                                          make_float2(vb.x, vb.y), make_float2(vb.z, vb.w)};
-                    const float2 w0 = make_float2(wr0[kk], wr0[kk]), w1 = make_float2(wr1[kk], wr1[kk]);
-#pragma unroll
-                    for (int q = 0; q < SH / 2; ++q) {
-                        acc0[q] = __ffma2_rn(w0, vv[q], acc0[q]);
-                        acc1[q] = __ffma2_rn(w1, vv[q], acc1[q]);
-                    }
-                }
-            }
-        };
-        prods(wih2, as, C1, ai0, ai1);
-        prods(whh2, hs, HD, ah0, ah1);
-#pragma unroll
-        for (int q = 0; q < SH / 2; ++q) {
-            const int s = SH * sh + 2 * q;
-            gi[s * G3 + jr] = ai0[q].x;
-            gi[(s + 1) * G3 + jr] = ai0[q].y;
-            gi[s * G3 + jr + G3 / 2] = ai1[q].x;
-            gi[(s + 1) * G3 + jr + G3 / 2] = ai1[q].y;
-            gh[s * G3 + jr] = ah0[q].x;
-            gh[(s + 1) * G3 + jr] = ah0[q].y;
-            gh[s * G3 + jr + G3 / 2] = ah1[q].x;
-            gh[(s + 1) * G3 + jr + G3 / 2] = ah1[q].y;
-        }
-        __syncthreads();
-        for (int e = j; e < S * HD; e += GRU_THREADS) {
-            const int s = e / HD, k = e % HD;
-            if (b0 + s < B && t < lens[s]) {
-                const float r = sigm(gi[s * G3 + k] + gh[s * G3 + k]);
-                const float z = sigm(gi[s * G3 + HD + k] + gh[s * G3 + HD + k]);
-                const float ghn = gh[s * G3 + 2 * HD + k];
-                const float n = tanhf(gi[s * G3 + 2 * HD + k] + r * ghn);
-                const float hp = hs[k * SPA + s];
-                const float hn = (1.f - z) * n + z * hp;
-                const int64_t o = ((int64_t)(b0 + s) * T + t) * HD + k;
-                R[o] = r;
-                Z[o] = z;
-                N[o] = n;
-                GHN[o] = ghn;
-                H[((int64_t)(b0 + s) * (T + 1) + t + 1) * HD + k] = hn;
-                hs[k * SPA + s] = hn;
-            }
-        }
-        __syncthreads();
-    }
-    for (int e = j; e < S * HD; e += GRU_THREADS) {
-        const int s = e / HD;
-        if (b0 + s < B) hl[(int64_t)(b0 + s) * HD + e % HD] = hs[(e % HD) * SPA + s];
-    }
 }
 
 // Point index of resampled point k (0 <= k < NS) of a trajectory of n >= 1
@@ -360,18 +145,23 @@ __global__ void enc_pair_loss(const float* __restrict__ E, const int32_t* __rest
 
 // dWo[o][k] += sum_b dE[b][o] hl[b][k]; dbo[o] += sum_b dE[b][o];
 // dhl[b][k] = sum_o Wo[o][k] dE[b][o].
+// (One CTA per output and HB_B trajectories, added with atomics: with one CTA
+// per output the sum over a batch was a chain of 2,048 dependent loads, 0.21 ms.)
+constexpr int HB_B = 128;
 __global__ void enc_head_bwd_w(const float* __restrict__ dE, const float* __restrict__ hl, int B,
                                float* __restrict__ grad) {
     const int o = blockIdx.x;  // EO blocks
     const int k = threadIdx.x; // 128 threads
     float acc = 0.f, accb = 0.f;
-    for (int b = 0; b < B; ++b) {
+    const int b1 = min(B, ((int)blockIdx.y + 1) * HB_B);
+#pragma unroll 8
+    for (int b = blockIdx.y * HB_B; b < b1; ++b) {
         const float g = dE[(int64_t)b * ED + o];
         acc = fmaf(g, hl[(int64_t)b * HD + k], acc);
         accb += g;
     }
-    grad[OFF_WO + o * HD + k] += acc;
-    if (k == 0) grad[OFF_BO + o] += accb;
+    atomicAdd(grad + OFF_WO + o * HD + k, acc);
+    if (k == 0) atomicAdd(grad + OFF_BO + o, accb);
 }
 
 __global__ void enc_head_bwd_h(const float* __restrict__ dE, int B, const float* __restrict__ p, float* __restrict__ dhl) {
@@ -397,205 +187,6 @@ __global__ void enc_skip_bwd(const float* __restrict__ dE, const float* __restri
     for (int64_t b = wid; b < B; b += nw) acc = fmaf(dE[b * ED + EO + q], X[b * SK + q], acc);
     acc += __shfl_xor_sync(0xffffffffu, acc, 1);
     if ((q & 1) == 0) atomicAdd(grad + OFF_SC + (q >> 1), expf(p[OFF_SC + (q >> 1)]) * acc);
-}
-
-// BPTT.  CTA = S trajectories, 384 threads.  Shared memory: Whh [384][128]
-// and Wih [384][64] BF16 (row-major: thread k reads column k of row j),
-// dh [S][128], dgi/dgh [S][384].  Writes, for every step t < len:
-//   G  [B][T][384]  input-side gate gradients (d pre-activation of r, z, n)
-//   GH [B][T][384]  hidden-side (r, z as G; n multiplied by r)
-//   dA [B][T][64]   gradient of the conv output
-// and zeros for steps t >= len.
-__global__ void __launch_bounds__(GRU_THREADS, 1) enc_gru_bwd(
-    const float* __restrict__ dhl, const int32_t* __restrict__ len, int B, int T, const __nv_bfloat16* __restrict__ wq,
-    const float* __restrict__ H, const float* __restrict__ R, const float* __restrict__ Z, const float* __restrict__ N,
-    const float* __restrict__ GHN, float* __restrict__ G, float* __restrict__ GH, float* __restrict__ dA,
-    float* __restrict__ gbih, float* __restrict__ gbhh) {
-    extern __shared__ __align__(16) unsigned char smraw[];
-    __nv_bfloat16* whh = reinterpret_cast<__nv_bfloat16*>(smraw);  // [384][128]
-    __nv_bfloat16* wih = whh + G3 * HD;                             // [384][64]
-    float* dh = reinterpret_cast<float*>(wih + G3 * C1);            // [S][128]
-    float* dhd = dh + S * HD;                                       // [S][128] direct part (dh * z)
-    float* dgi = dhd + S * HD;                                      // [384][SP] gate gradients, trajectory-minor
-    float* dgh = dgi + G3 * SP;                                     // [384][SP]
-    __shared__ int lens[S];
-    const int tid = threadIdx.x;
-    const int b0 = blockIdx.x * S;
-    for (int e = tid; e < G3 * HD; e += GRU_THREADS) whh[e] = wq[OFF_WHH + e];
-    for (int e = tid; e < G3 * C1; e += GRU_THREADS) wih[e] = wq[OFF_WIH + e];
-    if (tid < S) lens[tid] = (b0 + tid < B) ? len[b0 + tid] : 0;
-    for (int e = tid; e < S * HD; e += GRU_THREADS) {
-        const int s = e / HD;
-        dh[e] = (b0 + s < B) ? dhl[(int64_t)(b0 + s) * HD + e % HD] : 0.f;
-    }
-    __syncthreads();
-    // zero the caches of steps beyond each length
-    for (int s = 0; s < S; ++s) {
-        if (b0 + s >= B) break;
-        const int n0 = lens[s];
-        for (int64_t e = (int64_t)n0 * G3 + tid; e < (int64_t)T * G3; e += GRU_THREADS) {
-            G[(int64_t)(b0 + s) * T * G3 + e] = 0.f;
-            GH[(int64_t)(b0 + s) * T * G3 + e] = 0.f;
-        }
-        for (int64_t e = (int64_t)n0 * C1 + tid; e < (int64_t)T * C1; e += GRU_THREADS)
-            dA[(int64_t)(b0 + s) * T * C1 + e] = 0.f;
-    }
-    int tmax = 0;
-    for (int s = 0; s < S; ++s) tmax = max(tmax, lens[s]);
-    // The output products: threads 0..255 take 2 consecutive hidden units
-    // (dh) of four trajectories, threads 256..383 2 consecutive channels (dA)
-    // of four trajectories; per gate row jj one 4-byte load of 2 BF16 weights
-    // and one 16-byte load of the four trajectories' gate gradients feed 8
-    // FMAs.  Each sum runs over jj in order from the same start as a dot
-    // product per output would, so the values are those of one thread per output.
-    float sbi = 0.f, sbh = 0.f;  // this CTA's bias gradients of gate row tid (phase 2 maps e % 384 = tid)
-    const bool dh_part = tid < 256;
-    const int og = dh_part ? (tid & 63) : ((tid - 256) & 31);  // output pair: units / channels 2 og, 2 og + 1
-    const int s0 = 4 * (dh_part ? (tid >> 6) : ((tid - 256) >> 5));  // trajectories s0 .. s0 + 3
-    // this thread's cache values (elements e = tid + 384 i of step t), loaded
-    // a step ahead: the loads of step t - 1 are in flight during step t's products
-    constexpr int EN = (S * HD + GRU_THREADS - 1) / GRU_THREADS;
-    float cr[EN], cz[EN], cn[EN], cg[EN], ch[EN];
-    auto load_c = [&](int t) {
-#pragma unroll
-        for (int i = 0; i < EN; ++i) {
-            const int e = tid + GRU_THREADS * i;
-            const int s = e / HD, k = e % HD;
-            if (e < S * HD && b0 + s < B && t < lens[s]) {
-                const int64_t o = ((int64_t)(b0 + s) * T + t) * HD + k;
-                cr[i] = R[o];
-                cz[i] = Z[o];
-                cn[i] = N[o];
-                cg[i] = GHN[o];
-                ch[i] = H[((int64_t)(b0 + s) * (T + 1) + t) * HD + k];
-            }
-        }
-    };
-    if (tmax > 0) load_c(tmax - 1);
-    for (int t = tmax - 1; t >= 0; --t) {
-#pragma unroll
-        for (int i = 0; i < EN; ++i) {
-            const int e = tid + GRU_THREADS * i;
-            if (e >= S * HD) break;
-            const int s = e / HD, k = e % HD;
-            float gr = 0.f, gz = 0.f, gn = 0.f, gnh = 0.f, d = 0.f;
-            if (b0 + s < B && t < lens[s]) {
-                const float r = cr[i], z = cz[i], n = cn[i], ghn = cg[i];
-                const float hp = ch[i];
-                const float g = dh[e];
-                const float dn = g * (1.f - z);
-                const float dz = g * (hp - n);
-                d = g * z;
-                gn = dn * (1.f - n * n);
-                gr = gn * ghn * r * (1.f - r);
-                gz = dz * z * (1.f - z);
-                gnh = gn * r;
-            } else {
-                d = dh[e];  // frozen step: dh passes through unchanged
-            }
-            dgi[k * SP + s] = gr;
-            dgi[(HD + k) * SP + s] = gz;
-            dgi[(2 * HD + k) * SP + s] = gn;
-            dgh[k * SP + s] = gr;
-            dgh[(HD + k) * SP + s] = gz;
-            dgh[(2 * HD + k) * SP + s] = gnh;
-            dhd[e] = d;
-        }
-        __syncthreads();
-        if (t > 0) load_c(t - 1);
-        // gate gradients to global memory; thread tid always holds gate row
-        // jj = tid here, so it also sums that row's bias gradients
-        for (int e = tid; e < S * G3; e += GRU_THREADS) {
-            const int s = e / G3, jj = e % G3;
-            if (b0 + s < B && t < lens[s]) {
-                const int64_t o = ((int64_t)(b0 + s) * T + t) * G3 + jj;
-                const float vi = dgi[jj * SP + s], vh = dgh[jj * SP + s];
-                G[o] = vi;
-                GH[o] = vh;
-                sbi += vi;
-                sbh += vh;
-            }
-        }
-        // outputs: 128 dh values and 64 dA values per trajectory, each a dot
-        // product over the 384 gate gradients
-        bool act[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) act[q] = b0 + s0 + q < B && t < lens[s0 + q];
-        if (act[0] || act[1] || act[2] || act[3]) {
-            const __nv_bfloat16* w = dh_part ? whh + 2 * og : wih + 2 * og;
-            const int wstride = dh_part ? HD : C1;
-            const float* dg = (dh_part ? dgh : dgi) + s0;
-            float a[4][2];
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-#pragma unroll
-                for (int i = 0; i < 2; ++i) a[q][i] = dh_part ? dhd[(s0 + q) * HD + 2 * og + i] : 0.f;
-#pragma unroll 4
-            for (int jj = 0; jj < G3; ++jj) {
-                const uint32_t wv = *reinterpret_cast<const uint32_t*>(w + jj * wstride);
-                const float4 g4 = *reinterpret_cast<const float4*>(dg + jj * SP);
-                const float w0 = __uint_as_float(wv << 16), w1 = __uint_as_float(wv & 0xffff0000u);
-                const float gq[4] = {g4.x, g4.y, g4.z, g4.w};
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    a[q][0] = fmaf(w0, gq[q], a[q][0]);
-                    a[q][1] = fmaf(w1, gq[q], a[q][1]);
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                if (!act[q]) continue;
-                if (dh_part) {
-                    dhd[(s0 + q) * HD + 2 * og] = a[q][0];
-                    dhd[(s0 + q) * HD + 2 * og + 1] = a[q][1];
-                } else {
-                    *reinterpret_cast<float2*>(dA + ((int64_t)(b0 + s0 + q) * T + t) * C1 + 2 * og) =
-                        make_float2(a[q][0], a[q][1]);
-                }
-            }
-        }
-        __syncthreads();
-        for (int e = tid; e < S * HD; e += GRU_THREADS) dh[e] = dhd[e];
-        __syncthreads();
-    }
-    atomicAdd(gbih + tid, sbi);
-    atomicAdd(gbhh + tid, sbh);
-}
-
-// Conv weight gradients.  One CTA per trajectory, 704 threads: thread q
-// takes weight (c, i, k) = (q / 10, (q / 5) % 2, q % 5) of the 640, or the
-// bias of channel q - 640, summed over the trajectory's steps (one atomic per
-// thread and trajectory).  The normalised input points are staged in shared
-// memory, CBW_T steps (plus the window's two on either side) at a time.
-constexpr int CBW_THREADS = C1 * 2 * KW + C1;  // 704
-constexpr int CBW_T = 256;
-__global__ void __launch_bounds__(CBW_THREADS) enc_conv_bwd(const float2* __restrict__ pts,
-                                                           const int64_t* __restrict__ off,
-                                                           const int32_t* __restrict__ len, int T, float4 nrm,
-                                                           const float* __restrict__ A, const float* __restrict__ dA,
-                                                           float* __restrict__ grad) {
-    __shared__ float xs[CBW_T + KW - 1][2];  // xs[u][i] = input i at step t0 + u - 2
-    const int b = blockIdx.x;
-    const int n = len[b];
-    if (n <= 0) return;  // uniform per CTA
-    const int q = threadIdx.x;
-    const bool wt = q < C1 * 2 * KW;
-    const int c = wt ? q / (2 * KW) : q - C1 * 2 * KW, i = (q / KW) % 2, k = q % KW;
-    const int64_t o0 = off[b];
-    float acc = 0.f;
-    for (int t0 = 0; t0 < n; t0 += CBW_T) {
-        const int t1 = min(n, t0 + CBW_T);
-        __syncthreads();  // the previous chunk's readers are done
-        for (int e = q; e < (t1 - t0 + KW - 1) * 2; e += CBW_THREADS)
-            xs[e / 2][e % 2] = xin(pts, o0, n, t0 + e / 2 - 2, e % 2, nrm);
-        __syncthreads();
-        for (int t = t0; t < t1; ++t) {
-            const int64_t o = ((int64_t)b * T + t) * C1 + c;
-            const float g = A[o] > 0.f ? dA[o] : 0.f;
-            acc = wt ? fmaf(g, xs[t - t0 + k][i], acc) : acc + g;
-        }
-    }
-    atomicAdd(grad + (wt ? OFF_W1 + q : OFF_B1 + c), acc);
 }
 
 __global__ void enc_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
@@ -628,8 +219,8 @@ __global__ void enc_adam(float* __restrict__ p, const float* __restrict__ g, flo
 // The a_t part comes from enc_conv_fwd_tc as one 16 KB BF16 image per step
 // already in the operand layout; thread 0 bulk-copies step t+1's image into
 // the second of two a-buffers while step t computes (per-buffer mbarriers
-// count the bytes).  a_t and h_t enter the products as BF16 (the SIMT training
-// kernel multiplies FP32 a and h by the BF16 weights) and the gates use the
+// count the bytes).  a_t and h_t enter the products as BF16 (the training
+// kernels multiply FP32 a and h by the BF16 weights) and the gates use the
 // hardware tanh, so the embeddings agree with the training forward to BF16
 // rounding of the activations.
 constexpr int TC_M = 128;
@@ -674,7 +265,7 @@ __device__ __forceinline__ uint4 pack8_bf16(const float* v) {
     return u;
 }
 
-// Conv output for the tensor-core GRU (same arithmetic as enc_conv_fwd, then
+// Conv output for the tensor-core GRU (same arithmetic as train_conv, then
 // rounded to BF16): for block g of 128 trajectories and step t, the 16 KB
 // image of the a_t operand (rows = trajectories, k = channels, core-matrix
 // layout) at Ab + (g * T + t) * 128 * 64.  Rows past B and steps past a
@@ -927,9 +518,9 @@ namespace {
 
 struct EncWs {  // views into the caller's workspace
     int* status;  // first word: bits OR-ed in by the tensor-core weight-gradient kernel (zeroed by the caller)
-    float *A, *H, *R, *Z, *N, *GHN, *G, *GH, *dA, *hl, *E, *dE, *dhl, *pred, *loss, *X;
+    float *hl, *E, *dE, *dhl, *pred, *loss, *X;
     __nv_bfloat16* wq;
-    void* wg;  // scratch of tsm_wgrad_tc
+    enc::TrainWs tr;  // the recurrences' buffers (tsm_train.cu)
 };
 
 int64_t align64(int64_t n) { return (n + 63) & ~int64_t(63); }
@@ -943,19 +534,9 @@ int64_t ws_layout(int B, int T, int P, float* base, EncWs* w) {
     };
     EncWs tmp;
     EncWs* x = w ? w : &tmp;
-    const int64_t BT = (int64_t)B * T;
     float* st = nullptr;
     take(&st, 1);
     if (base) x->status = reinterpret_cast<int*>(st);
-    take(&x->A, BT * enc::C1);
-    take(&x->H, (int64_t)B * (T + 1) * enc::HD);
-    take(&x->R, BT * enc::HD);
-    take(&x->Z, BT * enc::HD);
-    take(&x->N, BT * enc::HD);
-    take(&x->GHN, BT * enc::HD);
-    take(&x->G, BT * enc::G3);
-    take(&x->GH, BT * enc::G3);
-    take(&x->dA, BT * enc::C1);
     take(&x->hl, (int64_t)B * enc::HD);
     take(&x->E, (int64_t)B * enc::ED);
     take(&x->dE, (int64_t)B * enc::ED);
@@ -966,20 +547,10 @@ int64_t ws_layout(int B, int T, int P, float* base, EncWs* w) {
     float* wqf = nullptr;
     take(&wqf, (enc::N_PARAMS + 1) / 2);  // BF16 copy of the weights
     if (base) x->wq = reinterpret_cast<__nv_bfloat16*>(wqf);
-    float* wg = nullptr;
-    take(&wg, (tsm_wgrad_scratch_bytes(B, T) + 3) / 4);
-    if (base) x->wg = wg;
+    // (align64 keeps every buffer on a 256-byte boundary)
+    o += align64((enc::train_layout(B, T, base ? reinterpret_cast<unsigned char*>(base + o) : nullptr, &x->tr) + 3) / 4);
     return o;
 }
-
-constexpr int kGruFwdSmem = (enc::C1 * enc::G3 + enc::HD * enc::G3) * 2 +
-                            (enc::HD * enc::SPA + enc::C1 * enc::SPA + 2 * enc::S * enc::G3) * 4;
-constexpr int kGruBwdSmem = (enc::G3 * enc::HD + enc::G3 * enc::C1) * 2 +
-                            (2 * enc::S * enc::HD + 2 * enc::G3 * enc::SP) * 4;
-// one CTA per SM: dynamic shared memory plus the kernels' 1 KB of static
-// shared memory must fit the 227 KB a CTA may use
-static_assert(kGruFwdSmem + 1024 <= 227 * 1024, "enc_gru_fwd shared memory");
-static_assert(kGruBwdSmem + 1024 <= 227 * 1024, "enc_gru_bwd shared memory");
 
 int enc_check(cudaError_t e, const char* what) {
     if (e == cudaSuccess) return TSM_OK;
@@ -1003,14 +574,9 @@ int enc_forward(const float* params, const float* pts, const int64_t* off, const
     using namespace enc;
     const float4 n4 = make_float4(nrm[0], nrm[1], nrm[2], nrm[3]);
     enc_round_bf16<<<(OFF_WO + 255) / 256, 256, 0, s>>>(params, w.wq);
-    const int64_t tot = (int64_t)B * T * C1;
-    enc_conv_fwd<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(reinterpret_cast<const float2*>(pts), off, len, B, T,
-                                                                n4, w.wq, params, w.A);
-    int rc = enc_check(cudaFuncSetAttribute(enc_gru_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, kGruFwdSmem),
-                       "cudaFuncSetAttribute(enc_gru_fwd)");
+    const int rc = train_forward(reinterpret_cast<const float2*>(pts), off, len, B, T, n4, w.wq, params, w.tr, w.hl,
+                                 w.status, s);
     if (rc) return rc;
-    enc_gru_fwd<<<(B + S - 1) / S, GRU_THREADS, kGruFwdSmem, s>>>(w.A, len, B, T, w.wq, params, w.H, w.R, w.Z, w.N,
-                                                                   w.GHN, w.hl);
     enc_head_fwd<<<(unsigned)((B + HEAD_B - 1) / HEAD_B), EO, 0, s>>>(w.hl, B, params, w.E,
                                                                       reinterpret_cast<const float2*>(pts), off, len,
                                                                       n4, w.X);
@@ -1021,23 +587,12 @@ int enc_backward(const float* params, const float* pts, const int64_t* off, cons
                  const float* nrm, EncWs& w, float* grad, cudaStream_t s) {
     using namespace enc;
     const float4 n4 = make_float4(nrm[0], nrm[1], nrm[2], nrm[3]);
-    enc_head_bwd_w<<<EO, HD, 0, s>>>(w.dE, w.hl, B, grad);
+    if ((B + HB_B - 1) / HB_B > 65535) return tsm_internal_fail(TSM_EINVAL, "encoder: batch too large");
+    enc_head_bwd_w<<<dim3(EO, (B + HB_B - 1) / HB_B), HD, 0, s>>>(w.dE, w.hl, B, grad);
     enc_skip_bwd<<<(unsigned)(((int64_t)B * SK + 255) / 256 < 256 ? ((int64_t)B * SK + 255) / 256 : 256), 256, 0, s>>>(
         w.dE, w.X, B, params, grad);
     enc_head_bwd_h<<<(unsigned)(((int64_t)B * HD + 255) / 256), 256, 0, s>>>(w.dE, B, params, w.dhl);
-    int rc = enc_check(cudaFuncSetAttribute(enc_gru_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, kGruBwdSmem),
-                       "cudaFuncSetAttribute(enc_gru_bwd)");
-    if (rc) return rc;
-    // the bias gradients (sums of the gate gradients over the valid (b, t)) come out of the BPTT kernel
-    enc_gru_bwd<<<(B + S - 1) / S, GRU_THREADS, kGruBwdSmem, s>>>(w.dhl, len, B, T, w.wq, w.H, w.R, w.Z, w.N,
-                                                                   w.GHN, w.G, w.GH, w.dA, grad + OFF_BIH,
-                                                                   grad + OFF_BHH);
-    // weight gradients dWih[j][c] += G . A, dWhh[j][k] += GH . H[t]: reductions over the valid (b, t) on the
-    // tensor cores (tsm_wgrad.cu)
-    if ((rc = tsm_wgrad_tc(w.G, w.GH, w.A, w.H, len, B, T, w.wg, w.status, grad + OFF_WIH, grad + OFF_WHH, s)))
-        return rc;
-    enc_conv_bwd<<<B, CBW_THREADS, 0, s>>>(reinterpret_cast<const float2*>(pts), off, len, T, n4, w.A, w.dA, grad);
-    return enc_check(cudaGetLastError(), "encoder backward launch");
+    return train_backward(reinterpret_cast<const float2*>(pts), off, len, B, T, n4, w.wq, w.dhl, w.tr, grad, w.status, s);
 }
 
 // Inference workspace: the BF16 a_t images (B rounded up to 128 rows), last
@@ -1184,7 +739,7 @@ int tsm_enc_train_status(void* workspace, int32_t* status, void* stream) {
     if (*status == 0) return TSM_OK;
     if ((rc = enc_check(cudaMemset(workspace, 0, 4), "tsm_enc_train_status: clear"))) return rc;
     char b[256];
-    snprintf(b, sizeof(b), "tsm_enc_loss_grad: a tensor-core wait ran out in the weight gradients (status %d%s); "
+    snprintf(b, sizeof(b), "tsm_enc_loss_grad: a tensor-core wait ran out (status %d%s); "
              "the gradients of the calls since the last check are incomplete", *status,
              (*status & 128) ? ": tensor memory not freed, reset the device" : "");
     return tsm_internal_fail(TSM_ETIMEOUT, b);

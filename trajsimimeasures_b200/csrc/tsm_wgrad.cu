@@ -1,10 +1,10 @@
 // Weight gradients of the encoder's GRU on the tensor cores (tcgen05):
-//     dW_ih[j][c]  = sum_(b,t) G [b][t][j] A[b][t][c]       384 x 64
-//     dW_hh[j][kk] = sum_(b,t) GH[b][t][j] H[b][t][kk]      384 x 128
-// over the valid steps t < len[b] only (the padded steps of a batch, about
-// half of b x T for lengths U{20..200}, are skipped), G / GH the gate
-// gradients of the input and hidden side written by the BPTT kernel, A the
-// conv activations and H the hidden state before step t.
+//     dW_ih[j][c]  = sum_(slot,s) G [j] A[c]       384 x 64
+//     dW_hh[j][kk] = sum_(slot,s) GH[j] H[kk]      384 x 128
+// over the batch's time slots and the 16 trajectories of each (tsm_train.h; the
+// gate gradients of a trajectory past its end are zero), G / GH the gate
+// gradients of the input and hidden side, which differ in the n rows only, A
+// the conv activations and H the hidden state before the step.
 //
 // Precision.  The four operands are FP32.  Each is split into BF16 parts,
 // x = hi + lo with lo = bf16(x - hi) (BF16 keeps FP32's exponent range, which
@@ -13,19 +13,16 @@
 // with FP32 accumulation: three MMAs per K step, about 2^-16 relative per
 // product (the split-product method of Markidis et al., IPDPSW 2018).
 //
-// Steps (one stream, no host synchronisation):
-//   wg_koff      exclusive scan of the clamped lengths -> koff[B + 1] (K = koff[B])
-//   wg_krow      krow[koff[b] + t] = b * T + t for t < len[b] (the compact K order)
-//   wg_image     FP32 rows -> BF16 hi and lo operand images, K-major core-matrix
-//                layout (tsm_umma.cuh), K rounded up to the stage size with zeros
-//   wg_kernel    split-K over the CTAs: CTA (m tile of 128 rows of j, K range)
-//                streams both products' operands through a four-stage ring
-//                (cp.async.bulk, mbarrier transaction counts), one thread issues
-//                six MMAs per K step into two accumulators (64 and 128 columns
-//                of tensor memory), and all four warps add the result to the
-//                gradient with atomics.  Waits are bounded (about 1 s of SM
-//                clocks); one that runs out ORs a bit into *status and the CTA
-//                adds nothing.
+// The recurrences write the hi and lo images themselves (tsm_train.cu), K-major
+// core-matrix layout (tsm_umma.cuh), 16 K per slot.  One kernel, split-K over
+// the CTAs: CTA (m tile of 128 rows of j, K range) streams both products'
+// operands through a four-stage ring (cp.async.bulk, mbarrier transaction
+// counts), one thread issues six MMAs per K step into four accumulators, and
+// all four warps add the results to the gradient with atomics.  The cross
+// products accumulate apart from the hi . hi ones: an accumulation step
+// truncates, and 900 instead of 300 of them on the large sums made the error of
+// dW_ih half again as large (1,024 pairs: 4.2e-6 of the gradient's norm).  Waits are bounded (about 1 s of SM clocks); one that
+// runs out ORs a bit into *status and the CTA adds nothing.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -57,102 +54,16 @@ constexpr int S_GHI = 0, S_GLO = M_PART, S_GHHI = 2 * M_PART, S_GHLO = 3 * M_PAR
 constexpr int STAGE = S_HLO + H_PART;  // 57,344
 constexpr int OFF_BAR = NST * STAGE;
 constexpr int SMEM = OFF_BAR + 128;    // 229,504
-constexpr uint32_t TMEM_COLS = 256;    // acc_ih at column 0 (64 wide), acc_hh at 64 (128 wide)
+// accumulators ih (64 columns) and hh (128) of the hi . hi products at column 0, of the cross products at T_X
+constexpr uint32_t TMEM_COLS = 512, T_X = 256;
 constexpr long long WAIT_CYCLES = 2000000000LL;
 static_assert(SMEM <= 227 * 1024, "shared memory");
 
 // status bits (OR-ed into the caller's word)
 constexpr int ERR_COPY = 16, ERR_MMA = 32, ERR_DONE = 64, ERR_TMEM = 128;
 
-// koff[b] = sum_{b' < b} min(max(len[b'], 0), T), koff[B] = K.  One CTA of 1024 threads.
-__global__ void __launch_bounds__(1024) wg_koff(const int32_t* __restrict__ len, int B, int T,
-                                                 int64_t* __restrict__ koff) {
-    __shared__ int64_t warp_tot[32];
-    __shared__ int64_t carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int b0 = 0; b0 < B; b0 += 1024) {
-        const int b = b0 + threadIdx.x;
-        const int64_t v = b < B ? (int64_t)min(max(len[b], 0), T) : 0;
-        int64_t x = v;  // inclusive warp scan
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) warp_tot[warp] = x;
-        __syncthreads();
-        if (warp == 0) {
-            int64_t w = warp_tot[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int64_t y = __shfl_up_sync(0xffffffffu, w, o);
-                if (lane >= o) w += y;
-            }
-            warp_tot[lane] = w;  // inclusive over warps
-        }
-        __syncthreads();
-        const int64_t before = carry + (warp > 0 ? warp_tot[warp - 1] : 0) + x - v;
-        if (b < B) koff[b] = before;
-        __syncthreads();
-        if (threadIdx.x == 0) carry += warp_tot[31];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) koff[B] = carry;
-}
-
-// krow[koff[b] + t] = b * T + t for t < len[b].  One thread per (b, t).
-__global__ void wg_krow(const int32_t* __restrict__ len, const int64_t* __restrict__ koff, int B, int T,
-                        int64_t* __restrict__ krow) {
-    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= (int64_t)B * T) return;
-    const int b = (int)(g / T), t = (int)(g % T);
-    if (t < min(max(len[b], 0), T)) krow[koff[b] + t] = g;
-}
-
-// Operand images of a source with `cols` values per row: image row r (of
-// cols, in tiles of R rows) holds, along K, the values src[row(k)][r], row(k)
-// = krow[k] (+ krow[k] / T when hrows: H keeps T + 1 rows per trajectory).
-// Chunks of 8 K values are split into BF16 hi and lo parts and stored in the
-// core-matrix layout: tile i at byte i * kp * R * 2, chunk c at c * R * 16,
-// row r % R at 16 (r % R).  Chunks up to the end of the last stage hold zeros
-// past K; later chunks are not written (the kernel reads only up to there).
-// One thread per (chunk, row); consecutive threads take consecutive rows
-// (coalesced reads and 16-byte stores).
-__global__ void wg_image(const float* __restrict__ src, int cols, int R, const int64_t* __restrict__ krow,
-                         const int64_t* __restrict__ koff, int B, int T, int hrows, int64_t kp,
-                         __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo) {
-    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= kp / 8 * cols) return;
-    const int r = (int)(g % cols);
-    const int64_t c = g / cols;
-    const int64_t K = koff[B];
-    const int64_t kend = (K + SKW - 1) / SKW * SKW;
-    if (8 * c >= kend) return;
-    __align__(16) __nv_bfloat16 vh[8], vl[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        const int64_t k = 8 * c + e;
-        float x = 0.f;
-        if (k < K) {
-            const int64_t kr = krow[k];
-            x = src[(kr + (hrows ? kr / T : 0)) * cols + r];
-        }
-        vh[e] = __float2bfloat16_rn(x);
-        vl[e] = __float2bfloat16_rn(x - __bfloat162float(vh[e]));
-    }
-    const int64_t o = (int64_t)(r / R) * kp * R * 2 + c * R * 16 + (int64_t)(r % R) * 16;
-    *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(hi) + o) = *reinterpret_cast<const uint4*>(vh);
-    *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(lo) + o) = *reinterpret_cast<const uint4*>(vl);
-}
-
 __global__ void __launch_bounds__(THREADS, 1) wg_kernel(
-    const __nv_bfloat16* __restrict__ g_hi, const __nv_bfloat16* __restrict__ g_lo,
-    const __nv_bfloat16* __restrict__ gh_hi, const __nv_bfloat16* __restrict__ gh_lo,
-    const __nv_bfloat16* __restrict__ a_hi, const __nv_bfloat16* __restrict__ a_lo,
-    const __nv_bfloat16* __restrict__ h_hi, const __nv_bfloat16* __restrict__ h_lo, const int64_t* __restrict__ koff,
-    int B, int64_t kp, float* __restrict__ d_ih, float* __restrict__ d_hh, int* __restrict__ status,
+    enc::TrainWs w, float* __restrict__ d_ih, float* __restrict__ d_hh, int* __restrict__ status,
     long long wait_cycles) {
     namespace U = tsm::umma;
     extern __shared__ __align__(1024) unsigned char sm[];
@@ -164,10 +75,10 @@ __global__ void __launch_bounds__(THREADS, 1) wg_kernel(
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + OFF_BAR + 16 * NST + 8);
     volatile int* flags = reinterpret_cast<volatile int*>(sm + OFF_BAR + 16 * NST + 12);  // bit 0 failed, 1 busy
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int mt = blockIdx.x;  // tile of j
-    // this CTA's stages [s0, s1) of the K range, from the device-side K
-    const int64_t K = koff[B];
-    const int64_t nst_all = (K + SKW - 1) / SKW;
+    const int mt = blockIdx.x;  // tile of j: gate r, z or n
+    const bool n_rows = mt == 2;
+    // this CTA's stages [s0, s1) of the K range (a stage: two slots of 16), from the device-side slot count
+    const int64_t nst_all = w.slot0[w.blocks] / 2;
     const int64_t per = (nst_all + gridDim.y - 1) / gridDim.y;
     const int64_t s0 = (int64_t)blockIdx.y * per;
     const int64_t s1 = min(nst_all, s0 + per);
@@ -190,10 +101,7 @@ __global__ void __launch_bounds__(THREADS, 1) wg_kernel(
     const uint32_t tmem = *tmem_slot;
 
     if (warp == 0 && lane == 0) {  // copies
-        const int64_t mt_off = (int64_t)mt * kp * MT * 2;  // byte offset of this j tile in the G / GH images
-        auto src = [&](const __nv_bfloat16* p, int64_t tile_off, int64_t part, int64_t s) {
-            return reinterpret_cast<const unsigned char*>(p) + tile_off + s * part;
-        };
+        const int64_t tile = w.slots * 2 * MT * 16;  // bytes of one gate's image
         int64_t g = 0;
         for (int64_t s = s0; s < s1; ++s, ++g) {
             const int slot = (int)(g % NST);
@@ -204,15 +112,20 @@ __global__ void __launch_bounds__(THREADS, 1) wg_kernel(
                 break;
             }
             const uint32_t st = sbase + slot * STAGE;
-            U::mbar_arrive_expect_tx(full(slot), STAGE);
-            U::bulk_load(st + S_GHI, src(g_hi, mt_off, M_PART, s), M_PART, full(slot));
-            U::bulk_load(st + S_GLO, src(g_lo, mt_off, M_PART, s), M_PART, full(slot));
-            U::bulk_load(st + S_GHHI, src(gh_hi, mt_off, M_PART, s), M_PART, full(slot));
-            U::bulk_load(st + S_GHLO, src(gh_lo, mt_off, M_PART, s), M_PART, full(slot));
-            U::bulk_load(st + S_AHI, src(a_hi, 0, A_PART, s), A_PART, full(slot));
-            U::bulk_load(st + S_ALO, src(a_lo, 0, A_PART, s), A_PART, full(slot));
-            U::bulk_load(st + S_HHI, src(h_hi, 0, H_PART, s), H_PART, full(slot));
-            U::bulk_load(st + S_HLO, src(h_lo, 0, H_PART, s), H_PART, full(slot));
+            U::mbar_arrive_expect_tx(full(slot), n_rows ? STAGE : STAGE - 2 * M_PART);
+            auto load = [&](int at, const unsigned char* src, int part) {
+                U::bulk_load(st + at, src + s * part, part, full(slot));
+            };
+            load(S_GHI, w.g_hi + mt * tile, M_PART);
+            load(S_GLO, w.g_lo + mt * tile, M_PART);
+            if (n_rows) {  // the hidden side has its own n gradients
+                load(S_GHHI, w.g_hi + 3 * tile, M_PART);
+                load(S_GHLO, w.g_lo + 3 * tile, M_PART);
+            }
+            load(S_AHI, w.a_hi, A_PART);
+            load(S_ALO, w.a_lo, A_PART);
+            load(S_HHI, w.h_hi, H_PART);
+            load(S_HLO, w.h_lo, H_PART);
         }
         // every copy issued lands before the CTA exits: the last use of each slot
         for (int slot = 0; slot < NST; ++slot)
@@ -235,18 +148,18 @@ __global__ void __launch_bounds__(THREADS, 1) wg_kernel(
                 const uint32_t first = (g == 0 && kk == 0) ? 0u : 1u;
                 const uint64_t gd_hi = U::smem_desc(st + S_GHI + kk * 2 * (MT * 16), MT * 16, 128);
                 const uint64_t gd_lo = U::smem_desc(st + S_GLO + kk * 2 * (MT * 16), MT * 16, 128);
-                const uint64_t ghd_hi = U::smem_desc(st + S_GHHI + kk * 2 * (MT * 16), MT * 16, 128);
-                const uint64_t ghd_lo = U::smem_desc(st + S_GHLO + kk * 2 * (MT * 16), MT * 16, 128);
+                const uint64_t ghd_hi = n_rows ? U::smem_desc(st + S_GHHI + kk * 2 * (MT * 16), MT * 16, 128) : gd_hi;
+                const uint64_t ghd_lo = n_rows ? U::smem_desc(st + S_GHLO + kk * 2 * (MT * 16), MT * 16, 128) : gd_lo;
                 const uint64_t ad_hi = U::smem_desc(st + S_AHI + kk * 2 * (NA * 16), NA * 16, 128);
                 const uint64_t ad_lo = U::smem_desc(st + S_ALO + kk * 2 * (NA * 16), NA * 16, 128);
                 const uint64_t hd_hi = U::smem_desc(st + S_HHI + kk * 2 * (NH * 16), NH * 16, 128);
                 const uint64_t hd_lo = U::smem_desc(st + S_HLO + kk * 2 * (NH * 16), NH * 16, 128);
                 U::mma_bf16(t_ih, gd_hi, ad_hi, id_ih, first);
-                U::mma_bf16(t_ih, gd_lo, ad_hi, id_ih, 1u);
-                U::mma_bf16(t_ih, gd_hi, ad_lo, id_ih, 1u);
+                U::mma_bf16(t_ih + T_X, gd_lo, ad_hi, id_ih, first);
+                U::mma_bf16(t_ih + T_X, gd_hi, ad_lo, id_ih, 1u);
                 U::mma_bf16(t_hh, ghd_hi, hd_hi, id_hh, first);
-                U::mma_bf16(t_hh, ghd_lo, hd_hi, id_hh, 1u);
-                U::mma_bf16(t_hh, ghd_hi, hd_lo, id_hh, 1u);
+                U::mma_bf16(t_hh + T_X, ghd_lo, hd_hi, id_hh, first);
+                U::mma_bf16(t_hh + T_X, ghd_hi, hd_lo, id_hh, 1u);
             }
             U::commit(empty(slot));
         }
@@ -266,16 +179,14 @@ __global__ void __launch_bounds__(THREADS, 1) wg_kernel(
         const int64_t j = (int64_t)mt * MT + 32 * warp + lane;
         const uint32_t ta = tmem + ((uint32_t)(32 * warp) << 16);
         for (int c0 = 0; c0 < NA + NH; c0 += 16) {
-            uint32_t r[16];
+            uint32_t r[16], x[16];
             U::ld16(ta + c0, r);
+            U::ld16(ta + T_X + c0, x);
             U::wait_ld(r);
-            if (c0 < NA) {
+            U::wait_ld(x);
+            float* dst = c0 < NA ? d_ih + j * NA + c0 : d_hh + j * NH + (c0 - NA);
 #pragma unroll
-                for (int i = 0; i < 16; ++i) atomicAdd(d_ih + j * NA + c0 + i, __uint_as_float(r[i]));
-            } else {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) atomicAdd(d_hh + j * NH + (c0 - NA) + i, __uint_as_float(r[i]));
-            }
+            for (int i = 0; i < 16; ++i) atomicAdd(dst + i, __uint_as_float(r[i]) + __uint_as_float(x[i]));
         }
     }
     U::fence_before_sync();
@@ -295,8 +206,6 @@ __global__ void __launch_bounds__(THREADS, 1) wg_kernel(
 
 namespace {
 
-int64_t al256(int64_t n) { return (n + 255) & ~int64_t(255); }
-
 int wg_check(cudaError_t e, const char* what) {
     if (e == cudaSuccess) return TSM_OK;
     char b[256];
@@ -304,60 +213,10 @@ int wg_check(cudaError_t e, const char* what) {
     return tsm_internal_fail(TSM_ECUDA, b);
 }
 
-struct WgScratch {
-    int64_t* koff;
-    int64_t* krow;
-    __nv_bfloat16 *g_hi, *g_lo, *gh_hi, *gh_lo, *a_hi, *a_lo, *h_hi, *h_lo;
-};
-
-// Lays the scratch out (base != NULL) and returns its size in bytes.
-int64_t wg_layout(int B, int T, unsigned char* base, WgScratch* w) {
-    using namespace tsm::wgrad;
-    const int64_t kp = ((int64_t)B * T + SKW - 1) / SKW * SKW;
-    int64_t o = 0;
-    auto take = [&](int64_t bytes) {
-        unsigned char* p = base ? base + o : nullptr;
-        o += al256(bytes);
-        return p;
-    };
-    WgScratch tmp;
-    WgScratch* x = w ? w : &tmp;
-    x->koff = reinterpret_cast<int64_t*>(take((int64_t)(B + 1) * 8));
-    x->krow = reinterpret_cast<int64_t*>(take(kp * 8));
-    x->g_hi = reinterpret_cast<__nv_bfloat16*>(take(kp * G3 * 2));
-    x->g_lo = reinterpret_cast<__nv_bfloat16*>(take(kp * G3 * 2));
-    x->gh_hi = reinterpret_cast<__nv_bfloat16*>(take(kp * G3 * 2));
-    x->gh_lo = reinterpret_cast<__nv_bfloat16*>(take(kp * G3 * 2));
-    x->a_hi = reinterpret_cast<__nv_bfloat16*>(take(kp * NA * 2));
-    x->a_lo = reinterpret_cast<__nv_bfloat16*>(take(kp * NA * 2));
-    x->h_hi = reinterpret_cast<__nv_bfloat16*>(take(kp * NH * 2));
-    x->h_lo = reinterpret_cast<__nv_bfloat16*>(take(kp * NH * 2));
-    return o;
-}
-
 }  // namespace
 
-int64_t tsm_wgrad_scratch_bytes(int B, int T) { return wg_layout(B, T, nullptr, nullptr); }
-
-int tsm_wgrad_tc(const float* G, const float* GH, const float* A, const float* H, const int32_t* len, int B, int T,
-                 void* scratch, int* status, float* d_ih, float* d_hh, cudaStream_t s) {
+int tsm_wgrad_tc(const enc::TrainWs& w, int* status, float* d_ih, float* d_hh, cudaStream_t s) {
     using namespace tsm::wgrad;
-    if (B < 1 || T < 1 || !scratch || !status) return tsm_internal_fail(TSM_EINVAL, "wgrad: bad arguments");
-    if (reinterpret_cast<uintptr_t>(scratch) % 256) return tsm_internal_fail(TSM_EINVAL, "wgrad: scratch alignment");
-    WgScratch w;
-    wg_layout(B, T, static_cast<unsigned char*>(scratch), &w);
-    const int64_t bt = (int64_t)B * T;
-    const int64_t kp = (bt + SKW - 1) / SKW * SKW;
-    wg_koff<<<1, 1024, 0, s>>>(len, B, T, w.koff);
-    wg_krow<<<(unsigned)((bt + 255) / 256), 256, 0, s>>>(len, w.koff, B, T, w.krow);
-    auto image = [&](const float* src, int cols, int R, int hrows, __nv_bfloat16* hi, __nv_bfloat16* lo) {
-        const int64_t n = kp / 8 * cols;
-        wg_image<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(src, cols, R, w.krow, w.koff, B, T, hrows, kp, hi, lo);
-    };
-    image(G, G3, MT, 0, w.g_hi, w.g_lo);
-    image(GH, G3, MT, 0, w.gh_hi, w.gh_lo);
-    image(A, NA, NA, 0, w.a_hi, w.a_lo);
-    image(H, NH, NH, 1, w.h_hi, w.h_lo);
     int rc = wg_check(cudaFuncSetAttribute(wg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM),
                       "cudaFuncSetAttribute(wg_kernel)");
     if (rc) return rc;
@@ -365,11 +224,8 @@ int tsm_wgrad_tc(const float* G, const float* GH, const float* A, const float* H
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // K split: one wave of CTAs over the three j tiles, at most the stages there can be
     int64_t ksplit = sms / (G3 / MT);
-    const int64_t nst_max = kp / SKW;
-    if (ksplit > nst_max) ksplit = nst_max;
+    if (ksplit > w.slots / 2) ksplit = w.slots / 2;
     if (ksplit < 1) ksplit = 1;
-    wg_kernel<<<dim3(G3 / MT, (unsigned)ksplit), THREADS, SMEM, s>>>(w.g_hi, w.g_lo, w.gh_hi, w.gh_lo, w.a_hi, w.a_lo,
-                                                                       w.h_hi, w.h_lo, w.koff, B, kp, d_ih, d_hh,
-                                                                       status, WAIT_CYCLES);
+    wg_kernel<<<dim3(G3 / MT, (unsigned)ksplit), THREADS, SMEM, s>>>(w, d_ih, d_hh, status, WAIT_CYCLES);
     return wg_check(cudaGetLastError(), "wgrad launch");
 }

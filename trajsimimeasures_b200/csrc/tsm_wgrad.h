@@ -1,17 +1,13 @@
 // Encoder weight gradients on the tensor cores (tsm_wgrad.cu), called by the
-// training backward of tsm_encoder.cu.
+// training backward (tsm_train.cu).
 #pragma once
 
 #include <cuda_runtime.h>
-#include <stdint.h>
 
-// Device scratch (bytes, 256-byte aligned start) for a batch of B
-// trajectories of at most T steps.
-int64_t tsm_wgrad_scratch_bytes(int B, int T);
+#include "tsm_train.h"
 
-// d_ih[384][64] += sum over valid (b, t) of G[b][t][:] (x) A[b][t][:],
-// d_hh[384][128] += sum of GH[b][t][:] (x) H[b][t][:] (H: T + 1 rows per
-// trajectory).  Stream-ordered; a bounded wait that runs out ORs a bit into
-// *status (device int) and its CTA adds nothing.
-int tsm_wgrad_tc(const float* G, const float* GH, const float* A, const float* H, const int32_t* len, int B, int T,
-                 void* scratch, int* status, float* d_ih, float* d_hh, cudaStream_t s);
+// d_ih[384][64] += sum over the batch's slots and trajectories of g (x) a,
+// d_hh[384][128] += sum of g (x) h (the hidden-side n gradients for the n
+// rows), from the BF16 hi/lo images of w.  Stream-ordered; a bounded wait that
+// runs out ORs a bit into *status (device int) and its CTA adds nothing.
+int tsm_wgrad_tc(const enc::TrainWs& w, int* status, float* d_ih, float* d_hh, cudaStream_t s);

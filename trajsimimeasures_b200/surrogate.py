@@ -135,9 +135,9 @@ class Encoder:
         return self._ws
 
     def check_training(self, stream=None):
-        """Raises TsmError if a bounded wait of the tensor-core weight-gradient
-        kernel ran out in a loss_grad call since the last check (the gradients
-        of those calls are incomplete).  Synchronises the stream; fit() calls
+        """Raises TsmError if a bounded wait of a training kernel ran out in a
+        loss_grad call since the last check (the gradients of those calls are
+        incomplete).  Synchronises the stream; fit() calls
         it once per epoch."""
         if self._ws is None:
             return
@@ -212,6 +212,8 @@ class Encoder:
                                          self._nrm_ptr(), _ptr(ws), _ptr(r), _stream_ptr(stream))
                 _lib.check(rc, "tsm_enc_forward")
         out[perm] = res
+        if not tensor_cores:
+            self.check_training(stream)  # the training kernels' status word
         if status is not None and status_out is None and int(status.item()):
             raise _lib.TsmError(f"tsm_enc_embed: a tensor-core wait ran out (status {int(status.item())}); "
                                 "the affected embeddings are NaN")
