@@ -166,7 +166,7 @@ __device__ __forceinline__ int bits_count(const float2* __restrict__ rowp, int n
                         if (rb + g >= nr) break;
 #pragma unroll
                         for (int r = g; r < g + 8; ++r) {
-                            const float d2 = d2nr<true>(n[r], c);
+                            const float d2 = d2nr(n[r], c);
                             asm("{\n\t.reg .pred q;\n\tsetp.lt.f32 q, %1, %2;\n\t@q add.u32 %0, %0, %3;\n\t}"
                                 : "+r"(m[r & 3])
                                 : "f"(d2), "f"(eps2), "r"(1u << r));
@@ -214,7 +214,7 @@ __device__ __forceinline__ int bits_count_warp(const float2* __restrict__ rowp, 
             const int e = min(32, nc - jb);
 #pragma unroll 4
             for (int i = 0; i < e; ++i) {
-                const uint32_t eq = __ballot_sync(kFull, d2nr<true>(n, cols[jb + i]) < eps2);
+                const uint32_t eq = __ballot_sync(kFull, d2nr(n, cols[jb + i]) < eps2);
                 bits_column<M>(eq, vp, vn, cp, cn);
             }
             if (lane == 0) {

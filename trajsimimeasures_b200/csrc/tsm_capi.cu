@@ -46,6 +46,8 @@ static_assert(tsm::kHeavyRows >= kTileCap, "a tile-heavy pair must have a side l
 // Matrix mode keeps the query as the tile kernel's columns: its boundary
 // rows (32 per warp) and staged columns must fit one CTA's shared memory.
 constexpr int kMatrixQueryMax = 1400;
+// Longest query of the matrix kernel with one lane per pair (see matrix_launch).
+constexpr int kMatrixLaneMax = 96;
 // Longest trajectory accepted by the paired kernels: the wave kernel keeps 4
 // bytes of shared memory per point of a pair's shorter side for each of its W
 // warps (W = 4 up to 8192 points, 2 up to 16384, 1 up to 32768: 128 KB).
@@ -385,11 +387,22 @@ int matrix_launch(const char* who, int measure, const float* q_pts, const int64_
         return launch(tsm_k::bits_matrix(measure), dim3((unsigned)ctas), dim3(threads), qg * qcap * 8 + carry_bytes, args, s);
     }
     const void* fn = tsm_k::dp_matrix(measure, R, exact);
-    const int W = warps_for(qcap, qcap * 16);
-    const int threads = 32 * W;
-    const int smem = qcap * 16 + W * 32 * qcap * 4;
+    // Two lanes per pair; one lane per pair where the query is short.  Measured, 2000 x 2000 random walks, two / one,
+    // ms: DTW 2..20 points 0.33 / 0.26, 20..64 2.18 / 2.08, 20..100 4.25 / 4.24, 20..140 7.3 / 7.6, 20..200 13.9 / 15.2;
+    // Frechet 0.31 / 0.26, 1.86 / 1.85, 3.60 / 3.68, 6.2 / 6.5, 11.6 / 12.3; ERP 0.50 / 0.54, 2.93 / 3.18, 5.6 / 6.0.
+    const bool lane = measure != TSM_ERP && R == 8 && qcap <= kMatrixLaneMax;
+    if (lane) fn = tsm_k::dp_matrix_lane(measure, exact);
+    // two lanes: four warps while two CTAs of them fit an SM (at 200 points four do: 16 warps), else as many as do
+    // (8 warps: DTW 14.1, one warp: 14.9)
+    auto smem_of = [&](int w) {
+        return lane ? qcap * 16 + w * 32 * qcap * 4 : (qcap + 3) * 16 + w * tsm::duo_ring(qcap) * 4;
+    };
+    int W = 4;
+    while (W > 1 && smem_of(W) > kSmemPerCta) --W;
+    const int threads = 32 * W, per = lane ? threads : threads / 2;
+    const int smem = smem_of(W);
     if (smem > kSmemMax) return fail(TSM_ETOOLONG, "%s: boundary rows need %d bytes", who, smem);
-    int chunks = (int)((nd + threads - 1) / threads);
+    int chunks = (int)((nd + per - 1) / per);
     if ((int64_t)chunks * nq > 0x7fffffffLL) return fail(TSM_EINVAL, "%s: grid too large", who);
     dim3 grid((unsigned)(chunks * nq));
     void* args[] = {&q2,   &q_off,  &q_len, &q_order, &d2,  &d_off,     &d_len, &d_order, &ndd,

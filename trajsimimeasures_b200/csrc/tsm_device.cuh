@@ -61,18 +61,12 @@ __device__ __forceinline__ float d2f(float ax, float ay, float bx, float by) {
 // The same squared distance with the row point held negated, nr = -r: the
 // difference c + nr = -(r - c) is exactly the negated scalar difference
 // (round-to-nearest is symmetric) and the squares do not see the sign, so
-// the value is bit-identical to d2f(r.x, r.y, c.x, c.y).  PACKED: the
-// difference is one f32x2 add instead of two scalar adds.  Measured on B200
-// (same inputs, same outputs): the packed add is faster for every measure
-// with per-lane global columns (paired batches, 5-15 %) and for DTW, EDR,
-// LCSS and ERP with columns staged in shared memory (all-pairs, 0.5-4 %);
-// discrete Frechet with shared-memory columns is 2 % faster with the scalar
-// adds (kPackedSmem in the cell policies).
-template <bool PACKED>
+// the value is bit-identical to d2f(r.x, r.y, c.x, c.y).  The difference is
+// one f32x2 add: it costs what two scalar adds do but one instruction less, and
+// measured (same inputs, same outputs) 5-15 % faster in the paired kernels, and
+// 4 to 6 % in the matrix kernels.
 __device__ __forceinline__ float d2nr(float2 nr, float2 c) {
-    float2 d;
-    if constexpr (PACKED) d = __fadd2_rn(nr, c);
-    else d = make_float2(__fadd_rn(nr.x, c.x), __fadd_rn(nr.y, c.y));
+    const float2 d = __fadd2_rn(nr, c);
     return __fmaf_rn(d.y, d.y, __fmul_rn(d.x, d.x));
 }
 
@@ -129,18 +123,12 @@ __device__ __forceinline__ float gapsum(const float2* __restrict__ t, int n, con
 template <bool EXACT>
 struct DtwCell {
     static constexpr bool kGap = false;
-    static constexpr bool kPackedSmem = true;  // f32x2 difference with shared-memory columns (see d2nr)
     __device__ __forceinline__ static float corner() { return 0.f; }
     __device__ __forceinline__ static float rowb(float /*srow*/, int /*i*/) { return CUDART_INF_F; }
     __device__ __forceinline__ static float topb(float /*scol*/, int /*j*/) { return CUDART_INF_F; }
     __device__ __forceinline__ static float cell(float dg, float up, float left, float d2,
                                                  float /*grow*/, float /*gcol*/, float /*eps2*/) {
         return __fadd_rn(tsqrt<EXACT>(d2), min3f(dg, up, left));
-    }
-    // split form (cell == comb(term(d2))): the local term alone, then the recurrence
-    __device__ __forceinline__ static float term(float d2, float) { return tsqrt<EXACT>(d2); }
-    __device__ __forceinline__ static float comb(float dg, float up, float left, float t, float, float) {
-        return __fadd_rn(t, min3f(dg, up, left));
     }
 };
 
@@ -149,17 +137,12 @@ struct DtwCell {
 template <bool EXACT>
 struct FrechetCell {
     static constexpr bool kGap = false;
-    static constexpr bool kPackedSmem = false;  // f32x2 difference with shared-memory columns (see d2nr)
     __device__ __forceinline__ static float corner() { return 0.f; }
     __device__ __forceinline__ static float rowb(float, int) { return CUDART_INF_F; }
     __device__ __forceinline__ static float topb(float, int) { return CUDART_INF_F; }
     __device__ __forceinline__ static float cell(float dg, float up, float left, float d2,
                                                  float, float, float) {
         return fmaxf(d2, min3f(dg, up, left));
-    }
-    __device__ __forceinline__ static float term(float d2, float) { return d2; }
-    __device__ __forceinline__ static float comb(float dg, float up, float left, float t, float, float) {
-        return fmaxf(t, min3f(dg, up, left));
     }
 };
 
@@ -168,17 +151,12 @@ struct FrechetCell {
 template <bool EXACT>
 struct ErpCell {
     static constexpr bool kGap = true;
-    static constexpr bool kPackedSmem = true;  // f32x2 difference with shared-memory columns (see d2nr)
     __device__ __forceinline__ static float corner() { return 0.f; }
     __device__ __forceinline__ static float rowb(float srow, int) { return srow; }
     __device__ __forceinline__ static float topb(float scol, int) { return scol; }
     __device__ __forceinline__ static float cell(float dg, float up, float left, float d2,
                                                  float grow, float gcol, float) {
         return min3f(__fadd_rn(left, gcol), __fadd_rn(up, grow), __fadd_rn(dg, tsqrt<EXACT>(d2)));
-    }
-    __device__ __forceinline__ static float term(float d2, float) { return tsqrt<EXACT>(d2); }
-    __device__ __forceinline__ static float comb(float dg, float up, float left, float t, float grow, float gcol) {
-        return min3f(__fadd_rn(left, gcol), __fadd_rn(up, grow), __fadd_rn(dg, t));
     }
 };
 
@@ -191,7 +169,6 @@ struct ErpCell {
 template <bool EXACT>
 struct EdrCell {
     static constexpr bool kGap = false;
-    static constexpr bool kPackedSmem = true;  // f32x2 difference with shared-memory columns (see d2nr)
     __device__ __forceinline__ static float corner() { return 2.f; }
     __device__ __forceinline__ static float rowb(float, int i) { return (float)(1 - i); }
     __device__ __forceinline__ static float topb(float, int j) { return (float)(1 - j); }
@@ -199,10 +176,6 @@ struct EdrCell {
                                                  float, float, float eps2) {
         const float s = (d2 < eps2) ? -2.f : -1.f;
         return min3f(__fadd_rn(dg, s), up, left);
-    }
-    __device__ __forceinline__ static float term(float d2, float eps2) { return (d2 < eps2) ? -2.f : -1.f; }
-    __device__ __forceinline__ static float comb(float dg, float up, float left, float t, float, float) {
-        return min3f(__fadd_rn(dg, t), up, left);
     }
 };
 
@@ -212,7 +185,6 @@ struct EdrCell {
 template <bool EXACT>
 struct LcssCell {
     static constexpr bool kGap = false;
-    static constexpr bool kPackedSmem = true;  // f32x2 difference with shared-memory columns (see d2nr)
     __device__ __forceinline__ static float corner() { return 0.f; }
     __device__ __forceinline__ static float rowb(float, int) { return 0.f; }
     __device__ __forceinline__ static float topb(float, int) { return 0.f; }
@@ -220,10 +192,6 @@ struct LcssCell {
                                                  float, float, float eps2) {
         float m = (d2 < eps2) ? 1.f : 0.f;
         return max3f(__fadd_rn(dg, m), up, left);
-    }
-    __device__ __forceinline__ static float term(float d2, float eps2) { return (d2 < eps2) ? 1.f : 0.f; }
-    __device__ __forceinline__ static float comb(float dg, float up, float left, float t, float, float) {
-        return max3f(__fadd_rn(dg, t), up, left);
     }
 };
 

@@ -5,6 +5,12 @@
 
 namespace tsm_k {
 
+const void* dp_matrix_lane(int measure, bool exact) {
+    if (!exact) return dp_matrix_lane_fast(measure);
+    return measure == TSM_DTW ? (const void*)&tsm::dp_matrix_lane_kernel<tsm::DTW, 8, true>
+                              : (const void*)&tsm::dp_matrix_lane_kernel<tsm::DFRECHET, 8, true>;
+}
+
 const void* dp_matrix(int measure, int R, bool exact) {
     if (!exact) return dp_matrix_fast(measure, R);
     TSM_DP_MATRIX_TABLE(tsm::dp_matrix_kernel, true, measure, R)

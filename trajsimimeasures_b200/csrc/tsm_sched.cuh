@@ -197,7 +197,7 @@ __device__ __forceinline__ void group_task(const PairsArgs& A, int first, int co
 #pragma unroll
                     for (int r = 0; r < R; ++r) {
                         const float left = Din[r];
-                        const float nv = C::cell(dg, up, left, d2nr<true>(rn[r], c), rg[r], gc, p.eps2);
+                        const float nv = C::cell(dg, up, left, d2nr(rn[r], c), rg[r], gc, p.eps2);
                         Dout[r] = nv;
                         dg = left;
                         up = nv;

@@ -12,17 +12,16 @@
 // Pairs mode: every thread has its own pair (rows = longer trajectory,
 // columns = shorter, which keeps the boundary row short).  Matrix mode: a CTA
 // owns one query trajectory Q_i, staged once in shared memory as the columns,
-// and each thread takes one database trajectory D_j as its rows; database
-// trajectories are visited in the caller's order (sorted by length, the 32
-// lanes of a warp have near-equal row counts and the column loop is uniform).
+// and two threads (one for short queries) take one database trajectory D_j as
+// its rows; database trajectories are visited in the caller's order (sorted by
+// length, the lanes of a warp have near-equal row counts and the column loop is
+// uniform).
 //
 // Reference kernels replaced: core/dtw.py:10-53, core/edr.py:10-52,
 // core/lcss.py:12-53, core/erp.py:10-91, core/discret_frechet.py:9-50 (one
 // CUDA block per pair, 64 threads, an FP64 3-diagonal ring in global memory
 // and a __syncthreads per anti-diagonal), core/hausdorff.py:12-93.
 #pragma once
-
-#include <type_traits>
 
 #include "tsm_bits.cuh"
 #include "tsm_device.cuh"
@@ -60,7 +59,7 @@ __device__ __forceinline__ float4 col4(const SmemCols& c, int j, const KParams&,
 
 // R consecutive rows of a pair's DP: their points (negated, for d2nr), their
 // ERP gap distances and their current DP values, all in registers.
-template <class C, int R, bool EXACT, bool PACKED = true>
+template <class C, int R, bool EXACT>
 struct RowBlock {
     float2 n[R];
     float g[R], D[R];
@@ -85,7 +84,7 @@ struct RowBlock {
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const float left = D[r];
-            const float nv = C::cell(dg, up, left, d2nr<PACKED>(n[r], make_float2(c.x, c.y)), g[r], c.z, eps2);
+            const float nv = C::cell(dg, up, left, d2nr(n[r], make_float2(c.x, c.y)), g[r], c.z, eps2);
             D[r] = nv;
             dg = left;
             up = nv;
@@ -102,7 +101,7 @@ struct RowBlock {
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const float left = Din[r];
-            const float nv = C::cell(dg, up, left, d2nr<PACKED>(n[r], make_float2(c.x, c.y)), g[r], c.z, eps2);
+            const float nv = C::cell(dg, up, left, d2nr(n[r], make_float2(c.x, c.y)), g[r], c.z, eps2);
             Dout[r] = nv;
             dg = left;
             up = nv;
@@ -118,13 +117,6 @@ struct RowBlock {
         return v;
     }
 };
-
-// The f32x2 form of the cell distance (d2nr): always with per-lane global
-// columns, per measure (C::kPackedSmem) with shared-memory columns.
-template <class C, class Cols>
-constexpr bool kPacked() {
-    return std::is_same<Cols, SmemCols>::value ? C::kPackedSmem : true;
-}
 
 // The DP of one pair, prefetching form (dp_pair's default).  rowp/nr: row
 // trajectory; cols/nc: column trajectory; buf: this thread's boundary row
@@ -148,15 +140,13 @@ constexpr bool kPacked() {
 // 17.6 ms, ERP 18.86 -> 23.96 ms on B200, bit-identical results.)
 template <int M, int R, bool EXACT, class Cols>
 __device__ __forceinline__ float dp_pair_prefetch(const float2* __restrict__ rowp, int nr, const Cols& cols,
-                                                  int nc, float* buf, const KParams& p, float srow, float scol,
-                                                  int rb0 = 0) {
+                                                  int nc, float* buf, const KParams& p, float srow, float scol) {
     using C = typename CellOf<M, EXACT>::type;
-    if (rb0 == 0)  // else buf holds row rb0 - 1 (after four-block passes)
-        for (int j = 0; j < nc; ++j) buf[32 * j] = C::topb(scol, j);
+    for (int j = 0; j < nc; ++j) buf[32 * j] = C::topb(scol, j);
     float dlast = 0.f;
-    int rb = rb0;
+    int rb = 0;
     for (; nr - rb > R; rb += 2 * R) {
-        RowBlock<C, R, EXACT, kPacked<C, Cols>()> hi, lo;
+        RowBlock<C, R, EXACT> hi, lo;
         hi.load(rowp, rb, nr, srow, p);
         lo.load(rowp, rb + R, nr, srow, p);
         float HA[R], HB[R], LA[R], LB[R];
@@ -216,7 +206,7 @@ __device__ __forceinline__ float dp_pair_prefetch(const float2* __restrict__ row
         buf[32 * (nc - 1)] = lb;
     }
     if (rb < nr) {  // last rows (at most R): one block
-        RowBlock<C, R, EXACT, kPacked<C, Cols>()> blk;
+        RowBlock<C, R, EXACT> blk;
         blk.load(rowp, rb, nr, srow, p);
         float diag = (rb == 0) ? C::corner() : C::rowb(srow, rb - 1);
         float4 cn = col4<EXACT>(cols, 0, p, C::kGap);
@@ -235,176 +225,123 @@ __device__ __forceinline__ float dp_pair_prefetch(const float2* __restrict__ row
     return dlast;
 }
 
-// Four-block pass (used for ERP, whose cells wait on a MUFU square root and a
-// three-way min of sums): rows rb .. rb + 4R - 1 as four blocks of R rows, block k
-// computing column s - k at step s, so a thread carries four independent
-// dependency chains instead of two, and reads and writes the boundary row
-// once per 4R rows.  Block k takes its top and diagonal values from the
-// bottom values of block k - 1 at the previous two steps; block 0 from the
-// boundary row; block 3 writes the boundary row.  Column results alternate
-// between two arrays per block (even columns in A, odd in B: no register
-// moves).  Needs nc >= 4; the cells and their order along each dependency
-// chain are those of the two-block pass, so the values are identical.
-// Returns the value of row nr - 1 at column nc - 1 when it lies in this pass.
-template <class C, int R, bool EXACT, bool PK, class Cols>
-__device__ __forceinline__ float quad_pass(const float2* __restrict__ rowp, int rb, int nr, const Cols& cols,
-                                           int nc, float* buf, const KParams& p, float srow) {
-    RowBlock<C, R, EXACT, PK> k0, k1, k2, k3;
-    k0.load(rowp, rb, nr, srow, p);
-    k1.load(rowp, rb + R, nr, srow, p);
-    k2.load(rowp, rb + 2 * R, nr, srow, p);
-    k3.load(rowp, rb + 3 * R, nr, srow, p);
-    float A0[R], B0[R], A1[R], B1[R], A2[R], B2[R], A3[R], B3[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {  // column -1 (the row borders) in the odd arrays
-        B0[r] = k0.D[r];
-        B1[r] = k1.D[r];
-        B2[r] = k2.D[r];
-        B3[r] = k3.D[r];
-    }
-    const float e2 = p.eps2;
-    // bottom values of blocks 0..2: at the last column computed (cur) and the one before (prv)
-    float c0 = C::rowb(srow, rb + R - 1), p0 = c0;
-    float c1 = C::rowb(srow, rb + 2 * R - 1), p1 = c1;
-    float c2 = C::rowb(srow, rb + 3 * R - 1), p2 = c2;
-    float d0 = (rb == 0) ? C::corner() : C::rowb(srow, rb - 1);  // block 0's diagonal: boundary row, column - 1
-    // columns of the four blocks: cs0 = column s, cs1 = s - 1, ...
-    float4 cs0 = col4<EXACT>(cols, 0, p, C::kGap), cs1 = cs0, cs2 = cs0, cs3 = cs0;
-    float t0 = buf[0];
-    // block 0 at column s (its result into O0 from I0); shifts its bottom values
-    auto blk0 = [&](const float (&I)[R], float (&O)[R], int s) {
-        const float nb = k0.step2(I, O, cs0, t0, d0, e2);
-        d0 = t0;
-        p0 = c0;
-        c0 = nb;
-    };
-    auto blk1 = [&](const float (&I)[R], float (&O)[R]) {
-        const float nb = k1.step2(I, O, cs1, c0, p0, e2);
-        p1 = c1;
-        c1 = nb;
-    };
-    auto blk2 = [&](const float (&I)[R], float (&O)[R]) {
-        const float nb = k2.step2(I, O, cs2, c1, p1, e2);
-        p2 = c2;
-        c2 = nb;
-    };
-    auto blk3 = [&](const float (&I)[R], float (&O)[R], int j) { buf[32 * j] = k3.step2(I, O, cs3, c2, p2, e2); };
-    // next step's columns: shift, and load column s for block 0 (and its top value)
-    auto advance = [&](int s) {
-        cs3 = cs2;
-        cs2 = cs1;
-        cs1 = cs0;
-        if (s < nc) {
-            cs0 = col4<EXACT>(cols, s, p, C::kGap);
-            t0 = buf[32 * s];
-        }
-    };
-    // prologue: steps 0, 1, 2 (blocks below start one step later each); bottom-up within a step
-    blk0(B0, A0, 0);
-    advance(1);
-    blk1(B1, A1);
-    blk0(A0, B0, 1);
-    advance(2);
-    blk2(B2, A2);
-    blk1(A1, B1);
-    blk0(B0, A0, 2);
-    advance(3);
-    // steady state: steps s = 3 .. nc - 1, all four blocks; s odd: blocks 0, 2 write B, blocks 1, 3 write A
-    int s = 3;
-    for (; s + 1 < nc; s += 2) {
-        blk3(B3, A3, s - 3);
-        blk2(A2, B2);
-        blk1(B1, A1);
-        blk0(A0, B0, s);
-        advance(s + 1);
-        blk3(A3, B3, s - 2);
-        blk2(B2, A2);
-        blk1(A1, B1);
-        blk0(B0, A0, s + 1);
-        advance(s + 2);
-    }
-    const int rr = nr - 1 - (rb + 3 * R);  // the last row's index in block 3 when this pass holds it
-    float dlast = 0.f;
-    if (s < nc) {  // one more full step (s odd), then the drain from an even step
-        blk3(B3, A3, s - 3);
-        blk2(A2, B2);
-        blk1(B1, A1);
-        blk0(A0, B0, s);
-        advance(s + 1);
-        ++s;
-        // drain: s = nc (even): block 3 column nc - 3 (odd -> B), block 2 nc - 2 (even -> A), block 1 nc - 1 (odd -> B)
-        blk3(A3, B3, s - 3);
-        blk2(B2, A2);
-        blk1(A1, B1);
-        advance(s + 1);
-        blk3(B3, A3, s - 2);  // column nc - 2 (even)
-        blk2(A2, B2);         // column nc - 1 (odd)
-        advance(s + 2);
-        blk3(A3, B3, s - 1);  // column nc - 1 (odd)
-        if (rr < R) {
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                if (r == rr) dlast = B3[r];
-        }
-    } else {  // s = nc (odd): block 3 column nc - 3 (even -> A), block 2 nc - 2 (odd -> B), block 1 nc - 1 (even -> A)
-        blk3(B3, A3, s - 3);
-        blk2(A2, B2);
-        blk1(B1, A1);
-        advance(s + 1);
-        blk3(A3, B3, s - 2);  // column nc - 2 (odd)
-        blk2(B2, A2);         // column nc - 1 (even)
-        advance(s + 2);
-        blk3(B3, A3, s - 1);  // column nc - 1 (even)
-        if (rr < R) {
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                if (r == rr) dlast = A3[r];
-        }
-    }
-    return dlast;
-}
-
-template <int M, int R, bool EXACT, class Cols>
-__device__ __forceinline__ float dp_pair_quad(const float2* __restrict__ rowp, int nr, const Cols& cols, int nc,
-                                              float* buf, const KParams& p, float srow, float scol) {
-    using C = typename CellOf<M, EXACT>::type;
-    if (nc < 4 || nr <= 3 * R) return dp_pair_prefetch<M, R, EXACT>(rowp, nr, cols, nc, buf, p, srow, scol);
-    for (int j = 0; j < nc; ++j) buf[32 * j] = C::topb(scol, j);
-    int rb = 0;
-    float dlast = 0.f;
-    for (; nr - rb > 3 * R; rb += 4 * R)
-        dlast = quad_pass<C, R, EXACT, kPacked<C, Cols>()>(rowp, rb, nr, cols, nc, buf, p, srow);
-    if (rb >= nr) return dlast;
-    return dp_pair_prefetch<M, R, EXACT>(rowp, nr, cols, nc, buf, p, srow, scol, rb);
-}
-
-// The DP of one pair (DTW, ERP, discrete Frechet): with shared-memory columns
-// (the matrix kernels) the four-block pass for ERP (kQuadPass), else the
-// prefetching one.  Measured on B200, all-pairs 2000 x 2000: ERP 18.84 ->
-// 18.05 ms with four blocks of 8 rows; DTW 15.29 -> 15.69 ms (four blocks of
-// 8) and 16.17 ms (of 4), so DTW keeps two blocks.  The four-block pass stays
-// out of the scheduled kernel: compiled into its ERP tile tasks it raised the
-// whole kernel from 127 to 190 registers, and the 500k-pair uneven batch from
-// 5.1 to 6.5 ms.  Also measured slower, bit-identical: the square roots one
-// column ahead of the recurrence (DTW 15.17 -> 16.02, ERP 18.05 -> 19.84,
-// Frechet 12.33 -> 12.94), the lower block first (DTW and ERP 25-30 %), and
-// the squared distances of two rows packed in f32x2 (DTW 15.2 -> 19.0, ERP
-// 18.1 -> 20.5, Frechet 12.35 -> 15.6: an f32x2 instruction holds the pipe and
-// the issue port as long as two scalar ones).
-#ifndef TSM_QUAD_PASS
-#define TSM_QUAD_PASS 1
-#endif
-constexpr bool kQuadPass = TSM_QUAD_PASS != 0;
+// The DP of one pair (DTW, ERP, discrete Frechet), one lane.
 template <int M, int R, bool EXACT, class Cols>
 __device__ __forceinline__ float dp_pair(const float2* __restrict__ rowp, int nr, const Cols& cols,
                                          int nc, float* buf, const KParams& p, float srow, float scol) {
     if (nr <= 0 || nc <= 0) return 0.f;
-    if constexpr (kQuadPass && M == ERP && R <= 8 && std::is_same<Cols, SmemCols>::value) {
-        // (16 rows: four blocks spill)
-        return dp_pair_quad<M, R, EXACT>(rowp, nr, cols, nc, buf, p, srow, scol);
-    } else {
-        return dp_pair_prefetch<M, R, EXACT>(rowp, nr, cols, nc, buf, p, srow, scol);
+    return dp_pair_prefetch<M, R, EXACT>(rowp, nr, cols, nc, buf, p, srow, scol);
+}
+
+// The DP of a pair by two lanes (lanes 2 q and 2 q + 1 of a warp, all 32 lanes
+// together; nc uniform, nr the pair's own), columns in shared memory.  Rows go
+// in strips of 2 R, lane u = 0, 1 taking rows u R .. u R + R - 1 of a strip and
+// column s - u at step s: lane 1's top values come from lane 0 by a shuffle, lane
+// 0's from the boundary row, which lane 1 rewrites one column behind.  The
+// boundary row is shared by two lanes (element j at ring[16 * j]), half the
+// shared memory of a pair per lane, so 16 warps fit an SM where 8 did with a
+// pair per lane: on a chain of cells alone 2 warps per scheduler take 11.1
+// cycles a cell, 4 take 9.1, against the square root's 8 (its unit's rate).
+// Strips are of 2 R rows while more than R are left to some pair of the warp,
+// then of R (the sweep of rows that are not there is what long blocks cost).
+//
+// Measured on B200, all-pairs 2000 x 2000 of 20..200 points, ms, against one
+// lane per pair (two, for ERP four, blocks of 8 rows a lane), same bits: DTW 15.2
+// -> 13.9, ERP 18.1 -> 17.1, Frechet 12.3 -> 11.6.  R = 16: 14.0, 17.3 (3 CTAs'
+// registers; 18.3 and 20.7 in 168 and 128), 11.5; R = 4: 16.9, 19.7, 14.1.  The
+// launch bound of 4 CTAs gives ptxas the registers that the shared memory allows
+// (without it DTW 14.1, ERP 19.9; with 6 CTAs 16.6, 20.0, 12.6).  Tried on one
+// lane per pair, slower, same bits: the square roots one column ahead of the
+// recurrence (DTW 15.2 -> 16.0, ERP 18.1 -> 19.8), the lower block first (25 %),
+// the squared distances of two rows packed in f32x2 (19.0, 20.5, Frechet 15.6:
+// an f32x2 instruction holds the pipe and the issue port as long as two scalar
+// ones).
+// cols.p[-1] .. cols.p[nc + 1] and ring[0 .. 16 (nc + 1)] are loaded (the values
+// past the ends are not used).  The cells are dp_pair_prefetch's.
+__host__ __device__ constexpr int duo_ring(int cap) { return 16 * (cap + 2); }  // floats per warp
+
+// One strip, rows rb .. rb + 2 R - 1.  Sets dlast to D(nr - 1, nc - 1) in the
+// lane that holds row nr - 1, and mine there, if the strip has that row.
+template <int M, int R, bool EXACT>
+__device__ __forceinline__ void duo_strip(const float2* __restrict__ rowp, int nr, const SmemCols& cols, int nc,
+                                          float* ring, const KParams& p, float srow, int u, int rb, float& dlast,
+                                          bool& mine) {
+    using C = typename CellOf<M, EXACT>::type;
+    constexpr unsigned kFull = 0xffffffffu;
+    const int row0 = rb + u * R;
+    const int lr = nr - 1 - row0;  // the last row, if it is in this lane's block
+    const bool last = lr >= 0 && lr < R;
+    RowBlock<C, R, EXACT> blk;
+    if (nr > 0) blk.load(rowp, row0, nr, srow, p);
+    float A[R], B[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) A[r] = blk.D[r];
+    const float diag0 = row0 == 0 ? C::corner() : C::rowb(srow, row0 - 1);
+    float diag = diag0, bottom = 0.f;
+    const float4* cp = cols.p - u;  // this lane's column of step 0
+    float* rp = ring;
+    float4 c = cp[0];
+    float t = rp[0];
+    // step s with cp and rp at step s - k: the next step's column and (for lane 0) top value are loaded first
+    auto step = [&](const float (&Di)[R], float (&Do)[R], int k) {
+        const float above = __shfl_up_sync(kFull, bottom, 1);
+        const float top = u ? above : t;
+        const float4 cc = c;
+        c = cp[k + 1];
+        t = rp[16 * (k + 1)];
+        bottom = blk.step2(Di, Do, cc, top, diag, p.eps2);
+        diag = top;
+    };
+    auto pick = [&](const float (&D)[R]) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (r == lr) dlast = D[r];
+        mine = true;
+    };
+    step(A, B, 0);
+    if (u) {  // lane 1 starts at step 1
+        diag = diag0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) B[r] = A[r];
     }
+    int s = 1;
+    for (; s + 1 < nc; s += 2, cp += 2, rp += 32) {
+        step(B, A, 1);
+        if (u) rp[0] = bottom;
+        step(A, B, 2);
+        if (u) rp[16] = bottom;
+    }
+    if (s < nc) {
+        step(B, A, 1);
+        if (u) rp[0] = bottom;
+        if (last && u == 0) pick(A);
+        step(A, B, 2);
+        if (u) rp[16] = bottom;
+        if (last && u == 1) pick(B);
+    } else {
+        if (last && u == 0) pick(B);
+        step(B, A, 1);
+        if (u) rp[0] = bottom;
+        if (last && u == 1) pick(A);
+    }
+    __syncwarp();
+}
+template <int M, int R, bool EXACT>
+__device__ __forceinline__ float dp_duo(const float2* __restrict__ rowp, int nr, const SmemCols& cols, int nc,
+                                        float* ring, const KParams& p, float srow, float scol, int u, bool& mine) {
+    using C = typename CellOf<M, EXACT>::type;
+    float dlast = 0.f;
+    mine = u == 0 && (nr <= 0 || nc <= 0);
+    if (nc <= 0) return dlast;
+    for (int j = u; j < nc; j += 2) ring[16 * j] = C::topb(scol, j);
+    const int most = __reduce_max_sync(0xffffffffu, nr);
+    __syncwarp();
+    int rb = 0;
+    for (; most - rb > (R > 4 ? R : 0); rb += 2 * R)
+        duo_strip<M, R, EXACT>(rowp, nr, cols, nc, ring, p, srow, u, rb, dlast, mine);
+    if constexpr (R > 4)
+        if (rb < most) duo_strip<M, R / 2, EXACT>(rowp, nr, cols, nc, ring, p, srow, u, rb, dlast, mine);
+    return dlast;
 }
 
 // The EDR or LCSS count of one pair per lane (na, nb < 0: none), the whole
@@ -494,21 +431,23 @@ __global__ void __launch_bounds__(128) dp_pairs_kernel(
 // query i (row i, whatever the processing order q_order), and slot t of query i
 // goes to out[i, t].  A database index outside 0..d_total-1 gives NaN.
 // (EDR and LCSS: bits_matrix_kernel, tsm_bits.cuh.)
-// Dynamic shared memory = cap float4 columns + W*32*cap floats.
+// Dynamic shared memory = cap + 3 float4 columns + W * duo_ring(cap) floats.
 
 template <int M, int R, bool EXACT>
-__global__ void __launch_bounds__(128) dp_matrix_kernel(
+__global__ void __launch_bounds__(128, 4) dp_matrix_kernel(
     const float2* __restrict__ q_pts, const int64_t* __restrict__ q_off, const int32_t* __restrict__ q_len,
     const int32_t* __restrict__ q_order, const float2* __restrict__ d_pts, const int64_t* __restrict__ d_off,
     const int32_t* __restrict__ d_len, const int32_t* __restrict__ d_order, int64_t nd, int64_t d_total, int chunks,
     int sym, int cap, int d_max_len, KParams p, float* __restrict__ out, int64_t ld) {
     extern __shared__ float smem[];
     __shared__ float s_scol;
-    float4* cols = reinterpret_cast<float4*>(smem);
-    float* buf = smem + 4 * cap + (threadIdx.x >> 5) * (32 * cap) + (threadIdx.x & 31);
+    float4* cols = reinterpret_cast<float4*>(smem) + 1;
+    const int u = threadIdx.x & 1;
+    float* ring = smem + 4 * (cap + 3) + (threadIdx.x >> 5) * duo_ring(cap) + ((threadIdx.x & 31) >> 1);
     const int64_t qs = blockIdx.x / chunks;
     const int chunk = blockIdx.x % chunks;
-    if (sym == 1 && (int64_t)(chunk + 1) * blockDim.x <= qs) return;  // below the diagonal (uniform per CTA)
+    const int per = blockDim.x >> 1;  // slots per CTA
+    if (sym == 1 && (int64_t)(chunk + 1) * per <= qs) return;  // below the diagonal (uniform per CTA)
     const int64_t qi = q_order ? (int64_t)q_order[qs] : qs;
     const int nq = q_len[qi];
     const bool qbad = nq < 0 || nq > cap;
@@ -528,6 +467,55 @@ __global__ void __launch_bounds__(128) dp_matrix_kernel(
         }
         __syncthreads();
     }
+    const int64_t slot = (int64_t)chunk * per + (threadIdx.x >> 1);
+    const bool mine = slot < nd && !(sym == 1 && slot < qs);  // (the whole warp runs dp_duo)
+    const int64_t dj = !mine ? -1 : d_order ? (int64_t)d_order[(sym == 2 ? qi * nd : 0) + slot] : slot;
+    const bool dbad = dj < 0 || dj >= d_total;
+    int ndl = dbad ? -1 : d_len[dj];
+    const bool bad = qbad || ndl < 0 || ndl > d_max_len;
+    if (bad) ndl = 0;
+    const float2* dp = bad ? d_pts : d_pts + d_off[dj];
+    float srow = 0.f, scol = 0.f;
+    if constexpr (M == ERP) {
+        srow = gapsum<EXACT>(dp, ndl, p);
+        scol = s_scol;
+    }
+    bool last;  // this lane has the pair's result
+    const float dl = dp_duo<M, R, EXACT>(dp, ndl, SmemCols{cols}, qbad ? 0 : nq, ring, p, srow, scol, u, last);
+    if (!mine || !last) return;
+    float o = CUDART_NAN_F;
+    int c;
+    if (!bad) finalize<M>(dl, nq, ndl, o, c);
+    out[qi * ld + (sym == 2 ? slot : dj)] = o;
+    if (sym == 1 && dj != qi) out[dj * ld + qi] = o;
+}
+
+// The same with one lane per pair, for short queries (DTW and discrete
+// Frechet): a pair's fixed work is then paid in one lane, not two.  Dynamic
+// shared memory = cap float4 columns + W*32*cap floats.
+template <int M, int R, bool EXACT>
+__global__ void __launch_bounds__(128) dp_matrix_lane_kernel(
+    const float2* __restrict__ q_pts, const int64_t* __restrict__ q_off, const int32_t* __restrict__ q_len,
+    const int32_t* __restrict__ q_order, const float2* __restrict__ d_pts, const int64_t* __restrict__ d_off,
+    const int32_t* __restrict__ d_len, const int32_t* __restrict__ d_order, int64_t nd, int64_t d_total, int chunks,
+    int sym, int cap, int d_max_len, KParams p, float* __restrict__ out, int64_t ld) {
+    extern __shared__ float smem[];
+    float4* cols = reinterpret_cast<float4*>(smem);
+    float* buf = smem + 4 * cap + (threadIdx.x >> 5) * (32 * cap) + (threadIdx.x & 31);
+    const int64_t qs = blockIdx.x / chunks;
+    const int chunk = blockIdx.x % chunks;
+    if (sym == 1 && (int64_t)(chunk + 1) * blockDim.x <= qs) return;  // below the diagonal (uniform per CTA)
+    const int64_t qi = q_order ? (int64_t)q_order[qs] : qs;
+    const int nq = q_len[qi];
+    const bool qbad = nq < 0 || nq > cap;
+    if (!qbad) {
+        const float2* qp = q_pts + q_off[qi];
+        for (int j = threadIdx.x; j < nq; j += blockDim.x) {
+            const float2 v = __ldg(qp + j);
+            cols[j] = make_float4(v.x, v.y, 0.f, 0.f);
+        }
+    }
+    __syncthreads();
     const int64_t slot = (int64_t)chunk * blockDim.x + threadIdx.x;
     if (slot >= nd || (sym == 1 && slot < qs)) return;
     const int64_t dj = d_order ? (int64_t)d_order[(sym == 2 ? qi * nd : 0) + slot] : slot;
@@ -541,12 +529,7 @@ __global__ void __launch_bounds__(128) dp_matrix_kernel(
         return;
     }
     const float2* dp = d_pts + d_off[dj];
-    float srow = 0.f, scol = 0.f;
-    if constexpr (M == ERP) {
-        srow = gapsum<EXACT>(dp, ndl, p);
-        scol = s_scol;
-    }
-    const float dl = dp_pair<M, R, EXACT>(dp, ndl, SmemCols{cols}, nq, buf, p, srow, scol);
+    const float dl = dp_pair<M, R, EXACT>(dp, ndl, SmemCols{cols}, nq, buf, p, 0.f, 0.f);
     float o;
     int c;
     finalize<M>(dl, nq, ndl, o, c);

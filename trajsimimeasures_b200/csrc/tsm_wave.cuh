@@ -106,7 +106,7 @@ __device__ __forceinline__ void wave_pair(const float2* __restrict__ rowp, const
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
                     const float left = Din[r];
-                    const float nv = C::cell(dg, up, left, d2nr<C::kPackedSmem>(rn[r], c), rg[r], cg, p.eps2);
+                    const float nv = C::cell(dg, up, left, d2nr(rn[r], c), rg[r], cg, p.eps2);
                     Dout[r] = nv;
                     dg = left;
                     up = nv;
