@@ -229,6 +229,16 @@ int tsm_pairs_sched_noalloc(const float* pts, const int64_t* off_a, const int32_
                             int32_t max_len, int32_t warp_smem_floats, const tsm_params* params, float* out,
                             int32_t* out_counts, int64_t out_stride, void* stream);
 
+/* Processing order for tsm_pairs: order[0 .. n_pairs - 1] = the pair indices,
+ * grouped by the shape of their DP (steps of 8 points on both sides up to 256,
+ * of an eighth of an octave above), the largest first; inside a group in any order.
+ * The reference processes a batch in its given order (core/dtw.py:69-72);
+ * results do not depend on it.  len_a / len_b int32 [n_pairs] (any values),
+ * order int32 [n_pairs], workspace tsm_pair_order_workspace_bytes() bytes, all
+ * device memory.  Stream-ordered. */
+int tsm_pair_order_workspace_bytes(void);
+int tsm_pair_order(const int32_t* len_a, const int32_t* len_b, int64_t n_pairs, int32_t* order, void* workspace,
+                   void* stream);
 /*
  * Row-wise k smallest (kNN result lists): for each row r < n_rows of the
  * float32 matrix d (row stride ld), the k smallest values in ascending order,

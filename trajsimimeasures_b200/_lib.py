@@ -26,7 +26,8 @@ EXPORTS = ("tsm_version", "tsm_last_error", "tsm_max_supported_len", "tsm_matrix
            "tsm_select_rows", "tsm_allpairs_sym", "tsm_matrix_gather", "tsm_enc_embed_workspace_bytes",
            "tsm_enc_embed", "tsm_enc_embed_status", "tsm_enc_train_status", "tsm_enc_embed_opts",
            "tsm_enc_loss_grad_w", "tsm_scan_dim",
-           "tsm_scan_image_bytes", "tsm_scan_prepare", "tsm_scan", "tsm_scan_opts")
+           "tsm_scan_image_bytes", "tsm_scan_prepare", "tsm_scan", "tsm_scan_opts", "tsm_pair_order",
+           "tsm_pair_order_workspace_bytes")
 
 
 class TsmParams(ctypes.Structure):
@@ -119,6 +120,9 @@ def load():
                                       _i64, _vp]
         lib.tsm_select_rows.restype = ctypes.c_int
         lib.tsm_select_rows.argtypes = [_vp, _i64, _i64, _i64, _i64, _vp, _vp]
+        lib.tsm_pair_order_workspace_bytes.restype = ctypes.c_int
+        lib.tsm_pair_order.restype = ctypes.c_int
+        lib.tsm_pair_order.argtypes = [_vp, _vp, _i64, _vp, _vp, _vp]
         lib.tsm_topk_rows.restype = ctypes.c_int
         lib.tsm_topk_rows.argtypes = [_vp, _i64, _i64, _i64, _i32, _vp, _vp, _vp]
         _lib = lib

@@ -429,7 +429,7 @@ def _matrix_into(m, qs, ds, out, cnt, *, eps, gpoint, exact, rows, stream=None):
         o = torch.empty(nd, dtype=torch.float32, device=dev)
         c = torch.empty(nd, dtype=torch.int32, device=dev) if cnt is not None else None
         pairs_raw(m, pool, off_a, len_a, ds.off, ds.lens, max(qs.max_len, ds.max_len), out=o, counts=c,
-                  order=engine.pair_order_dev(len_a, ds.lens), eps=eps, gpoint=shift_gpoint(gpoint, origin),
+                  order=engine.pair_order_dev(len_a, ds.lens, stream=stream), eps=eps, gpoint=shift_gpoint(gpoint, origin),
                   exact=exact, rows=rows, stream=stream)
         out[int(i)] = o
         if cnt is not None:

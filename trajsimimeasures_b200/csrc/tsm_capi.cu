@@ -15,6 +15,7 @@
 #include "tsm_bits.cuh"
 #include "tsm_haus.cuh"
 #include "tsm_kernels.h"
+#include "tsm_order.cuh"
 #include "tsm_sched.cuh"
 #include "tsm_tile.cuh"
 #include "tsm_topk.cuh"
@@ -474,6 +475,27 @@ int tsm_allpairs_sym(int measure, const float* pts, const int64_t* off, const in
     if (max_len < 0) return fail(TSM_EINVAL, "tsm_allpairs_sym: max_len < 0");
     return matrix_launch("tsm_allpairs_sym", measure, pts, off, len, order, n, max_len, pts, off, len, order, n,
                          n, max_len, 1, params, out, ld_out, out_counts, stream);
+}
+
+int tsm_pair_order_workspace_bytes(void) { return tsm::kOrderInts * 4; }
+
+int tsm_pair_order(const int32_t* len_a, const int32_t* len_b, int64_t n_pairs, int32_t* order, void* workspace,
+                   void* stream) {
+    g_err.clear();
+    if (n_pairs < 0) return fail(TSM_EINVAL, "tsm_pair_order: n_pairs < 0");
+    if (n_pairs == 0) return TSM_OK;
+    if (n_pairs > 0x7fffffffLL) return fail(TSM_EINVAL, "tsm_pair_order: a pair index exceeds int32");
+    if (!len_a || !len_b || !order || !workspace) return fail(TSM_EINVAL, "tsm_pair_order: null pointer");
+    cudaStream_t s = (cudaStream_t)stream;
+    int* ws = static_cast<int*>(workspace);
+    cudaError_t e = cudaMemsetAsync(ws, 0, tsm::kOrderInts * 4, s);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
+    const int64_t want = (n_pairs + 4 * tsm::kOrderThreads - 1) / (4 * tsm::kOrderThreads);
+    const unsigned grid = (unsigned)(want < 148 ? want : 148);
+    tsm::order_count<<<grid, tsm::kOrderThreads, 0, s>>>(len_a, len_b, n_pairs, ws);
+    tsm::order_scatter<<<grid, tsm::kOrderThreads, 0, s>>>(len_a, len_b, n_pairs, ws, order);
+    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "tsm_pair_order launch");
+    return TSM_OK;
 }
 
 int tsm_topk_rows(const float* d, int64_t n_rows, int64_t n_cols, int64_t ld, int32_t k, float* out_d,

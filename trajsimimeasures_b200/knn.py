@@ -105,7 +105,7 @@ def knn_rerank(Q: TrajSet, D: TrajSet, cand: torch.Tensor, k=10, measure="dtw", 
         dd = torch.empty(nq * c, dtype=torch.float32, device=Q.device)
         pairs_raw(m, pool, off_a, len_a, off_b, len_b, max(Q.max_len, D.max_len), out=dd, eps=eps,
                   gpoint=shift_gpoint(gpoint, same_origin(Q, D)), exact=exact, stream=stream,
-                  order=shape_order(len_a, len_b))
+                  order=shape_order(len_a, len_b, stream=stream))
         dd = dd.view(nq, c)
     # ties to the smaller database index, as in knn_exhaustive
     o = torch.argsort(cand, dim=1)
@@ -115,11 +115,11 @@ def knn_rerank(Q: TrajSet, D: TrajSet, cand: torch.Tensor, k=10, measure="dtw", 
     return v, torch.gather(ci, 1, j.long())
 
 
-def shape_order(len_a: torch.Tensor, len_b: torch.Tensor, rows=DEFAULT_ROWS) -> torch.Tensor:
+def shape_order(len_a: torch.Tensor, len_b: torch.Tensor, rows=DEFAULT_ROWS, stream=None) -> torch.Tensor:
     """engine.pair_order on the device: the pairs ordered by (row blocks,
     columns) of their DP, the largest first, so a warp's 32 lanes run loops of
     equal trip counts (int32 processing order for tsm_pairs)."""
-    return pair_order_dev(len_a, len_b, rows)
+    return pair_order_dev(len_a, len_b, rows, stream)
 
 
 def recall_at_k(approx_idx, exact_idx) -> float:
