@@ -58,52 +58,82 @@ __global__ void enc_round_bf16(const float* __restrict__ p, __nv_bfloat16* __res
 // points: round(k (n - 1) / (NS - 1)), halves rounded up, in integers.
 __device__ __forceinline__ int skip_index(int k, int n) { return (2 * k * (n - 1) + (NS - 1)) / (2 * (NS - 1)); }
 
-// E[b][o] = bo[o] + sum_k Wo[o][k] hl[b][k] (bias first, k ascending) for
-// o < EO; E[b][EO + 2 k + i] = sc_k * coordinate i of resampled point k (the
+// E[b][EO + 2 k + i] = sc_k * coordinate i of resampled point k (the
 // normalised input at skip_index(k, n); 0 for an empty trajectory), the
 // geometric skip, written unscaled to X[b][2 k + i] too when X is given (the
-// training forward keeps it for the gradients of sc_k).  One thread per head
-// output o, HEAD_B trajectories per CTA, their hidden states staged in
-// shared memory; each W_o row is read once per CTA.
-constexpr int HEAD_B = 32;
+// training forward keeps it for the gradients of sc_k).  One thread per value:
+// each is a chain of three loads, which inside the head's few CTAs cost 28 us.
+__global__ void __launch_bounds__(256) enc_skip_fwd(int B, const float* __restrict__ p, float* __restrict__ E,
+                                                    const float2* __restrict__ pts, const int64_t* __restrict__ off,
+                                                    const int32_t* __restrict__ len, float4 nrm, float* __restrict__ X) {
+    const int64_t g = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    const int64_t b = g / SK;
+    const int q = g % SK;
+    if (b >= B) return;
+    const int n = len[b];
+    const float x = n > 0 ? xin(pts, off[b], n, skip_index(q >> 1, n), q & 1, nrm) : 0.f;
+    E[b * ED + EO + q] = expf(p[OFF_SC + (q >> 1)]) * x;
+    if (X) X[b * SK + q] = x;
+}
+
+// E[b][o] = bo[o] + sum_k Wo[o][k] hl[b][k] (bias first, k ascending) for o <
+// EO.  A CTA keeps W_o transposed in shared memory and takes blocks of HEAD_B
+// trajectories in turn, their hidden states staged there too: lane l outputs l,
+// l + 32, l + 64, l + 96 of its warp's HEAD_R trajectories, so that a 16-byte
+// load of hidden states (4 clocks, broadcast or not) feeds 16 FMAs.  (One
+// output a thread, W_o rows read from global memory, 32 lines a load: 0.33 ms
+// for 100,000 trajectories.)
+constexpr int HEAD_R = 16;
+constexpr int HEAD_B = 4 * HEAD_R;
+constexpr int HEAD_LD = EO + 1;  // row stride of the transposed W_o: no bank conflicts either way
+constexpr int HEAD_SMEM = (HEAD_B * HD + HD * HEAD_LD) * 4;
 __global__ void __launch_bounds__(EO) enc_head_fwd(const float* __restrict__ hl, int B, const float* __restrict__ p,
-                                                   float* __restrict__ E, const float2* __restrict__ pts,
-                                                   const int64_t* __restrict__ off, const int32_t* __restrict__ len,
-                                                   float4 nrm, float* __restrict__ X) {
-    __shared__ __align__(16) float hs[HEAD_B][HD];
-    const int o = threadIdx.x;
-    const int64_t b0 = (int64_t)blockIdx.x * HEAD_B;
-    for (int e = o; e < HEAD_B * SK; e += EO) {
-        const int64_t b = b0 + e / SK;
-        const int q = e % SK;
-        if (b < B) {
-            const int n = len[b];
-            const float x = n > 0 ? xin(pts, off[b], n, skip_index(q >> 1, n), q & 1, nrm) : 0.f;
-            E[b * ED + EO + q] = expf(p[OFF_SC + (q >> 1)]) * x;
-            if (X) X[b * SK + q] = x;
+                                                   float* __restrict__ E) {
+    extern __shared__ __align__(16) float head_sm[];
+    float* hs = head_sm;                 // [HEAD_B][HD]
+    float* wt = head_sm + HEAD_B * HD;   // [HD][HEAD_LD]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+#pragma unroll 8
+    for (int r = 0; r < EO; ++r) wt[tid * HEAD_LD + r] = __ldg(p + OFF_WO + r * HD + tid);
+    float bo[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) bo[i] = p[OFF_BO + lane + 32 * i];
+    for (int64_t b0 = (int64_t)blockIdx.x * HEAD_B; b0 < B; b0 += (int64_t)gridDim.x * HEAD_B) {
+        __syncthreads();  // W_o is staged; the last block's readers are done
+#pragma unroll 8
+        for (int e = tid; e < HEAD_B * HD; e += EO) {
+            const int64_t b = b0 + e / HD;
+            hs[e] = b < B ? hl[b * HD + e % HD] : 0.f;
+        }
+        __syncthreads();
+        float acc[4][HEAD_R];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < HEAD_R; ++j) acc[i][j] = bo[i];
+        const float* hw = hs + warp * HEAD_R * HD;
+        for (int k = 0; k < HD; k += 4) {
+            float w[4][4];
+#pragma unroll
+            for (int d = 0; d < 4; ++d)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) w[i][d] = wt[(k + d) * HEAD_LD + lane + 32 * i];
+#pragma unroll
+            for (int j = 0; j < HEAD_R; ++j) {
+                const float4 h = *reinterpret_cast<const float4*>(hw + j * HD + k);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    acc[i][j] = fmaf(w[i][3], h.w, fmaf(w[i][2], h.z, fmaf(w[i][1], h.y, fmaf(w[i][0], h.x, acc[i][j]))));
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < HEAD_R; ++j) {
+            const int64_t b = b0 + warp * HEAD_R + j;
+            if (b < B)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) E[b * ED + lane + 32 * i] = acc[i][j];
         }
     }
-    for (int e = o; e < HEAD_B * HD; e += EO) {
-        const int64_t b = b0 + e / HD;
-        hs[e / HD][e % HD] = b < B ? hl[b * HD + e % HD] : 0.f;
-    }
-    __syncthreads();
-    float acc[HEAD_B];
-    const float bo = p[OFF_BO + o];
-#pragma unroll
-    for (int j = 0; j < HEAD_B; ++j) acc[j] = bo;
-    const float* w = p + OFF_WO + o * HD;  // the caller's buffer: 4-byte alignment only
-    for (int k = 0; k < HD; k += 4) {
-        const float w0 = __ldg(w + k), w1 = __ldg(w + k + 1), w2 = __ldg(w + k + 2), w3 = __ldg(w + k + 3);
-#pragma unroll
-        for (int j = 0; j < HEAD_B; ++j) {
-            const float4 h = *reinterpret_cast<const float4*>(&hs[j][k]);
-            acc[j] = fmaf(w3, h.w, fmaf(w2, h.z, fmaf(w1, h.y, fmaf(w0, h.x, acc[j]))));
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < HEAD_B; ++j)
-        if (b0 + j < B) E[(b0 + j) * ED + o] = acc[j];
 }
 
 // One warp per pair: pred = ||E[ia]-E[ib]|| (all ED embedding values), loss += w (pred-y)^2 / P,
@@ -203,40 +233,58 @@ __global__ void enc_adam(float* __restrict__ p, const float* __restrict__ g, flo
 
 // ---------------------------------------------------------------------------
 // Tensor-core GRU forward for inference (tcgen05).  CTA = 128 trajectories
-// (the MMA's M), 256 threads.  Per time step the operand [a_t | h_t]
-// (128 x 192 BF16, shared memory) is multiplied by the BF16 gate weights,
-// resident in shared memory for all steps, into three FP32 accumulators in
-// tensor memory (512 columns):
-//   columns   0..255  r and z pre-activations  [a_t | h_t] [Wih_rz | Whh_rz]^T  (K = 192)
-//   columns 256..383  Win a_t                   a_t Wih_n^T                      (K = 64)
-//   columns 384..511  Whn h_t                   h_t Whh_n^T                      (K = 128)
-// (n needs Whn h apart from Win a: r multiplies only the hidden part.)  One
-// thread issues the 24 MMAs and commits them to an mbarrier; then warp w reads
-// lanes 32 (w % 4) .. +31 (its 32 trajectories) and hidden units
-// 64 (w / 4) .. +63 (sixteen warps, 32 units each, measured no faster: 1.31 vs
-// 1.39 ms for 1,000 queries), applies the gates with the biases in FP32, keeps h in FP32
-// registers and writes it back to shared memory as BF16 for the next step.
-// The a_t part comes from enc_conv_fwd_tc as one 16 KB BF16 image per step
-// already in the operand layout; thread 0 bulk-copies step t+1's image into
-// the second of two a-buffers while step t computes (per-buffer mbarriers
-// count the bytes).  a_t and h_t enter the products as BF16 (the training
-// kernels multiply FP32 a and h by the BF16 weights) and the gates use the
-// hardware tanh, so the embeddings agree with the training forward to BF16
-// rounding of the activations.
+// (the MMA's M); per time step the operand [a_t | h_t] (128 x 192 BF16, shared
+// memory) is multiplied by the BF16 gate weights, resident in shared memory for
+// all steps, into FP32 accumulators in tensor memory (all 512 columns).  (n
+// needs Whn h apart from Win a: r multiplies only the hidden part.)
+//
+// The hidden units go in two halves of 64, each with accumulators of its own
+// (256 columns: Win a | r | z | Whn h), so that the tensor cores and the gate
+// math overlap although a step needs all of the step before: while the gates
+// of half 0 are computed the products of half 1 run, and under the gates of
+// half 1 the next step's products of half 0 with a and with the new h of half
+// 0.  Only the products of half 0 with the h of half 1 wait for the whole step.
+// h of half 0 has two buffers (half 1's products of step t read it while step
+// t + 1's is written), h of half 1 one.
+//
+// Threads: a ninth warp issues copies and MMAs (one elected lane); eight warps
+// do the gates, warp w the tensor-memory lanes (trajectories) 32 (w % 4) .. +31
+// and 32 of a half's 64 units, with the biases in FP32, h in FP32 registers and
+// written back to shared memory as BF16.  The a_t part comes from
+// enc_conv_fwd_tc as one 16 KB BF16 image per step already in the operand
+// layout, bulk-copied two buffers ahead.  a_t and h_t enter the products as BF16
+// (the training kernels multiply FP32 a and h by the BF16 weights) and the
+// gates use the hardware tanh, so the embeddings agree with the training
+// forward to BF16 rounding of the activations.
+//
+// What bounds it: the gate math.  The hardware tanh, three a unit at 16 a clock
+// and SM, takes 3,072 clocks a step; measured 5,100 with the six biases a unit
+// (shared-memory loads of 16 bytes, which take 4 clocks though broadcast; without
+// them 3,300), 900 for the tensor-memory loads, 700 for writing h back, 1,000
+// waiting for the first products: 7,700 a step against 12,500 when products and
+// gates took turns.  100,000 trajectories of 20..200 points in three launches:
+// 3.76 -> 2.33 ms.  Sixteen gate warps of 16 units spill (96 registers): 8,000.
+// The two biases of a gate are added one after the other: their sum would save
+// a quarter of the loads but round differently, and a BF16 rounding of h that
+// flips shows as 6e-4 of the embedding's size.
 constexpr int TC_M = 128;
-constexpr int TC_THREADS = 256;  // 8 warps: two per 32-lane quarter of tensor memory
-constexpr int TC_HU = HD / (TC_THREADS / 128);  // hidden units per thread (32)
-constexpr int TC_K = C1 + HD;                               // 192
+constexpr int TC_EPI = 256;                                 // gate threads: two warps per 32-lane quarter of tensor memory
+constexpr int TC_THREADS = TC_EPI + 32;
+constexpr int TC_HH = HD / 2;                               // hidden units of a half
+constexpr int TC_HU = TC_HH / (TC_EPI / 128);               // of them per thread (32)
+constexpr int TC_N = 3 * TC_HH;                             // MMA N: 192
 constexpr int TC_A_BYTES = TC_M * C1 * 2;                   // one a_t image: 16 KB
-constexpr int TC_OFF_A0 = 0;                                // a-buffers [128][64] BF16
-constexpr int TC_OFF_A1 = TC_OFF_A0 + TC_A_BYTES;
-constexpr int TC_OFF_XH = TC_OFF_A1 + TC_A_BYTES;           // h [128][128] BF16
-constexpr int TC_OFF_WRZ = TC_OFF_XH + TC_M * HD * 2;       // W_rz [256][192] BF16
-constexpr int TC_OFF_WIN = TC_OFF_WRZ + 2 * HD * TC_K * 2;  // W_in [128][64]
-constexpr int TC_OFF_WHN = TC_OFF_WIN + HD * C1 * 2;        // W_hn [128][128]
-constexpr int TC_OFF_BIAS = TC_OFF_WHN + HD * HD * 2;       // float b_ih[384], b_hh[384]
-constexpr int TC_OFF_BAR = TC_OFF_BIAS + 2 * G3 * 4;        // mbarriers: MMA, a0, a1 (8 B each); TMEM address
-constexpr int TC_SMEM = TC_OFF_BAR + 32;
+constexpr int TC_H_BYTES = TC_M * TC_HH * 2;                // one half of h: 16 KB
+constexpr int TC_WA_BYTES = TC_N * C1 * 2;                  // a half's weights of a: rows Win | Wir | Wiz, 24 KB
+constexpr int TC_WH_BYTES = TC_N * HD * 2;                  // of h: rows Whr | Whz | Whn, 48 KB
+constexpr int TC_OFF_A = 0;                                 // a-buffers [128][64] BF16
+constexpr int TC_OFF_H = TC_OFF_A + 2 * TC_A_BYTES;         // h: half 0 (two buffers), half 1
+constexpr int TC_OFF_WA = TC_OFF_H + 3 * TC_H_BYTES;
+constexpr int TC_OFF_WH = TC_OFF_WA + 2 * TC_WA_BYTES;
+constexpr int TC_OFF_BIAS = TC_OFF_WH + 2 * TC_WH_BYTES;    // float b_ir, b_hr, b_iz, b_hz, b_in [128], b_hn [112]
+constexpr int TC_OFF_BAR = TC_OFF_BIAS + (6 * HD - 16) * 4;        // mbarriers; tensor-memory address
+constexpr int TC_SMEM = TC_OFF_BAR + 64;
+static_assert(TC_SMEM <= 227 * 1024, "enc_gru_embed_tc shared memory");
 constexpr uint32_t TC_TMEM_COLS = 512;
 // a wait for the tensor cores or a copy longer than this many SM clocks (~1 s) is an error
 constexpr long long TC_WAIT_CYCLES = 2000000000LL;
@@ -269,52 +317,69 @@ __device__ __forceinline__ uint4 pack8_bf16(const float* v) {
 // rounded to BF16): for block g of 128 trajectories and step t, the 16 KB
 // image of the a_t operand (rows = trajectories, k = channels, core-matrix
 // layout) at Ab + (g * T + t) * 128 * 64.  Rows past B and steps past a
-// trajectory's length are zero.  One thread per (trajectory, step), all 64
-// channels, with the conv weights in shared memory; consecutive threads take
+// trajectory's length are zero.  One thread per (trajectory, CT steps), all 64
+// channels: a channel's ten weights (shared memory, 16-byte loads) serve CT
+// steps (with one step a thread and a load per weight the images of 100,000
+// trajectories of 20..200 steps took 0.75 ms, with four 0.66, with eight 0.79:
+// at 1.8 GB written it is near what plain writes reach).  Consecutive threads take
 // consecutive rows of one image, so a warp's 16-byte stores are contiguous.
 // Bp = B rounded up to a multiple of 128; blockDim = 256.
+constexpr int CT = 4;
 __global__ void __launch_bounds__(256) enc_conv_fwd_tc(const float2* __restrict__ pts, const int64_t* __restrict__ off,
                                                        const int32_t* __restrict__ len, int B, int Bp, int T,
                                                        float4 nrm, const __nv_bfloat16* __restrict__ wq,
                                                        const float* __restrict__ p, __nv_bfloat16* __restrict__ Ab) {
-    __shared__ float w1[C1 * 2 * KW], b1[C1];
-    for (int e = threadIdx.x; e < C1 * 2 * KW; e += blockDim.x) w1[e] = __bfloat162float(wq[OFF_W1 + e]);
-    for (int e = threadIdx.x; e < C1; e += blockDim.x) b1[e] = p[OFF_B1 + e];
+    __shared__ __align__(16) float w1[C1][12];  // the ten weights of a channel, its bias
+    for (int e = threadIdx.x; e < C1 * 2 * KW; e += blockDim.x) {
+        const int c = e / (2 * KW), i = e / KW % 2, k = e % KW;
+        w1[c][2 * k + i] = __bfloat162float(wq[OFF_W1 + e]);
+    }
+    for (int e = threadIdx.x; e < C1; e += blockDim.x) w1[e][2 * KW] = p[OFF_B1 + e];
     __syncthreads();
+    const int tq = (T + CT - 1) / CT;
     const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= (int64_t)Bp * T) return;
+    if (gid >= (int64_t)Bp * tq) return;
     const int row = gid % TC_M;
-    const int t = (gid / TC_M) % T;
-    const int g = gid / ((int64_t)TC_M * T);
+    const int t0 = (int)(gid / TC_M % tq) * CT;
+    const int g = (int)(gid / ((int64_t)TC_M * tq));
     const int b = g * TC_M + row;
     const int n = b < B ? len[b] : 0;
-    float x[KW][2];  // the window's normalised points
-    if (t < n) {
+    float x[KW - 1 + CT][2];  // the window's normalised points
+    if (t0 < n) {
         const int64_t o = off[b];
 #pragma unroll
-        for (int k = 0; k < KW; ++k)
+        for (int k = 0; k < KW - 1 + CT; ++k)
 #pragma unroll
-            for (int i = 0; i < 2; ++i) x[k][i] = xin(pts, o, n, t + k - 2, i, nrm);
+            for (int i = 0; i < 2; ++i) x[k][i] = xin(pts, o, n, t0 + k - 2, i, nrm);
     }
-    unsigned char* img = reinterpret_cast<unsigned char*>(Ab + ((int64_t)g * T + t) * (TC_M * C1));
+    unsigned char* img = reinterpret_cast<unsigned char*>(Ab + ((int64_t)g * T + t0) * (TC_M * C1));
 #pragma unroll 1
     for (int c8 = 0; c8 < C1 / 8; ++c8) {
-        float a[8];
+        float a[CT][8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const int c = 8 * c8 + q;
-            float v = 0.f;
-            if (t < n) {
-                float acc = b1[c];
+            const float4* w4 = reinterpret_cast<const float4*>(w1[8 * c8 + q]);
+            const float4 wa = w4[0], wb = w4[1], wc = w4[2];
+            const float w[2 * KW] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w, wc.x, wc.y};
 #pragma unroll
-                for (int k = 0; k < KW; ++k)
+            for (int d = 0; d < CT; ++d) {
+                float v = 0.f;
+                if (t0 + d < n) {
+                    float acc = wc.z;
 #pragma unroll
-                    for (int i = 0; i < 2; ++i) acc = fmaf(w1[(c * 2 + i) * KW + k], x[k][i], acc);
-                v = fmaxf(acc, 0.f);
+                    for (int k = 0; k < KW; ++k)
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) acc = fmaf(w[2 * k + i], x[d + k][i], acc);
+                    v = fmaxf(acc, 0.f);
+                }
+                a[d][q] = v;
             }
-            a[q] = v;
         }
-        *reinterpret_cast<uint4*>(img + tsm::umma::core_offset(row, 8 * c8, TC_M)) = pack8_bf16(a);
+#pragma unroll
+        for (int d = 0; d < CT; ++d)
+            if (t0 + d < T)
+                *reinterpret_cast<uint4*>(img + (int64_t)d * (TC_M * C1 * 2) + tsm::umma::core_offset(row, 8 * c8, TC_M)) =
+                    pack8_bf16(a[d]);
     }
 }
 
@@ -340,170 +405,231 @@ __global__ void __launch_bounds__(TC_THREADS, 1) enc_gru_embed_tc(const __nv_bfl
                                                                    long long wait_cycles, int stall_step) {
     namespace U = tsm::umma;
     extern __shared__ __align__(1024) unsigned char sm[];
-    unsigned char* XH = sm + TC_OFF_XH;
+    // (no static shared memory: the dynamic part, aligned to 1 KB, would start behind it and not fit)
+    // the CTA's steps; once all have read them, -1: MMAs may still write tensor memory
+    volatile int& steps = *reinterpret_cast<volatile int*>(sm + TC_OFF_BAR + 60);
     float* bias = reinterpret_cast<float*>(sm + TC_OFF_BIAS);
     const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(sm));
-    const uint32_t mbar = sbase + TC_OFF_BAR, abar0 = mbar + 8, abar1 = mbar + 16;
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + TC_OFF_BAR + 24);
+    // mbarriers: products of half p done, h of half p written, a-buffer i landed, the last products done
+    const uint32_t bar = sbase + TC_OFF_BAR;
+    auto dbar = [&](int p) { return bar + 8 * p; };
+    auto ebar = [&](int p) { return bar + 16 + 8 * p; };
+    auto abar = [&](int i) { return bar + 32 + 8 * i; };
+    const uint32_t last = bar + 48;
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + TC_OFF_BAR + 56);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int row = 32 * (warp & 3) + lane;  // this thread's trajectory (TMEM lane)
-    const int hc = warp >> 2;                // hidden units TC_HU hc .. +TC_HU-1
-    const int b = blockIdx.x * TC_M + row;
-    const int n = b < B ? len[b] : 0;
-    const __nv_bfloat16* img = Ab + (int64_t)blockIdx.x * T * (TC_M * C1);  // this block's a_t images
+    const int blk = gridDim.x - 1 - blockIdx.x;  // the last block, the longest of a batch in length order, first
+    const __nv_bfloat16* img = Ab + (int64_t)blk * T * (TC_M * C1);  // this block's a_t images
 
-    // weights -> core-matrix layout (16-byte chunks of 8 consecutive k)
-    for (int e = tid; e < 2 * HD * (TC_K / 8); e += TC_THREADS) {  // W_rz: gate rows 0..255, k < 192
-        const int r = e / (TC_K / 8), c = e % (TC_K / 8);
-        const __nv_bfloat16* src = c < C1 / 8 ? wq + OFF_WIH + r * C1 + 8 * c : wq + OFF_WHH + r * HD + 8 * (c - C1 / 8);
-        *reinterpret_cast<uint4*>(sm + TC_OFF_WRZ + U::core_offset(r, 8 * c, 2 * HD)) =
-            *reinterpret_cast<const uint4*>(src);
+    if (tid == 0) steps = 0;
+    // weights -> core-matrix layout (16-byte chunks of 8 consecutive k); operand row 64 g + i of half q is unit
+    // 64 q + i of the g-th gate of its list (gate rows r 0..127, z 128..255, n 256..383)
+    for (int e = tid; e < 2 * TC_N * (C1 / 8); e += TC_THREADS) {  // a: n, r, z
+        const int c = e % (C1 / 8), r = e / (C1 / 8) % TC_N, q = e / (TC_N * (C1 / 8)), g = r / TC_HH;
+        const int row = (g == 0 ? 2 : g - 1) * HD + TC_HH * q + r % TC_HH;
+        *reinterpret_cast<uint4*>(sm + TC_OFF_WA + q * TC_WA_BYTES + U::core_offset(r, 8 * c, TC_N)) =
+            *reinterpret_cast<const uint4*>(wq + OFF_WIH + row * C1 + 8 * c);
     }
-    for (int e = tid; e < HD * (C1 / 8); e += TC_THREADS) {  // W_in: gate rows 256..383, k < 64
-        const int r = e / (C1 / 8), c = e % (C1 / 8);
-        *reinterpret_cast<uint4*>(sm + TC_OFF_WIN + U::core_offset(r, 8 * c, HD)) =
-            *reinterpret_cast<const uint4*>(wq + OFF_WIH + (2 * HD + r) * C1 + 8 * c);
+    for (int e = tid; e < 2 * TC_N * (HD / 8); e += TC_THREADS) {  // h: r, z, n
+        const int c = e % (HD / 8), r = e / (HD / 8) % TC_N, q = e / (TC_N * (HD / 8)), g = r / TC_HH;
+        const int row = g * HD + TC_HH * q + r % TC_HH;
+        *reinterpret_cast<uint4*>(sm + TC_OFF_WH + q * TC_WH_BYTES + U::core_offset(r, 8 * c, TC_N)) =
+            *reinterpret_cast<const uint4*>(wq + OFF_WHH + row * HD + 8 * c);
     }
-    for (int e = tid; e < HD * (HD / 8); e += TC_THREADS) {  // W_hn: gate rows 256..383, k < 128
-        const int r = e / (HD / 8), c = e % (HD / 8);
-        *reinterpret_cast<uint4*>(sm + TC_OFF_WHN + U::core_offset(r, 8 * c, HD)) =
-            *reinterpret_cast<const uint4*>(wq + OFF_WHH + (2 * HD + r) * HD + 8 * c);
+    for (int e = tid; e < HD; e += TC_THREADS) {
+        bias[e] = p[OFF_BIH + e];
+        bias[HD + e] = p[OFF_BHH + e];
+        bias[2 * HD + e] = p[OFF_BIH + HD + e];
+        bias[3 * HD + e] = p[OFF_BHH + HD + e];
+        bias[4 * HD + e] = p[OFF_BIH + 2 * HD + e];
+        if (e < HD - 16) bias[5 * HD + e] = p[OFF_BHH + 2 * HD + e];  // (the last 16 do not fit: registers)
     }
-    for (int e = tid; e < 2 * G3; e += TC_THREADS) bias[e] = e < G3 ? p[OFF_BIH + e] : p[OFF_BHH + e - G3];
-    {  // h_0 = 0: this thread's 64 hidden units
-        const float z8[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int c = 0; c < TC_HU / 8; ++c)
-            *reinterpret_cast<uint4*>(XH + U::core_offset(row, TC_HU * hc + 8 * c, TC_M)) = pack8_bf16(z8);
-    }
+    for (int e = tid; e < 3 * TC_H_BYTES / 16; e += TC_THREADS)  // h_0 = 0
+        *reinterpret_cast<uint4*>(sm + TC_OFF_H + 16 * e) = make_uint4(0, 0, 0, 0);
     if (tid == 0) {
-        U::mbar_init(mbar, 1);
-        U::mbar_init(abar0, 1);
-        U::mbar_init(abar1, 1);
+        for (int q = 0; q < 2; ++q) {
+            U::mbar_init(dbar(q), 1);
+            U::mbar_init(ebar(q), TC_EPI / 32);
+            U::mbar_init(abar(q), 1);
+        }
+        U::mbar_init(last, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) U::tmem_alloc(sbase + TC_OFF_BAR + 24, TC_TMEM_COLS);
+    if (warp == 0) U::tmem_alloc(sbase + TC_OFF_BAR + 56, TC_TMEM_COLS);
     U::fence_smem_async();
     U::fence_before_sync();
     __syncthreads();
     U::fence_after_sync();
     const uint32_t tmem = *tmem_slot;
-    const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16);  // this warp's lane quarter
+    if (tid < TC_M && blk * TC_M + tid < B) atomicMax(const_cast<int*>(&steps), min(len[blk * TC_M + tid], T));
+    __syncthreads();
+    const int tmax = steps;
 
-    int tmax = 0;
-    for (int i = 0; i < TC_M; ++i) {
-        const int bi = blockIdx.x * TC_M + i;
-        if (bi < B) tmax = max(tmax, len[bi]);
-    }
-    tmax = min(tmax, T);
-    int pend = -1;    // thread 0: the step whose a_t copy is issued and not yet waited for
-    int issued = -1;  // thread 0: the last step whose MMAs were committed
-    if (tid == 0 && tmax > 0) {  // a_0 into buffer 0
-        U::mbar_arrive_expect_tx(abar0, TC_A_BYTES);
-        if (stall_step != 0) U::bulk_load(sbase + TC_OFF_A0, img, TC_A_BYTES, abar0);
-        pend = 0;
-    }
-    float h[TC_HU];
+    if (warp == TC_EPI / 32) {
+        if (tmax > 0) {  // the whole warp runs this, its leader issues
+            constexpr uint32_t kLBO = TC_M * 16, kWL = TC_N * 16;  // K-chunk strides of the operands
+            constexpr uint32_t id3 = U::idesc_bf16_f32(TC_M, TC_N), id2 = U::idesc_bf16_f32(TC_M, 2 * TC_HH),
+                               id1 = U::idesc_bf16_f32(TC_M, TC_HH);
+            const uint32_t leader = U::elect_leader();
+            auto step_of = [](int bytes) { return (uint64_t)(bytes >> 4); };  // descriptor increment of a start address
+            const uint64_t a_desc = U::smem_desc(sbase + TC_OFF_A, kLBO, 128), h_desc = U::smem_desc(sbase + TC_OFF_H, kLBO, 128);
+            const uint64_t wa = U::smem_desc(sbase + TC_OFF_WA, kWL, 128), wh = U::smem_desc(sbase + TC_OFF_WH, kWL, 128);
+            auto waited = [&](uint32_t b, int use) {
+                return (bool)__all_sync(0xffffffffu, U::mbar_wait(b, (uint32_t)(use & 1), wait_cycles));
+            };
+            int loaded = 0;
+            auto load_a = [&](int t) {
+                if (leader) {
+                    U::mbar_arrive_expect_tx(abar(t & 1), TC_A_BYTES);
+                    if (t != stall_step)
+                        U::bulk_load(sbase + TC_OFF_A + (t & 1) * TC_A_BYTES, img + (int64_t)t * (TC_M * C1), TC_A_BYTES,
+                                     abar(t & 1));
+                }
+                __syncwarp();
+                loaded = t + 1;
+            };
+            auto a_products = [&](int t, int q) {
+                const uint64_t a = a_desc + step_of((t & 1) * TC_A_BYTES), w = wa + step_of(q * TC_WA_BYTES);
 #pragma unroll
-    for (int i = 0; i < TC_HU; ++i) h[i] = 0.f;
-    bool failed = false;
-    int fail_t = -1;
-    for (int t = 0; t < tmax; ++t) {
-        const uint32_t abuf = sbase + ((t & 1) ? TC_OFF_A1 : TC_OFF_A0);
-        if (tid == 0) {
-            // a_t has landed in buffer t % 2 (its (t / 2)-th use)
-            if (!U::mbar_wait((t & 1) ? abar1 : abar0, (uint32_t)((t >> 1) & 1), wait_cycles)) {
-                atomicOr(status, TC_ERR_COPY);
-            } else {
-                pend = -1;
+                for (int ks = 0; ks < C1 / 16; ++ks)
+                    U::mma_bf16_warp(tmem + 256 * q, a + step_of(ks * 2 * kLBO), w + step_of(ks * 2 * kWL), id3, ks, leader);
+            };
+            auto h_products = [&](int t, int q, int part) {  // part: half of h
+                const uint64_t h = h_desc + step_of((part ? 2 : (t & 1)) * TC_H_BYTES);
+                const uint64_t w = wh + step_of(q * TC_WH_BYTES + part * (TC_HH / 8) * kWL);
+#pragma unroll
+                for (int ks = 0; ks < TC_HH / 16; ++ks) {
+                    const uint64_t hk = h + step_of(ks * 2 * kLBO), wk = w + step_of(ks * 2 * kWL);
+                    if (part == 0 && ks == 0) {  // Whn h starts here; r and z go on from the products with a
+                        U::mma_bf16_warp(tmem + 256 * q + TC_HH, hk, wk, id2, 1u, leader);
+                        U::mma_bf16_warp(tmem + 256 * q + 3 * TC_HH, hk, wk + step_of(2 * TC_HH * 16), id1, 0u, leader);
+                    } else {
+                        U::mma_bf16_warp(tmem + 256 * q + TC_HH, hk, wk, id3, 1u, leader);
+                    }
+                }
+            };
+            int err = 0;
+            load_a(0);
+            for (int t = 0; t < tmax && !err; ++t) {
+                if (!waited(abar(t & 1), t >> 1)) {
+                    err = TC_ERR_COPY;
+                    break;
+                }
+                if (t > 0 && !waited(ebar(0), t - 1)) {
+                    err = TC_ERR_MMA;
+                    break;
+                }
                 U::fence_after_sync();
-                constexpr uint32_t kRZ = U::idesc_bf16_f32(TC_M, 2 * HD), kN = U::idesc_bf16_f32(TC_M, HD);
-                constexpr uint32_t kLBO = TC_M * 16;  // K-chunk stride of the 128-row operands
-                for (int ks = 0; ks < TC_K / 16; ++ks) {  // r, z: [a_t | h_t] [W_ih | W_hh]^T, K = 192
-                    const uint32_t a = ks < C1 / 16 ? abuf + ks * 2 * kLBO : sbase + TC_OFF_XH + (ks - C1 / 16) * 2 * kLBO;
-                    U::mma_bf16(tmem, U::smem_desc(a, kLBO, 128),
-                                U::smem_desc(sbase + TC_OFF_WRZ + ks * 2 * (2 * HD * 16), 2 * HD * 16, 128), kRZ, ks);
+                a_products(t, 0);
+                h_products(t, 0, 0);
+                if (t > 0 && !waited(ebar(1), t - 1)) {
+                    err = TC_ERR_MMA;
+                    break;
                 }
-                for (int ks = 0; ks < C1 / 16; ++ks)  // Win a_t
-                    U::mma_bf16(tmem + 2 * HD, U::smem_desc(abuf + ks * 2 * kLBO, kLBO, 128),
-                                U::smem_desc(sbase + TC_OFF_WIN + ks * 2 * (HD * 16), HD * 16, 128), kN, ks);
-                for (int ks = 0; ks < HD / 16; ++ks)  // Whn h_t
-                    U::mma_bf16(tmem + 3 * HD, U::smem_desc(sbase + TC_OFF_XH + ks * 2 * kLBO, kLBO, 128),
-                                U::smem_desc(sbase + TC_OFF_WHN + ks * 2 * (HD * 16), HD * 16, 128), kN, ks);
-                U::commit(mbar);
-                issued = t;
-                if (t + 1 < tmax) {  // a_{t+1} into the other buffer (its last reader, step t-1, has completed)
-                    const uint32_t nb = (t & 1) ? abar0 : abar1;
-                    U::mbar_arrive_expect_tx(nb, TC_A_BYTES);
-                    if (t + 1 != stall_step)
-                        U::bulk_load(sbase + ((t & 1) ? TC_OFF_A0 : TC_OFF_A1), img + (int64_t)(t + 1) * (TC_M * C1),
-                                     TC_A_BYTES, nb);
-                    pend = t + 1;
-                }
+                U::fence_after_sync();
+                h_products(t, 0, 1);
+                if (leader) U::commit(dbar(0));
+                __syncwarp();
+                if (t + 1 < tmax) load_a(t + 1);  // its buffer's readers, step t - 1, are done
+                a_products(t, 1);
+                h_products(t, 1, 0);
+                h_products(t, 1, 1);
+                if (leader) U::commit(dbar(1));
+                __syncwarp();
             }
-        }
-        const bool ok = U::mbar_wait(mbar, (uint32_t)(t & 1), wait_cycles);
-        if (__syncthreads_or(!ok)) {
-            failed = true;
-            fail_t = t;
-            break;
-        }
-        U::fence_after_sync();
-        const bool live = t < n;
-#pragma unroll
-        for (int c = 0; c < TC_HU / 16; ++c) {  // 16 hidden units at a time
-            const int k0 = TC_HU * hc + 16 * c;
-            uint32_t rr[16], zz[16], ii[16], hh[16];
-            U::ld16(tl + k0, rr);
-            U::ld16(tl + HD + k0, zz);
-            U::ld16(tl + 2 * HD + k0, ii);
-            U::ld16(tl + 3 * HD + k0, hh);
-            U::wait_ld(rr);
-            U::wait_ld(zz);
-            U::wait_ld(ii);
-            U::wait_ld(hh);
-            float hv[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const int k = k0 + j;
-                const float r = sigm_hw(__uint_as_float(rr[j]) + bias[k] + bias[G3 + k]);
-                const float z = sigm_hw(__uint_as_float(zz[j]) + bias[HD + k] + bias[G3 + HD + k]);
-                const float nn = tanh_hw(__uint_as_float(ii[j]) + bias[2 * HD + k] +
-                                         r * (__uint_as_float(hh[j]) + bias[G3 + 2 * HD + k]));
-                const float hp = h[16 * c + j];
-                hv[j] = live ? (1.f - z) * nn + z * hp : hp;
-                h[16 * c + j] = hv[j];
+            // nothing of this CTA may be in flight when it exits
+            if (err) {
+                if (leader) atomicOr(status, err);
+                for (int i = max(0, loaded - 2); i < loaded; ++i)
+                    if (i != stall_step) waited(abar(i & 1), i >> 1);
             }
-            if (live) {
-                *reinterpret_cast<uint4*>(XH + U::core_offset(row, k0, TC_M)) = pack8_bf16(hv);
-                *reinterpret_cast<uint4*>(XH + U::core_offset(row, k0 + 8, TC_M)) = pack8_bf16(hv + 8);
-            }
-        }
-        U::fence_smem_async();
-        U::fence_before_sync();
-        __syncthreads();
-    }
-    __shared__ int tmem_busy;  // set by thread 0 when MMAs may still write tensor memory
-    if (tid == 0) {
-        tmem_busy = 0;
-        if (pend >= 0)  // after a failure: let this CTA's copy in flight land before exiting
-            U::mbar_wait((pend & 1) ? abar1 : abar0, (uint32_t)((pend >> 1) & 1), wait_cycles);
-        if (failed && issued == fail_t) {  // the failed step's MMAs were committed: wait for them once more
-            atomicOr(status, TC_ERR_MMA);
-            if (!U::mbar_wait(mbar, (uint32_t)(fail_t & 1), wait_cycles)) {
+            if (leader) U::commit(last);
+            __syncwarp();
+            if (!waited(last, 0) && leader) {
                 atomicOr(status, TC_ERR_TMEM_HELD);
-                tmem_busy = 1;
+                steps = -1;
             }
         }
-    }
-    if (b < B) {
-        float* dst = hl + (int64_t)b * HD + TC_HU * hc;
+    } else {
+        const int row = 32 * (warp & 3) + lane;  // this thread's trajectory (tensor-memory lane)
+        const int sub = warp >> 2;               // units TC_HU sub .. +TC_HU-1 of each half
+        const int b = blk * TC_M + row;
+        const int n = b < B ? len[b] : 0;
+        const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+        float h[2 * TC_HU], tail[16];
 #pragma unroll
-        for (int i = 0; i < TC_HU; ++i) dst[i] = failed ? __int_as_float(0x7fc00000) : h[i];
+        for (int i = 0; i < 2 * TC_HU; ++i) h[i] = 0.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) tail[i] = __ldg(p + OFF_BHH + 3 * HD - 16 + i);
+        bool failed = false;
+        for (int t = 0; t < tmax && !failed; ++t) {
+            const bool live = t < n;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                if (!__all_sync(0xffffffffu, U::mbar_wait(dbar(q), (uint32_t)(t & 1), wait_cycles))) {
+                    if (lane == 0) atomicOr(status, TC_ERR_MMA);
+                    failed = true;
+                    break;
+                }
+                U::fence_after_sync();
+                __syncwarp();
+                unsigned char* H = sm + TC_OFF_H + (q ? 2 : ((t + 1) & 1)) * TC_H_BYTES;
+#pragma unroll
+                for (int c = 0; c < TC_HU / 16; ++c) {  // 16 hidden units at a time
+                    const int u0 = TC_HU * sub + 16 * c, k0 = TC_HH * q + u0;
+                    uint32_t rr[16], zz[16], ii[16], hh[16];
+                    U::ld16(tl + 256 * q + u0, ii);
+                    U::ld16(tl + 256 * q + TC_HH + u0, rr);
+                    U::ld16(tl + 256 * q + 2 * TC_HH + u0, zz);
+                    U::ld16(tl + 256 * q + 3 * TC_HH + u0, hh);
+                    U::wait_ld(ii);
+                    U::wait_ld(rr);
+                    U::wait_ld(zz);
+                    U::wait_ld(hh);
+                    float hv[16];
+#pragma unroll
+                    for (int j4 = 0; j4 < 16; j4 += 4) {
+                        auto b4 = [&](int a) { return *reinterpret_cast<const float4*>(bias + a * HD + k0 + j4); };
+                        // the two biases of a gate are added one after the other
+                        const float4 r1 = b4(0), r2 = b4(1), z1 = b4(2), z2 = b4(3), bi = b4(4);
+                        const bool in_regs = q == 1 && c == TC_HU / 16 - 1;  // the last 16 units of the last warps
+                        float4 bh = make_float4(tail[j4], tail[j4 + 1], tail[j4 + 2], tail[j4 + 3]);
+                        if (!in_regs || sub == 0) bh = b4(5);
+                        const float xr1[4] = {r1.x, r1.y, r1.z, r1.w}, xr2[4] = {r2.x, r2.y, r2.z, r2.w};
+                        const float xz1[4] = {z1.x, z1.y, z1.z, z1.w}, xz2[4] = {z2.x, z2.y, z2.z, z2.w};
+                        const float xi[4] = {bi.x, bi.y, bi.z, bi.w}, xh[4] = {bh.x, bh.y, bh.z, bh.w};
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const int j = j4 + e;
+                            const float r = sigm_hw(__uint_as_float(rr[j]) + xr1[e] + xr2[e]);
+                            const float z = sigm_hw(__uint_as_float(zz[j]) + xz1[e] + xz2[e]);
+                            const float nn = tanh_hw(__uint_as_float(ii[j]) + xi[e] + r * (__uint_as_float(hh[j]) + xh[e]));
+                            const float hp = h[TC_HU * q + 16 * c + j];
+                            hv[j] = live ? (1.f - z) * nn + z * hp : hp;
+                            h[TC_HU * q + 16 * c + j] = hv[j];
+                        }
+                    }
+                    *reinterpret_cast<uint4*>(H + U::core_offset(row, u0, TC_M)) = pack8_bf16(hv);
+                    *reinterpret_cast<uint4*>(H + U::core_offset(row, u0 + 8, TC_M)) = pack8_bf16(hv + 8);
+                }
+                U::fence_smem_async();
+                U::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) U::mbar_arrive(ebar(q));
+            }
+        }
+        if (b < B) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                float* dst = hl + (int64_t)b * HD + TC_HH * q + TC_HU * sub;
+#pragma unroll
+                for (int i = 0; i < TC_HU; ++i) dst[i] = failed ? __int_as_float(0x7fc00000) : h[TC_HU * q + i];
+            }
+        }
     }
     U::fence_before_sync();
     __syncthreads();
-    if (warp == 0 && !tmem_busy) {
+    if (warp == 0 && steps >= 0) {
         U::fence_after_sync();
         U::tmem_dealloc(tmem, TC_TMEM_COLS);
     }
@@ -559,6 +685,19 @@ int enc_check(cudaError_t e, const char* what) {
     return tsm_internal_fail(TSM_ECUDA, b);
 }
 
+// The head over B trajectories: at most two CTAs per SM, each over blocks of HEAD_B.
+int enc_head(const float* hl, int B, const float* params, float* E, const float2* pts, const int64_t* off,
+             const int32_t* len, float4 n4, float* X, cudaStream_t s) {
+    using namespace enc;
+    int rc = enc_check(cudaFuncSetAttribute(enc_head_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, HEAD_SMEM),
+                       "cudaFuncSetAttribute(enc_head_fwd)");
+    if (rc) return rc;
+    const int blocks = (B + HEAD_B - 1) / HEAD_B;
+    enc_skip_fwd<<<(unsigned)(((int64_t)B * SK + 255) / 256), 256, 0, s>>>(B, params, E, pts, off, len, n4, X);
+    enc_head_fwd<<<blocks < 296 ? blocks : 296, EO, HEAD_SMEM, s>>>(hl, B, params, E);
+    return enc_check(cudaGetLastError(), "enc_head_fwd launch");
+}
+
 int enc_args(const void* params, const void* pts, const void* off, const void* len, int B, int T, const float* nrm,
              const void* ws) {
     if (!params || !pts || !off || !len || !nrm || !ws) return tsm_internal_fail(TSM_EINVAL, "encoder: null pointer");
@@ -577,10 +716,7 @@ int enc_forward(const float* params, const float* pts, const int64_t* off, const
     const int rc = train_forward(reinterpret_cast<const float2*>(pts), off, len, B, T, n4, w.wq, params, w.tr, w.hl,
                                  w.status, s);
     if (rc) return rc;
-    enc_head_fwd<<<(unsigned)((B + HEAD_B - 1) / HEAD_B), EO, 0, s>>>(w.hl, B, params, w.E,
-                                                                      reinterpret_cast<const float2*>(pts), off, len,
-                                                                      n4, w.X);
-    return enc_check(cudaGetLastError(), "encoder forward launch");
+    return enc_head(w.hl, B, params, w.E, reinterpret_cast<const float2*>(pts), off, len, n4, w.X, s);
 }
 
 int enc_backward(const float* params, const float* pts, const int64_t* off, const int32_t* len, int B, int T,
@@ -711,7 +847,7 @@ int tsm_enc_embed_opts(const float* params, const float* pts, const int64_t* off
     if ((rc = enc_check(cudaMemsetAsync(w.status, 0, 4, s), "memset embed status"))) return rc;
     enc_round_bf16<<<(OFF_WO + 255) / 256, 256, 0, s>>>(params, w.wq);
     const int Bp = (B + TC_M - 1) / TC_M * TC_M;
-    const int64_t tot = (int64_t)Bp * T;
+    const int64_t tot = (int64_t)Bp * ((T + CT - 1) / CT);
     enc_conv_fwd_tc<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(reinterpret_cast<const float2*>(pts), off, len, B,
                                                                    Bp, T, n4, w.wq, params, w.Ab);
     rc = enc_check(cudaFuncSetAttribute(enc_gru_embed_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM),
@@ -719,10 +855,7 @@ int tsm_enc_embed_opts(const float* params, const float* pts, const int64_t* off
     if (rc) return rc;
     enc_gru_embed_tc<<<Bp / TC_M, TC_THREADS, TC_SMEM, s>>>(w.Ab, len, B, T, w.wq, params, w.hl, w.status,
                                                             wait_cycles, stall_step);
-    enc_head_fwd<<<(unsigned)((B + HEAD_B - 1) / HEAD_B), EO, 0, s>>>(w.hl, B, params, emb,
-                                                                      reinterpret_cast<const float2*>(pts), off, len,
-                                                                      n4, nullptr);
-    return enc_check(cudaGetLastError(), "tsm_enc_embed launch");
+    return enc_head(w.hl, B, params, emb, reinterpret_cast<const float2*>(pts), off, len, n4, nullptr, s);
 }
 
 int tsm_enc_embed(const float* params, const float* pts, const int64_t* off, const int32_t* len, int32_t B,

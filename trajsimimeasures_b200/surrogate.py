@@ -175,8 +175,9 @@ class Encoder:
         perm = torch.argsort(lens_d, stable=True) if tensor_cores else torch.arange(n, device=s.device)
         sel_all = idx[perm]
         off_all, ln_all = s.off[sel_all].contiguous(), s.lens[sel_all].contiguous()
-        starts = list(range(0, n, batch))
-        ends = [min(b0 + batch, n) for b0 in starts]
+        # the batch that is not full first: in length order its launch, which leaves SMs idle, is then the shortest
+        starts = [0] + list(range(n % batch or batch, n, batch)) if tensor_cores else list(range(0, n, batch))
+        ends = starts[1:] + [n]
         if tensor_cores and len(starts) == 1 and idx_given is False:  # the whole set: its max length is known
             tmax = np.array([s.max_len])
         elif tensor_cores:  # sorted: a batch's longest trajectory is its last
