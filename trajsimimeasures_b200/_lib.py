@@ -27,7 +27,7 @@ EXPORTS = ("tsm_version", "tsm_last_error", "tsm_max_supported_len", "tsm_matrix
            "tsm_enc_embed", "tsm_enc_embed_status", "tsm_enc_train_status", "tsm_enc_embed_opts",
            "tsm_enc_loss_grad_w", "tsm_scan_dim",
            "tsm_scan_image_bytes", "tsm_scan_prepare", "tsm_scan", "tsm_scan_opts", "tsm_pair_order",
-           "tsm_pair_order_workspace_bytes")
+           "tsm_pair_order_workspace_bytes", "tsm_pack_pairs")
 
 
 class TsmParams(ctypes.Structure):
@@ -121,6 +121,9 @@ def load():
         lib.tsm_select_rows.restype = ctypes.c_int
         lib.tsm_select_rows.argtypes = [_vp, _i64, _i64, _i64, _i64, _vp, _vp]
         lib.tsm_pair_order_workspace_bytes.restype = ctypes.c_int
+        lib.tsm_pack_pairs.restype = ctypes.c_int
+        lib.tsm_pack_pairs.argtypes = [_vp, _i64, _i64, _vp, _vp, _i64, _i64, _vp, _i64, _i32, _i32, _vp, _vp, _vp, _vp,
+                                       _vp, _vp, _i64]
         lib.tsm_pair_order.restype = ctypes.c_int
         lib.tsm_pair_order.argtypes = [_vp, _vp, _i64, _vp, _vp, _vp]
         lib.tsm_topk_rows.restype = ctypes.c_int

@@ -128,6 +128,11 @@ def pair_origins(measure, t1, len1, t2, len2):
         f1, f2 = _first_points(p1[0], la), _first_points(p2[0], lb)
     if measure_id(measure) == _lib.ERP:
         return np.asarray(origin_of_points(np.concatenate([f1[la > 0], f2[lb > 0]])), dtype=np.float64)
+    return _pair_origin_of(f1, f2, la, lb)
+
+
+def _pair_origin_of(f1, f2, la, lb):
+    """One origin per pair from the trajectories' first points [n, 2]."""
     o = np.where((la > 0)[:, None], f1, np.where((lb > 0)[:, None], f2, 0.0))
     o = o.astype(np.float32).astype(np.float64)
     o[~np.isfinite(o).all(axis=1)] = 0.0
@@ -182,36 +187,45 @@ def release_staging():
     _tls.pinned = None
 
 
+def _packable(a):
+    """Whether tsm_pack_pairs reads the array as it is: float64 or float32 in
+    native byte order, aligned, the two coordinates of a point adjacent."""
+    return a.dtype in (np.dtype(np.float64), np.dtype(np.float32)) and a.flags.aligned and a.strides[2] == a.itemsize
+
+
 def _stage_padded(a1, a2, la, lb, order, dev, origin=None):
     """Padded host pair arrays [n, L, >=2] to the device through one pinned
-    buffer and one copy: the points are rounded to float32 straight into the
-    buffer (the rounding of astype; with an origin, [2] or per pair [n, 2],
-    after an FP64 translation by it), followed by the int32 lengths and
-    processing order; the offsets are made on the device.
-    -> (pts [n*L1 + n*L2, 2] float32, len_a, len_b, order int32, off_a, off_b int64)."""
-    n, L1, L2 = a1.shape[0], a1.shape[1], a2.shape[1]
-    nf1, nf2 = n * L1 * 2, n * L2 * 2
-    pts_bytes = 4 * (nf1 + nf2)  # a multiple of 8: nf1 and nf2 are even
-    nbytes = pts_bytes + 12 * n
+    buffer and one copy: offsets, lengths, processing order, and the valid
+    points rounded to float32 (the rounding of astype; with an origin, [2], after
+    an FP64 translation by it), back to back (tsm_pack_pairs).  origin "per
+    pair": each pair's own, as pair_origins gives it.
+    -> (pts [P, 2] float32, len_a, len_b, order int32, off_a, off_b int64)."""
+    n = a1.shape[0]
+    P = int(la.sum() + lb.sum())
+    ints_at = 16 * n                            # int64 offsets first
+    pts_at = (ints_at + 12 * n + 7) // 8 * 8    # int32 lengths and order, then the points
+    nbytes = pts_at + 8 * (P + 1)               # (one to spare: never an empty buffer)
     pin = _pinned(nbytes)
     host = pin.numpy()
-    f = host[:pts_bytes].view(np.float32)
-    if origin is None:
-        np.copyto(f[:nf1].reshape(n, L1, 2), a1[..., :2], casting="unsafe")
-        np.copyto(f[nf1:].reshape(n, L2, 2), a2[..., :2], casting="unsafe")
-    else:
-        o = np.asarray(origin, dtype=np.float64).reshape(-1, 1, 2)
-        sub_origin_f32(a1[..., :2], o, f[:nf1].reshape(n, L1, 2))
-        sub_origin_f32(a2[..., :2], o, f[nf1:].reshape(n, L2, 2))
-    ints = host[pts_bytes:nbytes].view(np.int32)
-    ints[:n] = la
-    ints[n:2 * n] = lb
+    off = host[:ints_at].view(np.int64)
+    ints = host[ints_at:ints_at + 12 * n].view(np.int32)
+    own = isinstance(origin, str)
+    if a1.dtype != a2.dtype or not (_packable(a1) and _packable(a2)):
+        dt = np.float32 if origin is None else np.float64
+        a1, a2 = np.ascontiguousarray(a1[..., :2], dtype=dt), np.ascontiguousarray(a2[..., :2], dtype=dt)
+    o = None if own or origin is None else np.ascontiguousarray(origin, dtype=np.float64)
+    l1, l2 = np.ascontiguousarray(la, dtype=np.int64), np.ascontiguousarray(lb, dtype=np.int64)
+    rc = _lib.load().tsm_pack_pairs(a1.ctypes.data, a1.strides[0], a1.strides[1], l1.ctypes.data, a2.ctypes.data,
+                                    a2.strides[0], a2.strides[1], l2.ctypes.data, n, int(a1.dtype == np.float64),
+                                    1 if own else 0 if o is None else 2, None if o is None else o.ctypes.data,
+                                    off.ctypes.data, off[n:].ctypes.data, ints.ctypes.data, ints[n:].ctypes.data,
+                                    host.ctypes.data + pts_at, P)
+    _lib.check(rc, "tsm_pack_pairs")
     ints[2 * n:] = order
     d = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     d.copy_(pin[:nbytes], non_blocking=True)
-    di = d[pts_bytes:].view(torch.int32)
-    ar = torch.arange(n, dtype=torch.int64, device=dev)
-    return d[:pts_bytes].view(torch.float32).view(-1, 2), di[:n], di[n:2 * n], di[2 * n:], ar * L1, n * L1 + ar * L2
+    do, di = d[:ints_at].view(torch.int64), d[ints_at:ints_at + 12 * n].view(torch.int32)
+    return d[pts_at:].view(torch.float32).view(P + 1, 2), di[:n], di[n:2 * n], di[2 * n:], do[:n], do[n:]
 
 
 def _normalise_counts(m, counts, la, lb):
@@ -240,8 +254,11 @@ def pairs(measure, t1, len1, t2, len2, *, eps=0.0, gpoint=(0.0, 0.0), exact=Fals
             raise ValueError("a length is negative or exceeds the padded width")
         dev = torch.device("cuda")
         max_len = int(max(la.max(), lb.max()))
-        origin = pair_origins(m, t1, la, t2, lb)
-        if origin is not None and origin.ndim == 1:
+        if m != _lib.ERP and (needs_origin(t1.dtype) or needs_origin(t2.dtype)):
+            origin = "per pair"  # formed where the points are packed
+        else:
+            origin = pair_origins(m, t1, la, t2, lb)
+        if origin is not None and m == _lib.ERP:
             gpoint = shift_gpoint(gpoint, origin)
         pts_t, la_t, lb_t, order_t, off_a_t, off_b_t = _stage_padded(t1, t2, la, lb, pair_order(la, lb), dev,
                                                                      origin)
