@@ -4,26 +4,33 @@
 //
 // Each time step's products are W [gates x features] times the features of 16
 // trajectories: the weights are the MMA's A operand (M = 128 gate rows, BF16,
-// resident in shared memory for all steps) and the trajectories its N.  The
+// resident in tensor memory for all steps) and the trajectories its N.  The
 // activations are FP32: x = hi + mid + lo, three BF16 parts that hold all 24
 // bits, stand side by side as N = 3 x 16 columns, and the epilogue adds the
 // three FP32 results.  Products of BF16 values are exact in FP32, so a sum
 // differs from an FP32 one only in how it is accumulated.
 //
-// Threads: 256 of the epilogue, thread (k, half) with k = hidden unit
-// (tensor-memory lane) and half = 8 of the block's 16 trajectories, whose h
-// (dh) it keeps in registers, and a ninth warp that issues copies and MMAs.  Eight values of one unit are eight consecutive N, so the three
-// parts go to the operand in shared memory as one 16-byte store each
-// (MN-major: element (n, k) at (k / 8) * 768 + (n / 8) * 128 + (k % 8) * 16 +
-// (n % 8) * 2), and to the weight gradient's operand images likewise, whose K
-// runs over (slot, trajectory).
+// Threads: 512 of the epilogue, thread (k, q) with k = hidden unit
+// (tensor-memory lane) and q = 4 of the block's 16 trajectories, whose h (dh)
+// it keeps in registers, and a seventeenth warp that issues copies and MMAs.  An
+// operand stands in shared memory as [part][half][k][8 trajectories] (MN-major,
+// N group stride 16 K bytes), so each part is also the operand image of the
+// weight gradients, whose K runs over (slot, trajectory): the issuing warp
+// stores it with one bulk copy and the epilogue never touches it.
 //
 // Blocks take trajectories of similar length (a counting sort by length), so
 // few of a block's 16 rows idle, and time steps are stored compactly.
 //
-// What bounds it: the chain of steps.  A step is 24 MMAs (M = 128, N = 48, K =
-// 16) on the previous step's result, a commit, the tensor-memory loads and the
-// gate math; the input products of the next step run under the gate math.
+// What bounds it: the chain of steps.  A forward step (1.55 us) is 24 MMAs (M =
+// 128, N = 48, K = 16, about 40 cycles each) on the previous step's result, a
+// commit, the tensor-memory loads (370 cycles), the gate math (900) and the
+// operand stores (110); the input products of the next step run under the gate
+// math.  A backward step (1.7 us) has 24 MMAs on the chain and 24 (dA) beside it.
+// 48 KB leave and 40 KB enter the SM a step, all by bulk copies off the chain.
+// Measured, 1,024 pairs of 20..200 points (128 blocks): forward 309 us, backward
+// 347 us.  With the weights in shared memory (64 cycles an MMA: bound by reading
+// A; 128 for the 64-row dA), eight values a thread and every value stored and
+// loaded by the epilogue: about 560 us each.
 #include <cstdio>
 
 #include "tsm.h"
@@ -39,69 +46,81 @@ namespace enc {
 namespace U = tsm::umma;
 
 constexpr int NN = 3 * TB;             // MMA N: three parts of 16 trajectories
-constexpr int KG = NN * 16;            // bytes of 8 K rows of an operand (the K-group stride): 768
-constexpr int A_OP = C1 / 8 * KG;      // 6,144
-constexpr int H_OP = HD / 8 * KG;      // 12,288
-constexpr int G_OP = G3 / 8 * KG;      // 36,864
-constexpr int EPI = 256;               // epilogue threads
+constexpr int A_PARTB = C1 * TB * 2;   // bytes of one part of the operands: 2,048
+constexpr int H_PARTB = HD * TB * 2;   // 4,096
+constexpr int A_OP = 3 * A_PARTB;      // 6,144
+constexpr int H_OP = 3 * H_PARTB;      // 12,288
+constexpr int EPI = 512;               // epilogue threads
 constexpr int THREADS = EPI + 32;      // + the issuing warp
 constexpr int NBUF = 3;                // a-operand buffers of the forward
-constexpr int W_HH = HD * HD * 2;      // one gate's Whh tile: 32 KB
-constexpr int W_IH = HD * C1 * 2;      // one gate's Wih tile: 16 KB
+constexpr int C_OP = 5 * HD * TB * 4;  // what BPTT reads of a step: 40,960
 constexpr long long WAIT_CYCLES = 2000000000LL;  // ~1 s of SM clocks
 // status bits
 constexpr int ERR_FWD_COPY = 256, ERR_FWD_MMA = 512, ERR_BWD_MMA = 1024, ERR_HELD = 128;
 
-__device__ __forceinline__ uint64_t op_desc(uint32_t saddr) { return U::smem_desc(saddr, KG, 128); }
+// Descriptor of an operand of `rows` K rows; a K step of 16 is 256 bytes on.
+__device__ __forceinline__ uint64_t op_desc(uint32_t saddr, int rows) { return U::smem_desc(saddr, 128, rows * 16); }
 
-__device__ __forceinline__ float sigm(float x) { return 1.f / (1.f + expf(-x)); }
+// 2^x and 1 / x to about 2 ulp.
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rcp(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+constexpr float LOG2E = 1.44269504f;
+// Within 1.2e-7 of the sigmoid: an error of 2^-24 |x| in the exponent and of 2
+// ulp in the power are multiplied by s (1 - s) <= 1/4.
+__device__ __forceinline__ float sigm(float x) { return rcp(1.f + ex2(-LOG2E * x)); }
 
-// Eight values as three BF16 parts, x = hi + mid + lo.
+// Two values as three BF16 parts each, x = hi + mid + lo.
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&v);
 }
 __device__ __forceinline__ float lo_of(uint32_t u) { return __uint_as_float(u << 16); }
 __device__ __forceinline__ float hi_of(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
-__device__ __forceinline__ void split8(const float (&v)[8], uint4& hi, uint4& mid, uint4& lo) {
-    uint32_t h[4], m[4], l[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float a = v[2 * i], b = v[2 * i + 1];
-        h[i] = pack2(a, b);
-        const float a1 = a - lo_of(h[i]), b1 = b - hi_of(h[i]);
-        m[i] = pack2(a1, b1);
-        l[i] = pack2(a1 - lo_of(m[i]), b1 - hi_of(m[i]));
+__device__ __forceinline__ void split2(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
+    h = pack2(a, b);
+    const float a1 = a - lo_of(h), b1 = b - hi_of(h);
+    m = pack2(a1, b1);
+    l = pack2(a1 - lo_of(m), b1 - hi_of(m));
+}
+// The three parts of this thread's four trajectories.
+struct Split {
+    uint2 part[3];
+    __device__ __forceinline__ explicit Split(const float (&v)[4]) {
+        split2(v[0], v[1], part[0].x, part[1].x, part[2].x);
+        split2(v[2], v[3], part[0].y, part[1].y, part[2].y);
     }
-    hi = make_uint4(h[0], h[1], h[2], h[3]);
-    mid = make_uint4(m[0], m[1], m[2], m[3]);
-    lo = make_uint4(l[0], l[1], l[2], l[3]);
-}
-// K row k of an operand: the three parts of this thread's 8 trajectories.
-__device__ __forceinline__ void put_op(unsigned char* op, int k, int half, const uint4& hi, const uint4& mid,
-                                       const uint4& lo) {
-    unsigned char* d = op + (k >> 3) * KG + half * 128 + (k & 7) * 16;
-    *reinterpret_cast<uint4*>(d) = hi;
-    *reinterpret_cast<uint4*>(d + 256) = mid;
-    *reinterpret_cast<uint4*>(d + 512) = lo;
-}
-// One group row of an image: [group][rows][8] BF16.
-__device__ __forceinline__ void put_img(unsigned char* img, int64_t group, int rows, int r, const uint4& v) {
-    *reinterpret_cast<uint4*>(img + ((group * rows + r) << 4)) = v;
+    // to K row k of an operand of HD rows
+    __device__ __forceinline__ void put(unsigned char* op, int k, int q) const {
+        unsigned char* d = op + (q >> 1) * (HD * 16) + k * 16 + (q & 1) * 8;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(d + i * H_PARTB) = part[i];
+    }
+};
+// This thread's zeros in the image [group][HD][8] of one slot.
+__device__ __forceinline__ void zero_img(unsigned char* img, int64_t slot, int k, int q) {
+    *reinterpret_cast<uint2*>(img + (((2 * slot + (q >> 1)) * HD + k) << 4) + (q & 1) * 8) = make_uint2(0, 0);
 }
 
-// The sum of the three parts' results, 8 columns from `col` (this thread's
-// lane and half; parts 16 columns apart).
+// The sum of the three parts' results, 4 columns from `col` (this thread's
+// lane and trajectories; parts 16 columns apart).
 struct Parts {
-    uint32_t r[3][8];
+    uint32_t r[3][4];
     __device__ __forceinline__ void load(uint32_t taddr) {
         __syncwarp();
 #pragma unroll
-        for (int i = 0; i < 3; ++i) U::ld8(taddr + 16 * i, r[i]);
+        for (int i = 0; i < 3; ++i) U::ld4(taddr + 16 * i, r[i]);
     }
     __device__ __forceinline__ void wait() {
 #pragma unroll
-        for (int i = 0; i < 3; ++i) U::wait_ld8(r[i]);
+        for (int i = 0; i < 3; ++i) U::wait_ld4(r[i]);
     }
     __device__ __forceinline__ float sum(int s) const {
         return __uint_as_float(r[0][s]) + (__uint_as_float(r[1][s]) + __uint_as_float(r[2][s]));
@@ -170,8 +189,8 @@ __global__ void __launch_bounds__(1024) train_plan(const int32_t* __restrict__ l
     if (tid == 0) slot0[blocks] = carry;
 }
 
-// conv + relu of every slot: the recurrence's operand, the weight gradient's
-// images and the relu's sign bits.  CTA = (block, 16 slots); thread (half, c).
+// conv + relu of every slot: the operand of the recurrence and of the weight
+// gradient, and the relu's sign bits.  CTA = (block, 16 slots); thread (half, c).
 // Steps at or past a trajectory's length are zero.
 constexpr int CV_T = 16;
 __global__ void __launch_bounds__(128) train_conv(const float2* __restrict__ pts, const int64_t* __restrict__ off,
@@ -211,22 +230,27 @@ __global__ void __launch_bounds__(128) train_conv(const float2* __restrict__ pts
             a[e] = t < n_s[s] ? fmaxf(acc, 0.f) : 0.f;
             on |= (a[e] > 0.f ? 1u : 0u) << e;
         }
-        uint4 hi, mid, lo;
-        split8(a, hi, mid, lo);
+        uint32_t part[3][4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) split2(a[2 * e], a[2 * e + 1], part[0][e], part[1][e], part[2][e]);
         const int64_t u = u0 + t, g = 2 * u + half;
-        put_op(w.a_op + u * A_OP, c, half, hi, mid, lo);
-        put_img(w.a_hi, g, C1, c, hi);
-        put_img(w.a_lo, g, C1, c, mid);
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            *reinterpret_cast<uint4*>(w.a_op + u * A_OP + i * A_PARTB + (half * C1 + c) * 16) =
+                make_uint4(part[i][0], part[i][1], part[i][2], part[i][3]);
         w.a_on[g * C1 + c] = (unsigned char)on;
     }
 }
 
-// Shared memory of the forward: Whh (3 tiles), Wih (3 tiles), h, a (NBUF buffers), barriers
-constexpr int F_WHH = 0, F_WIH = F_WHH + 3 * W_HH, F_H = F_WIH + 3 * W_IH, F_A = F_H + H_OP, F_BAR = F_A + NBUF * A_OP,
-              F_SMEM = F_BAR + 64;
+// Shared memory of the forward: h (two buffers), a (NBUF buffers), what BPTT
+// reads (three buffers), barriers.  (More than half an SM's: a block needs all
+// of tensor memory.)
+constexpr int F_H = 0, F_A = F_H + 2 * H_OP, F_C = F_A + NBUF * A_OP, F_BAR = F_C + 3 * C_OP, F_SMEM = F_BAR + 128;
 static_assert(F_SMEM + 1024 <= 227 * 1024, "train_gru_fwd shared memory");
-constexpr uint32_t F_COLS = 512;  // two sets of accumulators r, z, n (hidden), n (input), 48 columns each
-constexpr uint32_t F_SET = 4 * NN;
+// Tensor memory: Whh (3 gates, K = 128), Wih (3 gates, K = 64), accumulators r, z, n (hidden), n (input)
+constexpr uint32_t COLS = 512;
+constexpr uint32_t F_WHH = 0, F_WIH = F_WHH + 3 * HD / 2, F_ACC = F_WIH + 3 * C1 / 2;
+static_assert(F_ACC + 4 * NN <= COLS, "train_gru_fwd tensor memory");
 
 __global__ void __launch_bounds__(THREADS, 1) train_gru_fwd(const int32_t* __restrict__ len, int T,
                                                             const __nv_bfloat16* __restrict__ wq,
@@ -236,25 +260,16 @@ __global__ void __launch_bounds__(THREADS, 1) train_gru_fwd(const int32_t* __res
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ int n_s[TB], b_s[TB], busy;
     const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(sm));
-    // mbarriers: a step's products done, its h written, a-buffer i landed, the last products done
-    const uint32_t hbar = sbase + F_BAR, rbar = hbar + 8, abar = hbar + 16, last = abar + 8 * NBUF;
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + F_BAR + 56);
+    // mbarriers: a step's products done, loaded, its h written, a-buffer i landed, the last products done, the last values written
+    const uint32_t hbar = sbase + F_BAR, lbar = hbar + 8, rbar = hbar + 16, abar = hbar + 24, last = abar + 8 * NBUF, fin = last + 8;
+    constexpr int SLOT = F_BAR + 24 + 8 * NBUF + 16;
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + SLOT);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int k = 32 * (warp & 3) + lane, half = warp >> 2;
+    const int k = 32 * (warp & 3) + lane, q = warp >> 2;
     const int blk = blockIdx.x;
     const int64_t u0 = w.slot0[blk];
     const int nt = w.slot0[blk + 1] - (int)u0;
 
-    for (int e = tid; e < G3 * (HD / 8); e += THREADS) {
-        const int r = e / (HD / 8), c = e % (HD / 8);
-        *reinterpret_cast<uint4*>(sm + F_WHH + (r / HD) * W_HH + U::core_offset(r % HD, 8 * c, HD)) =
-            *reinterpret_cast<const uint4*>(wq + OFF_WHH + r * HD + 8 * c);
-    }
-    for (int e = tid; e < G3 * (C1 / 8); e += THREADS) {
-        const int r = e / (C1 / 8), c = e % (C1 / 8);
-        *reinterpret_cast<uint4*>(sm + F_WIH + (r / HD) * W_IH + U::core_offset(r % HD, 8 * c, HD)) =
-            *reinterpret_cast<const uint4*>(wq + OFF_WIH + r * C1 + 8 * c);
-    }
     for (int e = tid; e < H_OP / 16; e += THREADS) *reinterpret_cast<uint4*>(sm + F_H + 16 * e) = make_uint4(0, 0, 0, 0);
     if (tid < TB) {
         const int b = w.perm[blk * TB + tid];
@@ -263,18 +278,37 @@ __global__ void __launch_bounds__(THREADS, 1) train_gru_fwd(const int32_t* __res
     }
     if (tid == 0) {
         U::mbar_init(hbar, 1);
+        U::mbar_init(lbar, EPI / 32);
         U::mbar_init(rbar, EPI / 32);
+        U::mbar_init(fin, EPI / 32);
         for (int i = 0; i < NBUF; ++i) U::mbar_init(abar + 8 * i, 1);
         U::mbar_init(last, 1);
         busy = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) U::tmem_alloc(sbase + F_BAR + 56, F_COLS);
+    if (warp == 0) U::tmem_alloc(sbase + SLOT, COLS);
     U::fence_smem_async();
     U::fence_before_sync();
     __syncthreads();
     U::fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    if (warp < EPI / 32) {  // the weights: lane = row of a gate, 16 K a write
+        const uint32_t tw = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+        constexpr int NH = 3 * HD / 16, NI = 3 * C1 / 16;
+        for (int i = q; i < NH + NI; i += 4) {
+            const int j = i - NH;
+            const __nv_bfloat16* src = i < NH ? wq + OFF_WHH + (i / (HD / 16) * HD + k) * HD + i % (HD / 16) * 16
+                                              : wq + OFF_WIH + (j / (C1 / 16) * HD + k) * C1 + j % (C1 / 16) * 16;
+            const uint4 x = *reinterpret_cast<const uint4*>(src), y = *reinterpret_cast<const uint4*>(src + 8);
+            const uint32_t r[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+            __syncwarp();
+            U::st8(tw + F_WHH + 8 * i, r);  // (Wih's columns follow Whh's)
+        }
+        U::wait_st();
+    }
+    U::fence_before_sync();
+    __syncthreads();
+    U::fence_after_sync();
     int tmax = 0;
     for (int s = 0; s < TB; ++s) tmax = max(tmax, n_s[s]);
 
@@ -282,9 +316,7 @@ __global__ void __launch_bounds__(THREADS, 1) train_gru_fwd(const int32_t* __res
         if (tmax > 0) {  // the whole warp runs this, its leader issues
             constexpr uint32_t id = U::idesc_bf16_f32_bmn(HD, NN);
             const uint32_t leader = U::elect_leader();
-            const uint64_t whh = U::smem_desc(sbase + F_WHH, HD * 16, 128), wih = U::smem_desc(sbase + F_WIH, HD * 16, 128);
-            const uint64_t hop = op_desc(sbase + F_H);
-            auto step_of = [](int bytes) { return (uint64_t)(bytes >> 4); };  // descriptor increment of a start address
+            const uint32_t acc = tmem + F_ACC;
             int loaded = 0;
             auto load_a = [&](int t) {
                 const uint32_t bar = abar + 8 * (t % NBUF);
@@ -299,16 +331,18 @@ __global__ void __launch_bounds__(THREADS, 1) train_gru_fwd(const int32_t* __res
                 return (bool)__all_sync(0xffffffffu, U::mbar_wait(bar, (uint32_t)(parity & 1), wait_cycles));
             };
             auto a_landed = [&](int t) { return waited(abar + 8 * (t % NBUF), t / NBUF); };
-            // the input products of step t into its accumulator set
+            auto store_c = [&](int t) {
+                U::bulk_store(reinterpret_cast<unsigned char*>(w.cache) + (u0 + t) * C_OP, sbase + F_C + t % 3 * C_OP, C_OP);
+            };
+            // the input products of step t
             auto input_mmas = [&](int t) {
-                const uint32_t d = tmem + (t & 1) * F_SET;
-                const uint64_t a = op_desc(sbase + F_A + (t % NBUF) * A_OP);
+                const uint64_t a = op_desc(sbase + F_A + (t % NBUF) * A_OP, C1);
 #pragma unroll
-                for (int g = 0; g < 3; ++g)
+                for (int ks = 0; ks < C1 / 16; ++ks)
 #pragma unroll
-                    for (int ks = 0; ks < C1 / 16; ++ks)
-                        U::mma_bf16_warp(d + (g == 2 ? 3 * NN : g * NN), wih + step_of(g * W_IH + ks * 2 * (HD * 16)),
-                                         a + step_of(ks * 2 * KG), id, ks, leader);
+                    for (int g = 0; g < 3; ++g)
+                        U::mma_bf16_warp_ta(acc + (g == 2 ? 3 : g) * NN, tmem + F_WIH + g * (C1 / 2) + ks * 8, a + ks * 16,
+                                            id, ks, leader);
             };
             for (int t = 0; t < min(NBUF - 1, tmax); ++t) load_a(t);
             int err = a_landed(0) ? 0 : ERR_FWD_COPY;
@@ -319,20 +353,29 @@ __global__ void __launch_bounds__(THREADS, 1) train_gru_fwd(const int32_t* __res
                     err = ERR_FWD_MMA;
                     break;
                 }
+                U::fence_smem_async();
                 U::fence_after_sync();
-                const uint32_t d = tmem + (t & 1) * F_SET;
+                const uint32_t hs = sbase + F_H + (t & 1) * H_OP;
+                const uint64_t hop = op_desc(hs, HD);
 #pragma unroll
-                for (int g = 0; g < 3; ++g)
+                for (int ks = 0; ks < HD / 16; ++ks)
 #pragma unroll
-                    for (int ks = 0; ks < HD / 16; ++ks)
-                        U::mma_bf16_warp(d + g * NN, whh + step_of(g * W_HH + ks * 2 * (HD * 16)),
-                                         hop + step_of(ks * 2 * KG), id, (g < 2 || ks > 0) ? 1u : 0u, leader);
-                if (leader) U::commit(hbar);
+                    for (int g = 0; g < 3; ++g)
+                        U::mma_bf16_warp_ta(acc + g * NN, tmem + F_WHH + g * (HD / 2) + ks * 8, hop + ks * 16, id,
+                                            (g < 2 || ks > 0) ? 1u : 0u, leader);
+                if (leader) {  // the weight gradient's images of h before this step
+                    U::bulk_store(w.h_hi + (u0 + t) * H_PARTB, hs, H_PARTB);
+                    U::bulk_store(w.h_lo + (u0 + t) * H_PARTB, hs + H_PARTB, H_PARTB);
+                    if (t > 1) store_c(t - 2);  // written before h of step t - 1
+                    U::bulk_commit();
+                    U::bulk_wait_read_but_last();  // (the other buffer, which the epilogue writes next)
+                    U::commit(hbar);
+                }
                 __syncwarp();
                 // a free buffer: its last reader, step t - 1, is done (h of that step is written)
                 if (t + NBUF - 1 < tmax) load_a(t + NBUF - 1);
-                if (t + 1 < tmax) {  // under this step's gate math
-                    if (a_landed(t + 1)) {
+                if (t + 1 < tmax) {  // under this step's gate math, once its accumulators are loaded
+                    if (waited(lbar, t) && a_landed(t + 1)) {
                         U::fence_after_sync();
                         input_mmas(t + 1);
                     } else {
@@ -340,12 +383,26 @@ __global__ void __launch_bounds__(THREADS, 1) train_gru_fwd(const int32_t* __res
                     }
                 }
             }
+            if (!err && waited(fin, 0)) {  // the last two steps' values
+                U::fence_smem_async();
+                if (leader) {
+                    if (tmax > 1) store_c(tmax - 2);
+                    store_c(tmax - 1);
+                    U::bulk_commit();
+                }
+                __syncwarp();
+            } else if (!err) {
+                err = ERR_FWD_MMA;
+            }
             // nothing of this CTA may be in flight when it exits
             if (err) {
                 if (leader) atomicOr(status, err);
                 for (int i = max(0, loaded - NBUF); i < loaded; ++i) a_landed(i);
             }
-            if (leader) U::commit(last);
+            if (leader) {
+                U::bulk_wait();
+                U::commit(last);
+            }
             __syncwarp();
             if (!waited(last, 0) && leader) {
                 atomicOr(status, ERR_HELD);
@@ -353,12 +410,12 @@ __global__ void __launch_bounds__(THREADS, 1) train_gru_fwd(const int32_t* __res
             }
         }
     } else {
-        const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 8 * half;
-        int n[8];
-        float h[8];
+        const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + F_ACC + 4 * q;
+        int n[4];
+        float h[4];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            n[e] = n_s[8 * half + e];
+        for (int e = 0; e < 4; ++e) {
+            n[e] = n_s[4 * q + e];
             h[e] = 0.f;
         }
         const float br = p[OFF_BIH + k] + p[OFF_BHH + k], bz = p[OFF_BIH + HD + k] + p[OFF_BHH + HD + k];
@@ -371,19 +428,21 @@ __global__ void __launch_bounds__(THREADS, 1) train_gru_fwd(const int32_t* __res
                 break;
             }
             U::fence_after_sync();
-            const uint32_t ta = tl + (t & 1) * F_SET;
             Parts pr, pz, ph, pi;
-            pr.load(ta);
-            pz.load(ta + NN);
-            ph.load(ta + 2 * NN);
-            pi.load(ta + 3 * NN);
+            pr.load(tl);
+            pz.load(tl + NN);
+            ph.load(tl + 2 * NN);
+            pi.load(tl + 3 * NN);
             pr.wait();
             pz.wait();
             ph.wait();
             pi.wait();
-            float vr[8], vz[8], vn[8], vg[8], hp[8];
+            U::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) U::mbar_arrive(lbar);
+            float vr[4], vz[4], vn[4], vg[4], hp[4];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
+            for (int e = 0; e < 4; ++e) {
                 vr[e] = sigm(pr.sum(e) + br);
                 vz[e] = sigm(pz.sum(e) + bz);
                 vg[e] = ph.sum(e) + bnh;
@@ -391,37 +450,31 @@ __global__ void __launch_bounds__(THREADS, 1) train_gru_fwd(const int32_t* __res
                 hp[e] = h[e];
                 if (t < n[e]) h[e] = (1.f - vz[e]) * vn[e] + vz[e] * h[e];
             }
-            uint4 hi, mid, lo;
-            split8(h, hi, mid, lo);
-            put_op(sm + F_H, k, half, hi, mid, lo);
-            U::fence_smem_async();
+            Split(h).put(sm + F_H + ((t + 1) & 1) * H_OP, k, q);
             U::fence_before_sync();
             __syncwarp();
             if (lane == 0) U::mbar_arrive(rbar);
-            // off the chain: what BPTT and the weight gradients read
-            const int64_t u = u0 + t;
-            float* cp = w.cache + ((u * 5 * 2 + half) * HD + k) * 8;
-            auto put8 = [&](int i, const float (&v)[8]) {
-                float4* q = reinterpret_cast<float4*>(cp + (int64_t)i * 2 * HD * 8);
-                q[0] = make_float4(v[0], v[1], v[2], v[3]);
-                q[1] = make_float4(v[4], v[5], v[6], v[7]);
+            // Off the chain: what BPTT reads, copied out two steps later.  (Stored
+            // from here, 40 KB a step stalled the warps for 1,200 cycles.)
+            unsigned char* cp = sm + F_C + t % 3 * C_OP + (q * HD + k) * 16;
+            auto put4 = [&](int i, const float (&v)[4]) {
+                *reinterpret_cast<float4*>(cp + i * (C_OP / 5)) = make_float4(v[0], v[1], v[2], v[3]);
             };
-            put8(0, vr);
-            put8(1, vz);
-            put8(2, vn);
-            put8(3, vg);
-            put8(4, hp);
-            split8(hp, hi, mid, lo);
-            put_img(w.h_hi, 2 * u + half, HD, k, hi);
-            put_img(w.h_lo, 2 * u + half, HD, k, mid);
+            put4(0, vr);
+            put4(1, vz);
+            put4(2, vn);
+            put4(3, vg);
+            put4(4, hp);
         }
+        __syncwarp();
+        if (lane == 0 && !failed) U::mbar_arrive(fin);  // the last step's values written
         if (tmax < nt) {  // the slot that rounds the block up
-            put_img(w.h_hi, 2 * (u0 + nt - 1) + half, HD, k, make_uint4(0, 0, 0, 0));
-            put_img(w.h_lo, 2 * (u0 + nt - 1) + half, HD, k, make_uint4(0, 0, 0, 0));
+            zero_img(w.h_hi, u0 + nt - 1, k, q);
+            zero_img(w.h_lo, u0 + nt - 1, k, q);
         }
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const int b = b_s[8 * half + e];
+        for (int e = 0; e < 4; ++e) {
+            const int b = b_s[4 * q + e];
             if (b >= 0) hl[(int64_t)b * HD + k] = failed ? __int_as_float(0x7fc00000) : h[e];
         }
     }
@@ -429,16 +482,18 @@ __global__ void __launch_bounds__(THREADS, 1) train_gru_fwd(const int32_t* __res
     __syncthreads();
     if (warp == 0 && !busy) {
         U::fence_after_sync();
-        U::tmem_dealloc(tmem, F_COLS);
+        U::tmem_dealloc(tmem, COLS);
     }
 }
 
-// Shared memory of the backward: Whh^T (128 x 384), Wih^T (64 x 384), hidden-side
-// gate gradients (K = 384), input-side n gradients (K = 128), barriers
-constexpr int B_WHH = 0, B_WIH = B_WHH + HD * G3 * 2, B_G = B_WIH + C1 * G3 * 2, B_N = B_G + G_OP, B_BAR = B_N + H_OP,
-              B_SMEM = B_BAR + 64;
+// Shared memory of the backward: the gate gradients r, z, n (input), n
+// (hidden), an operand each, two buffers; the forward's values, two buffers; barriers
+constexpr int B_G = 0, B_SET = 4 * H_OP, B_C = B_G + 2 * B_SET, B_BAR = B_C + 2 * C_OP, B_SMEM = B_BAR + 64;
 static_assert(B_SMEM + 1024 <= 227 * 1024, "train_gru_bwd shared memory");
-constexpr uint32_t B_COLS = 128;  // dh at column 0, dA at 64
+// Tensor memory: Whh^T (lane = k, K = gate rows), Wih^T (lanes 0..63 = c; M = 64 would take the tensor cores twice
+// as long as M = 128), dh, dA
+constexpr uint32_t B_WHH = 0, B_WIH = B_WHH + G3 / 2, B_DH = B_WIH + G3 / 2, B_DA = B_DH + NN;
+static_assert(B_DA + NN <= COLS, "train_gru_bwd tensor memory");
 
 __global__ void __launch_bounds__(THREADS, 1) train_gru_bwd(const int32_t* __restrict__ len, int T,
                                                             const __nv_bfloat16* __restrict__ wq,
@@ -448,25 +503,16 @@ __global__ void __launch_bounds__(THREADS, 1) train_gru_bwd(const int32_t* __res
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ int n_s[TB], b_s[TB], busy;
     const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(sm));
-    // mbarriers: a step's dh products done, its dA products done, its gate gradients written, the last products done
-    const uint32_t hbar = sbase + B_BAR, abar = hbar + 8, rbar = hbar + 16, last = hbar + 24;
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + B_BAR + 32);
+    // mbarriers: a step's dh products done, its dA products done, its gate gradients written, the last products done,
+    // the forward's values landed (one a buffer)
+    const uint32_t hbar = sbase + B_BAR, abar = hbar + 8, rbar = hbar + 16, last = hbar + 24, cbar = hbar + 32;
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + B_BAR + 48);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int k = 32 * (warp & 3) + lane, half = warp >> 2;
+    const int k = 32 * (warp & 3) + lane, q = warp >> 2;
     const int blk = blockIdx.x;
     const int64_t u0 = w.slot0[blk];
     const int nt = w.slot0[blk + 1] - (int)u0;
 
-    for (int e = tid; e < G3 * HD / 2; e += THREADS) {  // Whh[j][k] -> row k, K = j
-        const int j = 2 * (e / HD), kk = e % HD;
-        const __nv_bfloat162 v{wq[OFF_WHH + j * HD + kk], wq[OFF_WHH + (j + 1) * HD + kk]};
-        *reinterpret_cast<__nv_bfloat162*>(sm + B_WHH + U::core_offset(kk, j, HD)) = v;
-    }
-    for (int e = tid; e < G3 * C1 / 2; e += THREADS) {
-        const int j = 2 * (e / C1), c = e % C1;
-        const __nv_bfloat162 v{wq[OFF_WIH + j * C1 + c], wq[OFF_WIH + (j + 1) * C1 + c]};
-        *reinterpret_cast<__nv_bfloat162*>(sm + B_WIH + U::core_offset(c, j, C1)) = v;
-    }
     if (tid < TB) {
         const int b = w.perm[blk * TB + tid];
         b_s[tid] = b;
@@ -477,48 +523,101 @@ __global__ void __launch_bounds__(THREADS, 1) train_gru_bwd(const int32_t* __res
         U::mbar_init(abar, 1);
         U::mbar_init(rbar, EPI / 32);
         U::mbar_init(last, 1);
+        for (int i = 0; i < 2; ++i) U::mbar_init(cbar + 8 * i, 1);
         busy = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) U::tmem_alloc(sbase + B_BAR + 32, B_COLS);
+    if (warp == 0) U::tmem_alloc(sbase + B_BAR + 48, COLS);
     U::fence_smem_async();
     U::fence_before_sync();
     __syncthreads();
     U::fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    if (warp < EPI / 32) {  // the weights, transposed: 16 K (gate rows) a write
+        const uint32_t tw = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+        const unsigned short* whh = reinterpret_cast<const unsigned short*>(wq + OFF_WHH) + k;
+        const unsigned short* wih = reinterpret_cast<const unsigned short*>(wq + OFF_WIH) + k;
+        for (int i = q; i < G3 / 16; i += 4) {
+            uint32_t r[8], x[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int row = 16 * i + 2 * j;
+                r[j] = (uint32_t)whh[row * HD] | (uint32_t)whh[(row + 1) * HD] << 16;
+                x[j] = k < C1 ? (uint32_t)wih[row * C1] | (uint32_t)wih[(row + 1) * C1] << 16 : 0u;
+            }
+            __syncwarp();
+            U::st8(tw + B_WHH + 8 * i, r);
+            U::st8(tw + B_WIH + 8 * i, x);
+        }
+        U::wait_st();
+    }
+    U::fence_before_sync();
+    __syncthreads();
+    U::fence_after_sync();
     int tmax = 0;
     for (int s = 0; s < TB; ++s) tmax = max(tmax, n_s[s]);
 
     if (warp == EPI / 32) {  // MMAs
         if (tmax > 0) {  // the whole warp runs this, its leader issues
-            constexpr uint32_t id_h = U::idesc_bf16_f32_bmn(HD, NN), id_a = U::idesc_bf16_f32_bmn(C1, NN);
+            constexpr uint32_t id = U::idesc_bf16_f32_bmn(HD, NN);
             const uint32_t leader = U::elect_leader();
-            const uint64_t whh = U::smem_desc(sbase + B_WHH, HD * 16, 128), wih = U::smem_desc(sbase + B_WIH, C1 * 16, 128);
-            const uint64_t gop = op_desc(sbase + B_G), nop = op_desc(sbase + B_N);
-            auto step_of = [](int bytes) { return (uint64_t)(bytes >> 4); };  // descriptor increment of a start address
+            const int64_t img_tile = w.slots * H_PARTB;  // bytes between the images of two gates
             auto waited = [&](uint32_t bar, int parity) {
                 return (bool)__all_sync(0xffffffffu, U::mbar_wait(bar, (uint32_t)(parity & 1), wait_cycles));
             };
+            int loaded = 0;
+            auto load_c = [&]() {  // the next step's values of the forward
+                if (loaded == tmax) return;
+                const uint32_t bar = cbar + 8 * (loaded & 1);
+                if (leader) {
+                    U::mbar_arrive_expect_tx(bar, C_OP);
+                    U::bulk_load(sbase + B_C + (loaded & 1) * C_OP,
+                                 reinterpret_cast<const unsigned char*>(w.cache) + (u0 + tmax - 1 - loaded) * C_OP, C_OP, bar);
+                }
+                __syncwarp();
+                ++loaded;
+            };
+            load_c();
+            load_c();
             for (int i = 0; i < tmax; ++i) {
                 if (!waited(rbar, i)) {
                     if (leader) atomicOr(status, ERR_BWD_MMA);
+                    for (int j = max(0, loaded - 2); j < loaded; ++j) waited(cbar + 8 * (j & 1), j / 2);
                     break;
                 }
+                U::fence_smem_async();
                 U::fence_after_sync();
+                const uint32_t gs = sbase + B_G + (i & 1) * B_SET;
+                const uint64_t gop = op_desc(gs, HD);
+                auto mma = [&](uint32_t d, uint32_t a, int kg, int n_op) {  // 16 K: rows 16 kg of the gates r, z, n of one side
+                    const int g = kg / (HD / 16);
+                    U::mma_bf16_warp_ta(d, a + 8 * kg, gop + ((g == 2 ? n_op : g) * H_OP >> 4) + kg % (HD / 16) * 16, id, kg,
+                                        leader);
+                };
 #pragma unroll
-                for (int ks = 0; ks < G3 / 16; ++ks)
-                    U::mma_bf16_warp(tmem, whh + step_of(ks * 2 * (HD * 16)), gop + step_of(ks * 2 * KG), id_h, ks, leader);
+                for (int kg = 0; kg < G3 / 16; ++kg) mma(tmem + B_DH, tmem + B_WHH, kg, 3);
                 if (leader) U::commit(hbar);
                 __syncwarp();
+                load_c();  // into this step's buffer
 #pragma unroll
-                for (int ks = 0; ks < G3 / 16; ++ks)
-                    U::mma_bf16_warp(tmem + 64, wih + step_of(ks * 2 * (C1 * 16)),
-                                     ks < 2 * HD / 16 ? gop + step_of(ks * 2 * KG) : nop + step_of((ks - 2 * HD / 16) * 2 * KG),
-                                     id_a, ks, leader);
-                if (leader) U::commit(abar);
+                for (int kg = 0; kg < G3 / 16; ++kg) mma(tmem + B_DA, tmem + B_WIH, kg, 2);
+                if (leader) {  // the weight gradient's images
+                    const int64_t at = (u0 + tmax - 1 - i) * H_PARTB;
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        U::bulk_store(w.g_hi + g * img_tile + at, gs + g * H_OP, H_PARTB);
+                        U::bulk_store(w.g_lo + g * img_tile + at, gs + g * H_OP + H_PARTB, H_PARTB);
+                    }
+                    U::bulk_commit();
+                    U::bulk_wait_read_but_last();  // (the other buffer, which the epilogue writes next)
+                    U::commit(abar);
+                }
                 __syncwarp();
             }
-            if (leader) U::commit(last);  // nothing of this CTA may be in flight when it exits
+            if (leader) {  // nothing of this CTA may be in flight when it exits
+                U::bulk_wait();
+                U::commit(last);
+            }
             __syncwarp();
             if (!waited(last, 0) && leader) {
                 atomicOr(status, ERR_HELD);
@@ -526,51 +625,29 @@ __global__ void __launch_bounds__(THREADS, 1) train_gru_bwd(const int32_t* __res
             }
         }
     } else {
-        const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 8 * half;
-        int n[8];
-        float dh[8];
+        const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 4 * q;
+        int n[4];
+        float dh[4];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            n[e] = n_s[8 * half + e];
-            const int b = b_s[8 * half + e];
+        for (int e = 0; e < 4; ++e) {
+            n[e] = n_s[4 * q + e];
+            const int b = b_s[4 * q + e];
             dh[e] = b >= 0 ? dhl[(int64_t)b * HD + k] : 0.f;
         }
-        const int64_t img_tile = w.slots * 2 * HD * 16;  // bytes between the images of two gates
-        if (tmax < nt) {
+        if (tmax < nt)
             for (int g = 0; g < 4; ++g) {
-                put_img(w.g_hi + g * img_tile, 2 * (u0 + nt - 1) + half, HD, k, make_uint4(0, 0, 0, 0));
-                put_img(w.g_lo + g * img_tile, 2 * (u0 + nt - 1) + half, HD, k, make_uint4(0, 0, 0, 0));
+                zero_img(w.g_hi + g * w.slots * H_PARTB, u0 + nt - 1, k, q);
+                zero_img(w.g_lo + g * w.slots * H_PARTB, u0 + nt - 1, k, q);
             }
-        }
-        // this thread's cached values of a step, loaded a step ahead
-        float c[5][8];
-        auto load_c = [&](int t) {
-            const float* cp = w.cache + (((u0 + t) * 5 * 2 + half) * HD + k) * 8;
+        // the conv gradient of step t (lanes 0..63), from the loaded accumulators
+        const bool has_dA = (warp & 3) < C1 / 32;
+        auto signs = [&](int t) { return (uint32_t)__ldg(w.a_on + (2 * (u0 + t) + (q >> 1)) * C1 + k); };
+        auto put_dA = [&](int t, const Parts& pa, uint32_t on) {
+            const int64_t u = u0 + t;
+            float v[4];
 #pragma unroll
-            for (int i = 0; i < 5; ++i) {
-                const float4* q = reinterpret_cast<const float4*>(cp + (int64_t)i * 2 * HD * 8);
-                const float4 x = __ldg(q), y = __ldg(q + 1);
-                c[i][0] = x.x; c[i][1] = x.y; c[i][2] = x.z; c[i][3] = x.w;
-                c[i][4] = y.x; c[i][5] = y.y; c[i][6] = y.z; c[i][7] = y.w;
-            }
-        };
-        // the conv gradient of step t (M = 64: rows 16 q .. 16 q + 15 in the first 16 lanes of quarter q)
-        auto put_dA = [&](int t) {
-            Parts pa;
-            pa.load(tl + 64);
-            pa.wait();
-            if (lane < 16) {
-                const int ch = 16 * (warp & 3) + lane;
-                const int64_t g = 2 * (u0 + t) + half;
-                const uint32_t on = w.a_on[g * C1 + ch];
-                float v[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) v[e] = (on >> e & 1u) ? pa.sum(e) : 0.f;
-                float4* q = reinterpret_cast<float4*>(w.dA + (g * C1 + ch) * 8);
-                q[0] = make_float4(v[0], v[1], v[2], v[3]);
-                q[1] = make_float4(v[4], v[5], v[6], v[7]);
-            }
-            __syncwarp();
+            for (int e = 0; e < 4; ++e) v[e] = (on >> (4 * (q & 1) + e) & 1u) ? pa.sum(e) : 0.f;
+            *reinterpret_cast<float4*>(w.dA + ((4 * u + q) * C1 + k) * 4) = make_float4(v[0], v[1], v[2], v[3]);
         };
         auto waited = [&](uint32_t bar, uint32_t parity) {
             const bool ok = __all_sync(0xffffffffu, U::mbar_wait(bar, parity, wait_cycles));
@@ -580,59 +657,79 @@ __global__ void __launch_bounds__(THREADS, 1) train_gru_bwd(const int32_t* __res
         };
         float sr = 0.f, sz = 0.f, sn = 0.f, snh = 0.f;  // bias gradients
         bool ok = true;
-        if (tmax > 0) load_c(tmax - 1);
+        // What a step's gate gradients need besides dh, formed while the previous
+        // step's products run: dn = (1 - z)(1 - n^2) dh, dr = (Whn h + bhn) r (1 - r)
+        // dn, dz = (h - n) z (1 - z) dh
+        float cn[4], cr[4], cz[4], r[4], z[4];
+        auto coefficients = [&](uint32_t i) {
+            if (!waited(cbar + 8 * (i & 1), (i >> 1) & 1)) return false;
+            const float* cp = reinterpret_cast<const float*>(sm + B_C + (i & 1) * C_OP + (q * HD + k) * 16);
+            float c[5][4];
+#pragma unroll
+            for (int j = 0; j < 5; ++j) {
+                const float4 x = *reinterpret_cast<const float4*>(cp + j * (C_OP / 20));
+                c[j][0] = x.x; c[j][1] = x.y; c[j][2] = x.z; c[j][3] = x.w;
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                r[e] = c[0][e];
+                z[e] = c[1][e];
+                const float nn = c[2][e];
+                cn[e] = (1.f - z[e]) * (1.f - nn * nn);
+                cr[e] = c[3][e] * r[e] * (1.f - r[e]);
+                cz[e] = (c[4][e] - nn) * z[e] * (1.f - z[e]);
+            }
+            return true;
+        };
+        if (tmax > 0) ok = coefficients(0);
         for (int t = tmax - 1; t >= 0 && ok; --t) {
             const uint32_t i = (uint32_t)(tmax - 1 - t);  // steps before this one
-            float gr[8], gz[8], gn[8], gh[8], d[8];
+            const uint32_t on = i > 0 && has_dA ? signs(t + 1) : 0;
+            float gr[4], gz[4], gn[4], gh[4], d[4];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
+            for (int e = 0; e < 4; ++e) {
                 const bool live = t < n[e];
-                const float r = c[0][e], z = c[1][e], nn = c[2][e], g = dh[e];
-                const float dn = g * (1.f - z), dz = g * (c[4][e] - nn);
-                const float vn = dn * (1.f - nn * nn);
+                const float g = dh[e], vn = g * cn[e];
                 gn[e] = live ? vn : 0.f;
-                gr[e] = live ? vn * c[3][e] * r * (1.f - r) : 0.f;
-                gz[e] = live ? dz * z * (1.f - z) : 0.f;
-                gh[e] = live ? vn * r : 0.f;
-                d[e] = live ? g * z : g;  // past its end a trajectory's dh passes through
+                gr[e] = live ? vn * cr[e] : 0.f;
+                gz[e] = live ? g * cz[e] : 0.f;
+                gh[e] = live ? vn * r[e] : 0.f;
+                d[e] = live ? g * z[e] : g;  // past its end a trajectory's dh passes through
                 sr += gr[e];
                 sz += gz[e];
                 sn += gn[e];
                 snh += gh[e];
             }
-            if (t > 0) load_c(t - 1);
-            uint4 hi[4], mid[4], lo[4];
-            split8(gr, hi[0], mid[0], lo[0]);
-            split8(gz, hi[1], mid[1], lo[1]);
-            split8(gn, hi[2], mid[2], lo[2]);
-            split8(gh, hi[3], mid[3], lo[3]);
-            if (i > 0) {  // the previous step's dA products have read the operand
+            const Split xr(gr), xz(gz), xn(gn), xh(gh);
+            Parts pa;
+            if (i > 0) {  // the previous step's dA products are done (and the copies out of this step's buffer)
                 if (!(ok = waited(abar, (i - 1) & 1))) break;
-                put_dA(t + 1);
+                if (has_dA) pa.load(tl + B_DA);
             }
-            put_op(sm + B_G, k, half, hi[0], mid[0], lo[0]);
-            put_op(sm + B_G, HD + k, half, hi[1], mid[1], lo[1]);
-            put_op(sm + B_G, 2 * HD + k, half, hi[3], mid[3], lo[3]);
-            put_op(sm + B_N, k, half, hi[2], mid[2], lo[2]);
-            U::fence_smem_async();
+            unsigned char* g_op = sm + B_G + (i & 1) * B_SET;
+            xr.put(g_op, k, q);
+            xz.put(g_op + H_OP, k, q);
+            xn.put(g_op + 2 * H_OP, k, q);
+            xh.put(g_op + 3 * H_OP, k, q);
+            if (i > 0 && has_dA) pa.wait();
             U::fence_before_sync();
             __syncwarp();
             if (lane == 0) U::mbar_arrive(rbar);
-            // the weight gradient's images, while the products run
-            const int64_t g2 = 2 * (u0 + t) + half;
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                put_img(w.g_hi + g * img_tile, g2, HD, k, hi[g]);
-                put_img(w.g_lo + g * img_tile, g2, HD, k, mid[g]);
-            }
+            if (i > 0 && has_dA) put_dA(t + 1, pa, on);
+            if (t > 0 && !(ok = coefficients(i + 1))) break;
             if (!(ok = waited(hbar, i & 1))) break;
             Parts pd;
-            pd.load(tl);
+            pd.load(tl + B_DH);
             pd.wait();
 #pragma unroll
-            for (int e = 0; e < 8; ++e) dh[e] = d[e] + pd.sum(e);
+            for (int e = 0; e < 4; ++e) dh[e] = d[e] + pd.sum(e);
         }
-        if (tmax > 0 && ok && waited(abar, (uint32_t)(tmax - 1) & 1)) put_dA(0);
+        if (tmax > 0 && ok && waited(abar, (uint32_t)(tmax - 1) & 1) && has_dA) {
+            Parts pa;
+            pa.load(tl + B_DA);
+            pa.wait();
+            put_dA(0, pa, signs(0));
+        }
         if (tmax > 0) {
             atomicAdd(gbih + k, sr);
             atomicAdd(gbih + HD + k, sz);
@@ -646,7 +743,7 @@ __global__ void __launch_bounds__(THREADS, 1) train_gru_bwd(const int32_t* __res
     __syncthreads();
     if (warp == 0 && !busy) {
         U::fence_after_sync();
-        U::tmem_dealloc(tmem, B_COLS);
+        U::tmem_dealloc(tmem, COLS);
     }
 }
 
@@ -685,16 +782,13 @@ __global__ void __launch_bounds__(CB_THREADS) train_conv_bwd(const float2* __res
 #pragma unroll 4
     for (int t = t0; t < t1; ++t) {
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const float4* g = reinterpret_cast<const float4*>(w.dA + ((2 * (u0 + t) + half) * C1 + c) * 8);
-            const float4 g0 = __ldg(g), g1 = __ldg(g + 1);
+        for (int j = 0; j < 4; ++j) {
+            const float4 g = __ldg(reinterpret_cast<const float4*>(w.dA + ((4 * (u0 + t) + j) * C1 + c) * 4));
             if (wt) {
-                const float4* x = reinterpret_cast<const float4*>(xs + (t - t0 + k) * CB_U + i * CB_I + 8 * half);
-                const float4 x0 = x[0], x1 = x[1];
-                acc = fmaf(g0.x, x0.x, fmaf(g0.y, x0.y, fmaf(g0.z, x0.z, fmaf(g0.w, x0.w, acc))));
-                acc = fmaf(g1.x, x1.x, fmaf(g1.y, x1.y, fmaf(g1.z, x1.z, fmaf(g1.w, x1.w, acc))));
+                const float4 x = *reinterpret_cast<const float4*>(xs + (t - t0 + k) * CB_U + i * CB_I + 4 * j);
+                acc = fmaf(g.x, x.x, fmaf(g.y, x.y, fmaf(g.z, x.z, fmaf(g.w, x.w, acc))));
             } else {
-                acc += ((g0.x + g0.y) + (g0.z + g0.w)) + ((g1.x + g1.y) + (g1.z + g1.w));
+                acc += (g.x + g.y) + (g.z + g.w);
             }
         }
     }
@@ -724,8 +818,6 @@ int64_t train_layout(int B, int T, unsigned char* base, TrainWs* w) {
     x.perm = reinterpret_cast<int32_t*>(take((int64_t)x.blocks * TB * 4));
     x.slot0 = reinterpret_cast<int32_t*>(take((int64_t)(x.blocks + 1) * 4));
     x.a_op = take(x.slots * A_OP);
-    x.a_hi = take(groups * C1 * 16);
-    x.a_lo = take(groups * C1 * 16);
     x.a_on = take(groups * C1);
     x.h_hi = take(groups * HD * 16);
     x.h_lo = take(groups * HD * 16);

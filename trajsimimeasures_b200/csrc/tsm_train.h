@@ -18,13 +18,12 @@ constexpr int TB = 16;  // trajectories per block of the recurrences
 struct TrainWs {
     int32_t* perm;   // [blocks * TB] trajectory of each row, -1 past the batch
     int32_t* slot0;  // [blocks + 1]
-    unsigned char* a_op;              // [slot] conv output as the recurrence's operand: 3 BF16 parts, 6 KB
-    unsigned char *a_hi, *a_lo;       // [group][64][8] BF16: conv output, parts hi and lo
+    unsigned char* a_op;              // [slot][3 parts][half][64][8] BF16: conv output
     unsigned char* a_on;              // [group][64] bit s: conv output of trajectory s positive
-    unsigned char *h_hi, *h_lo;       // [group][128][8] BF16: hidden state before the step
-    float* cache;                     // [slot][5][2][128][8]: r, z, n, Whn h + bhn, h before the step
+    unsigned char *h_hi, *h_lo;       // [group][128][8] BF16: hidden state before the step, first two parts
+    float* cache;                     // [slot][5][4][128][4]: r, z, n, Whn h + bhn, h before the step
     unsigned char *g_hi, *g_lo;       // [4][group][128][8] BF16: gate gradients r, z, n (input), n (hidden)
-    float* dA;                        // [group][64][8] gradient of the conv output (before the relu)
+    float* dA;                        // [slot][4][64][4] gradient of the conv output (before the relu)
     int64_t slots;                    // capacity
     int blocks;
 };

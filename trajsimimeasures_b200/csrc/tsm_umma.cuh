@@ -80,6 +80,18 @@ __device__ __forceinline__ void mma_bf16_warp(uint32_t tmem_d, uint64_t adesc, u
         :
         : "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader));
 }
+// The same with A in tensor memory: 128 lanes (rows of A), two consecutive K a
+// 32-bit column, even K in the low half.
+__device__ __forceinline__ void mma_bf16_warp_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                                 uint32_t accumulate, uint32_t leader) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
+        :
+        : "r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader));
+}
 // 1 in one lane of the converged warp, 0 in the others.
 __device__ __forceinline__ uint32_t elect_leader() {
     uint32_t l;
@@ -146,6 +158,18 @@ __device__ __forceinline__ void bulk_load(uint32_t dst_saddr, const void* src, u
                  : "memory");
 }
 
+// Bulk copy of `bytes` from shared to this GPU's global memory (same rules),
+// in the calling thread's bulk group; bulk_commit closes the group,
+// bulk_wait_read_but_last waits until the sources of all groups but the last
+// may be overwritten, bulk_wait until all copies are complete.
+__device__ __forceinline__ void bulk_store(void* dst, uint32_t src_saddr, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src_saddr), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read_but_last() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 // Tensor-memory allocation by one whole warp: ncols columns (a power of two
 // >= 32); the address is written to shared memory at slot_saddr.
 __device__ __forceinline__ void tmem_alloc(uint32_t slot_saddr, uint32_t ncols) {
@@ -171,18 +195,26 @@ __device__ __forceinline__ void ld16(uint32_t taddr, uint32_t (&r)[16]) {
         : "r"(taddr));
 }
 
-// The same for 8 columns.
-__device__ __forceinline__ void ld8(uint32_t taddr, uint32_t (&r)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+// The same for 4 columns.
+__device__ __forceinline__ void ld4(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(taddr));
 }
-__device__ __forceinline__ void wait_ld8(uint32_t (&r)[8]) {
+__device__ __forceinline__ void wait_ld4(uint32_t (&r)[4]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3])
                  :
                  : "memory");
 }
+// 8 consecutive columns of this thread's lane written; wait_st waits for all of
+// this thread's writes.
+__device__ __forceinline__ void st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]),
+                 "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+__device__ __forceinline__ void wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // Waits for this thread's tensor-memory loads; r (one load's registers) is
 // tied to the wait.  Call it once per loaded array (the later calls return at

@@ -13,8 +13,8 @@
 // with FP32 accumulation: three MMAs per K step, about 2^-16 relative per
 // product (the split-product method of Markidis et al., IPDPSW 2018).
 //
-// The recurrences write the hi and lo images themselves (tsm_train.cu), K-major
-// core-matrix layout (tsm_umma.cuh), 16 K per slot.  One kernel, split-K over
+// The operands of the recurrences are the hi and lo images (tsm_train.cu),
+// K-major core-matrix layout (tsm_umma.cuh), 16 K per slot.  One kernel, split-K over
 // the CTAs: CTA (m tile of 128 rows of j, K range) streams both products'
 // operands through a four-stage ring (cp.async.bulk, mbarrier transaction
 // counts), one thread issues six MMAs per K step into four accumulators, and
@@ -122,8 +122,11 @@ __global__ void __launch_bounds__(THREADS, 1) wg_kernel(
                 load(S_GHHI, w.g_hi + 3 * tile, M_PART);
                 load(S_GHLO, w.g_lo + 3 * tile, M_PART);
             }
-            load(S_AHI, w.a_hi, A_PART);
-            load(S_ALO, w.a_lo, A_PART);
+            for (int j = 0; j < 2; ++j) {  // a slot's three parts stand together
+                const unsigned char* src = w.a_op + (2 * s + j) * (3 * A_PART / 2);
+                U::bulk_load(st + S_AHI + j * (A_PART / 2), src, A_PART / 2, full(slot));
+                U::bulk_load(st + S_ALO + j * (A_PART / 2), src + A_PART / 2, A_PART / 2, full(slot));
+            }
             load(S_HHI, w.h_hi, H_PART);
             load(S_HLO, w.h_lo, H_PART);
         }
