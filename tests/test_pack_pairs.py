@@ -19,7 +19,7 @@ def _pack(a1, la, a2, lb, mode, origin=None):
     return rc, off, ln, pts
 
 
-@pytest.mark.parametrize("n,L", [(1, 1), (7, 13), (1400, 230)])  # the last: about 290,000 points, several threads
+@pytest.mark.parametrize("n,L", [(1, 1), (7, 13), (5200, 230)])  # the last: about 1.8 million points, several threads
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("layout", ["plain", "wide", "transposed", "reversed"])
 @pytest.mark.parametrize("mode", [0, 1, 2])

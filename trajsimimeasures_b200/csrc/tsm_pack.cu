@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstring>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "tsm.h"
@@ -33,6 +34,10 @@ void pack_rows(const Side& s, int64_t k0, int64_t k1, const double* origin, bool
         const unsigned char* p = s.base + k * s.traj;
         float* d = dst + 2 * s.off[k];
         if (!origin) {
+            if (std::is_same<T, float>::value && s.pt == 8) {  // as they are
+                if (n > 0) std::memcpy(d, p, (size_t)(8 * n));
+                continue;
+            }
             for (int64_t i = 0; i < n; ++i) {
                 const T* q = reinterpret_cast<const T*>(p + i * s.pt);
                 d[2 * i] = (float)q[0];
@@ -83,11 +88,13 @@ void pack_all(const Side& a, const Side& b, int64_t n, int mode, const double* o
         pack_rows<T>(a, k0, k1, o, per_pair, dst);
         pack_rows<T>(b, k0, k1, o, per_pair, dst);
     };
-    // Threads only where the pass is long: 441,000 points take 404 us in one
-    // thread and 190 in four to six; but 112,000, which take 67 us in three
-    // threads instead of 113 in a loop of nothing else, made a whole call
-    // slower (399 us against 352: threads started on idle cores).
-    int64_t nt = total / 98304;
+    // Threads only where the pass is long: started on idle cores, they cost a call
+    // more than the pass they share.  A call in one thread / in threads of
+    // 262,144 / of 524,288 / of 98,304 points (float64 pairs of 20..200): 1,000
+    // pairs 0.49 ms / - / - / 0.54, 4,096 (0.9 million points) 1.34 / 1.20 / - /
+    // 1.54 (float32 1.11 / 1.21 / - / 1.74), 6,000 (float32) 1.55 / 1.87 / 1.48,
+    // 20,000 12.5 / 5.1 / 5.0.
+    int64_t nt = total / 524288;
     const int64_t hw = (int64_t)std::thread::hardware_concurrency();
     if (nt > 8) nt = 8;
     if (nt > hw) nt = hw;
