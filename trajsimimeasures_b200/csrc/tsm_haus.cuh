@@ -18,9 +18,11 @@
 // the bounds are compared with a margin delta above the rounding error of an
 // evaluation.  With M the extent of the two trajectories' common bounding box
 // and u = 2^-24, an evaluated foot offset differs from the offset to a point
-// of the segment by at most 3 u M per coordinate; delta = 2^-19 M is 7 times
-// the resulting length.  Non-finite coordinates set delta to infinity, which
-// turns every skip off.
+// of the segment by at most 3 u M per coordinate; delta = 2^-19 M + 2^-62 is 7
+// times the resulting length, plus what underflow can take: the approximate
+// square root of a bound flushes squared distances below 2^-126 (lengths below
+// 2^-63) to 0, and a widened bound stays a normal number (2^-124 at least).
+// Non-finite coordinates set delta to infinity, which turns every skip off.
 //
 // What bounds it: issue, and the latency of its warp votes and reductions.  On
 // pairs of random walks of 20..200 points, of 8 groups (both directions) 3.8
@@ -159,7 +161,7 @@ __device__ __forceinline__ float haus_directed(const HausTraj& P, const HausTraj
     if (T.n < 2 || P.n <= 0) return m;
     const int ngrp = (P.n + 31) >> 5, nblk = (T.n + kHausBlk - 1) / kHausBlk, npair = (T.n + 1) >> 1;
     for (int g0 = 0; g0 < ngrp; g0 += 32) {
-        // lane l keeps the bound of group g0 + l and the block it came from
+        // lane l keeps the bound of group g0 + l (0: done; a bound is not, see delta) and the block it came from
         const int ng = min(32, ngrp - g0);
         uint32_t ub = 0;
         int ubb = 0;
@@ -223,7 +225,7 @@ __device__ __forceinline__ float haus_directed(const HausTraj& P, const HausTraj
 // The Hausdorff distance of two staged trajectories.
 __device__ __forceinline__ float haus_pair(const HausTraj& a, const HausTraj& b, int lane) {
     const float w = fmaxf(a.bb.y, b.bb.y) - fminf(a.bb.x, b.bb.x), h = fmaxf(a.bb.w, b.bb.w) - fminf(a.bb.z, b.bb.z);
-    const float delta = 0x1p-19f * (w + h);
+    const float delta = fmaf(0x1p-19f, w + h, 0x1p-62f);
     const float m = haus_directed(a, b, 0.f, delta, lane);
     return __fsqrt_rn(haus_directed(b, a, m, delta, lane));
 }
