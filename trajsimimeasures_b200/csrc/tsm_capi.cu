@@ -8,6 +8,7 @@
 
 #include <cmath>
 #include <cstdarg>
+#include <cstdint>
 #include <cstdio>
 #include <string>
 
@@ -102,8 +103,31 @@ int warps_for(int cap, int extra_bytes) {
     return 1;
 }
 
+// A kernel's static shared memory: a property of the compiled function, looked
+// up once per thread (a table of slots by address, overwritten on a clash).
+cudaError_t static_smem(const void* fn, int& bytes) {
+    struct Known {
+        const void* fn;
+        int bytes;
+    };
+    thread_local Known known[64] = {};
+    Known& k = known[(reinterpret_cast<uintptr_t>(fn) >> 4) % 64];
+    if (k.fn != fn) {
+        cudaFuncAttributes a;
+        const cudaError_t e = cudaFuncGetAttributes(&a, fn);
+        if (e != cudaSuccess) return e;
+        k = {fn, (int)a.sharedSizeBytes};
+    }
+    bytes = k.bytes;
+    return cudaSuccess;
+}
+
+// Opts a kernel in to more shared memory than the default 48 KB, which covers
+// the static and the dynamic part together.
 cudaError_t set_smem(const void* fn, int bytes) {
-    if (bytes <= 48 * 1024) return cudaSuccess;
+    int own = 0;
+    const cudaError_t e = static_smem(fn, own);
+    if (e != cudaSuccess || own + bytes <= 48 * 1024) return e;
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
