@@ -6,6 +6,7 @@
 // and joined back to it).  No device allocation happens here.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdint>
@@ -123,12 +124,14 @@ cudaError_t static_smem(const void* fn, int& bytes) {
 }
 
 // Opts a kernel in to more shared memory than the default 48 KB, which covers
-// the static and the dynamic part together.
+// the static and the dynamic part together: always to the most there is, so
+// that a host thread cannot lower the limit between another's call here and
+// its launch.
 cudaError_t set_smem(const void* fn, int bytes) {
     int own = 0;
     const cudaError_t e = static_smem(fn, own);
     if (e != cudaSuccess || own + bytes <= 48 * 1024) return e;
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(bytes, kSmemMax - own));
 }
 
 int launch(const void* fn, dim3 grid, dim3 block, int smem, void** args, cudaStream_t s) {
