@@ -413,7 +413,7 @@ def _set_of(t, lens, device, origin=None):
     return TrajSet.from_padded(a, la, device=device, origin=o)
 
 
-def _matrix_into(m, qs, ds, out, cnt, *, eps, gpoint, exact, rows, stream=None):
+def _matrix_into(m, qs, ds, out, cnt, *, eps, gpoint, exact, rows):
     """out (and cnt) [qs.n, ds.n] = measure over Q x D.  Queries up to the
     matrix forms' limit (MATRIX_QUERY_MAX points; Hausdorff: any) in one
     tsm_matrix launch; the rows of longer queries with tsm_pairs over
@@ -421,7 +421,7 @@ def _matrix_into(m, qs, ds, out, cnt, *, eps, gpoint, exact, rows, stream=None):
     up to tsm_max_supported_len.  Both give the same values bit for bit."""
     lq = qs.lens_host if qs.lens_host is not None else qs.lens.cpu().numpy()
     if m == _lib.HAUSDORFF or qs.max_len <= MATRIX_QUERY_MAX:
-        matrix_raw(m, qs, ds, out=out, counts=cnt, eps=eps, gpoint=gpoint, exact=exact, rows=rows, stream=stream)
+        matrix_raw(m, qs, ds, out=out, counts=cnt, eps=eps, gpoint=gpoint, exact=exact, rows=rows)
         return
     dev = qs.device
     long_i = np.nonzero(np.asarray(lq) > MATRIX_QUERY_MAX)[0]
@@ -432,7 +432,7 @@ def _matrix_into(m, qs, ds, out, cnt, *, eps, gpoint, exact, rows, stream=None):
                       np.asarray(lq)[short_i].astype(np.int32), origin=qs.origin)
         o = torch.empty((sub.n, ds.n), dtype=torch.float32, device=dev)
         c = torch.empty((sub.n, ds.n), dtype=torch.int32, device=dev) if cnt is not None else None
-        matrix_raw(m, sub, ds, out=o, counts=c, eps=eps, gpoint=gpoint, exact=exact, rows=rows, stream=stream)
+        matrix_raw(m, sub, ds, out=o, counts=c, eps=eps, gpoint=gpoint, exact=exact, rows=rows)
         out[si] = o
         if cnt is not None:
             cnt[si] = c
@@ -446,8 +446,8 @@ def _matrix_into(m, qs, ds, out, cnt, *, eps, gpoint, exact, rows, stream=None):
         o = torch.empty(nd, dtype=torch.float32, device=dev)
         c = torch.empty(nd, dtype=torch.int32, device=dev) if cnt is not None else None
         pairs_raw(m, pool, off_a, len_a, ds.off, ds.lens, max(qs.max_len, ds.max_len), out=o, counts=c,
-                  order=engine.pair_order_dev(len_a, ds.lens, stream=stream), eps=eps, gpoint=shift_gpoint(gpoint, origin),
-                  exact=exact, rows=rows, stream=stream)
+                  order=engine.pair_order_dev(len_a, ds.lens), eps=eps, gpoint=shift_gpoint(gpoint, origin),
+                  exact=exact, rows=rows)
         out[int(i)] = o
         if cnt is not None:
             cnt[int(i)] = c
@@ -525,32 +525,35 @@ def matrix_many(measures, Q, lenQ, D, lenD, *, eps=0.0, gpoint=None, exact=False
     qs = _set_of(Q, lenQ, dev, origin)
     ds = qs if (D is Q and lenD is lenQ) else _set_of(D, lenD, dev, origin)
     g = _gpoint(gpoint)
-    s = stream if stream is not None else torch.cuda.current_stream(dev)
+    ds.order_by_length()  # (kept by the set: not made on `stream`)
     copy = torch.cuda.Stream(device=dev)
-    with torch.cuda.stream(s):
+    host = {}
+
+    def work():
+        s = torch.cuda.current_stream(dev)
         lq = qs.lens.double()[:, None]
         ld = ds.lens.double()[None, :]
-    host = {}
-    for meas in measures:
-        m = measure_id(meas)
-        out = torch.empty((qs.n, ds.n), dtype=torch.float32, device=dev)
-        cnt = torch.empty((qs.n, ds.n), dtype=torch.int32, device=dev) if m in (_lib.EDR, _lib.LCSS) else None
-        _matrix_into(m, qs, ds, out, cnt, eps=eps, gpoint=g, exact=exact, rows=rows, stream=s)
-        with torch.cuda.stream(s):
+        for meas in measures:
+            m = measure_id(meas)
+            out = torch.empty((qs.n, ds.n), dtype=torch.float32, device=dev)
+            cnt = torch.empty((qs.n, ds.n), dtype=torch.int32, device=dev) if m in (_lib.EDR, _lib.LCSS) else None
+            _matrix_into(m, qs, ds, out, cnt, eps=eps, gpoint=g, exact=exact, rows=rows)
             if m == _lib.EDR:
                 res = cnt.double() / torch.maximum(lq, ld)
             elif m == _lib.LCSS:
                 res = 1.0 - cnt.double() / torch.minimum(lq, ld)
             else:
                 res = out.double()
-        done = torch.cuda.Event()
-        done.record(s)
-        h = torch.empty(res.shape, dtype=torch.float64, pin_memory=True)
-        copy.wait_event(done)
-        with torch.cuda.stream(copy):
-            h.copy_(res, non_blocking=True)
-        res.record_stream(copy)
-        host[_lib.MEASURE_NAMES[m]] = h
+            done = torch.cuda.Event()
+            done.record(s)
+            h = torch.empty(res.shape, dtype=torch.float64, pin_memory=True)
+            copy.wait_event(done)
+            with torch.cuda.stream(copy):
+                h.copy_(res, non_blocking=True)
+            res.record_stream(copy)
+            host[_lib.MEASURE_NAMES[m]] = h
+        return ()
+    engine.on_stream(stream, (qs.pts, qs.off, qs.lens, ds.pts, ds.off, ds.lens, ds.order_by_length()), work)
     copy.synchronize()
     return {k: v.numpy() for k, v in host.items()}
 

@@ -33,6 +33,27 @@ def _stream_ptr(stream):
     return ctypes.c_void_p(s.cuda_stream)
 
 
+def on_stream(stream, used, work):
+    """work(), with every tensor it makes and every kernel it launches on
+    `stream` (None: the current one), after what the current stream holds so
+    far.  used: the caller's tensors that it reads, which stay allocated until
+    `stream` is done with them; its results (a tuple, None among them allowed)
+    may be dropped while the current stream still reads them."""
+    current = torch.cuda.current_stream(stream.device) if stream is not None else None
+    if stream is None or stream == current:
+        return work()
+    stream.wait_stream(current)
+    for t in used:
+        if isinstance(t, torch.Tensor) and t.is_cuda:
+            t.record_stream(stream)
+    with torch.cuda.stream(stream):
+        res = work()
+    for t in res:
+        if t is not None:
+            t.record_stream(current)
+    return res
+
+
 def measure_id(measure) -> int:
     if isinstance(measure, str):
         try:
@@ -345,16 +366,15 @@ def pair_order_dev(len_a: torch.Tensor, len_b: torch.Tensor, rows=DEFAULT_ROWS, 
     """pair_order on the device (tsm_pair_order): an int32 processing order for
     tsm_pairs, by classes of loop shapes (steps of 8 points, whatever rows),
     the largest first."""
-    la, lb = len_a.to(torch.int32).contiguous(), len_b.to(torch.int32).contiguous()
-    n = int(la.shape[0])
-    lib = _lib.load()
-    order = torch.empty(n, dtype=torch.int32, device=la.device)
-    ws = torch.empty(lib.tsm_pair_order_workspace_bytes() // 4, dtype=torch.int32, device=la.device)
-    _lib.check(lib.tsm_pair_order(_ptr(la), _ptr(lb), n, _ptr(order), _ptr(ws), _stream_ptr(stream)), "tsm_pair_order")
-    if stream is not None:  # allocated on the current stream, used on this one
-        for t in (la, lb, ws, order):
-            t.record_stream(stream)
-    return order
+    def work():
+        la, lb = len_a.to(torch.int32).contiguous(), len_b.to(torch.int32).contiguous()
+        n = int(la.shape[0])
+        lib = _lib.load()
+        order = torch.empty(n, dtype=torch.int32, device=la.device)
+        ws = torch.empty(lib.tsm_pair_order_workspace_bytes() // 4, dtype=torch.int32, device=la.device)
+        _lib.check(lib.tsm_pair_order(_ptr(la), _ptr(lb), n, _ptr(order), _ptr(ws), _stream_ptr(None)), "tsm_pair_order")
+        return (order,)
+    return on_stream(stream, (len_a, len_b), work)[0]
 
 
 # Pairs per SM from which a batch without an order is worth sorting by loop
@@ -411,10 +431,7 @@ def matrix(measure, q: TrajSet, d: TrajSet, *, eps=0.0, gpoint=(0.0, 0.0), exact
     return out, counts
 
 
-def pairs_in_set(measure, s: TrajSet, idx_a, idx_b, *, eps=0.0, gpoint=(0.0, 0.0), exact=False, rows=0,
-                 stream=None, order=None, with_counts=None):
-    """Pairs (idx_a[k], idx_b[k]) of one device set -> (out float32 [n], counts)."""
-    m = measure_id(measure)
+def _pairs_in_set(m, s, idx_a, idx_b, order, with_counts, **kw):
     ia = torch.as_tensor(idx_a, device=s.device).long()
     ib = torch.as_tensor(idx_b, device=s.device).long()
     off_a, len_a = s.off[ia], s.lens[ia]
@@ -427,7 +444,15 @@ def pairs_in_set(measure, s: TrajSet, idx_a, idx_b, *, eps=0.0, gpoint=(0.0, 0.0
             n > ORDER_PAIRS_PER_SM * _sm_count(s.device):
         # lanes of a warp that take unequal pairs wait for the longest (EDR and LCSS: 0.29 -> 0.27 ms for 200,000 pairs,
         # less than the sort takes)
-        order = pair_order_dev(len_a, len_b, stream=stream)
-    pairs_raw(m, s.pts, off_a, len_a, off_b, len_b, s.max_len, out=out, counts=counts, order=order,
-              eps=eps, gpoint=shift_gpoint(gpoint, s.origin), exact=exact, rows=rows, stream=stream)
+        order = pair_order_dev(len_a, len_b)
+    pairs_raw(m, s.pts, off_a, len_a, off_b, len_b, s.max_len, out=out, counts=counts, order=order, **kw)
     return out, counts
+
+
+def pairs_in_set(measure, s: TrajSet, idx_a, idx_b, *, eps=0.0, gpoint=(0.0, 0.0), exact=False, rows=0,
+                 stream=None, order=None, with_counts=None):
+    """Pairs (idx_a[k], idx_b[k]) of one device set -> (out float32 [n], counts)."""
+    # (on_stream: an order formed while the lengths still change would not be a permutation)
+    return on_stream(stream, (idx_a, idx_b, order, s.pts, s.off, s.lens), lambda: _pairs_in_set(
+        measure_id(measure), s, idx_a, idx_b, order, with_counts, eps=eps, gpoint=shift_gpoint(gpoint, s.origin),
+        exact=exact, rows=rows))

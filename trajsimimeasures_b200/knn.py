@@ -25,7 +25,7 @@ import torch
 
 from . import _lib
 from .engine import (DEFAULT_ROWS, MATRIX_QUERY_MAX, TrajSet, _ptr, _stream_ptr, matrix_gather_raw, matrix_raw,
-                     measure_id, pair_order_dev, pairs_raw, same_origin, shift_gpoint)
+                     measure_id, on_stream, pair_order_dev, pairs_raw, same_origin, shift_gpoint)
 
 
 def topk_rows(d: torch.Tensor, k: int, stream=None):
@@ -55,6 +55,12 @@ def knn_exhaustive(Q: TrajSet, D: TrajSet, k=10, measure="dtw", *, chunk=1 << 18
     """Exact k nearest database trajectories of every query: (dist float32
     [nq, k], index int64 [nq, k]) ascending, ties to the smaller index."""
     m = measure_id(measure)
+    by_length = D.order_by_length()  # (kept by the set: not made on `stream`)
+    return on_stream(stream, (Q.pts, Q.off, Q.lens, D.pts, D.off, D.lens, by_length), lambda: _knn_exhaustive(
+        Q, D, k, m, chunk, eps, gpoint, exact))
+
+
+def _knn_exhaustive(Q, D, k, m, chunk, eps, gpoint, exact):
     order = D.order_by_length().long()
     best_d, best_i = [], []
     buf = torch.empty((Q.n, min(chunk, D.n)), dtype=torch.float32, device=Q.device)
@@ -62,8 +68,8 @@ def knn_exhaustive(Q: TrajSet, D: TrajSet, k=10, measure="dtw", *, chunk=1 << 18
         ids = order[s:s + chunk]
         sub = _subset(D, ids)
         out = buf[:, :sub.n]
-        matrix_raw(m, Q, sub, out=out, eps=eps, gpoint=gpoint, exact=exact, stream=stream)
-        v, j = topk_rows(out, min(k, sub.n), stream=stream)
+        matrix_raw(m, Q, sub, out=out, eps=eps, gpoint=gpoint, exact=exact)
+        v, j = topk_rows(out, min(k, sub.n))
         best_d.append(v)
         best_i.append(ids[j.long()])
     dcat = torch.cat(best_d, dim=1)
@@ -75,7 +81,7 @@ def knn_exhaustive(Q: TrajSet, D: TrajSet, k=10, measure="dtw", *, chunk=1 << 18
     o = torch.argsort(icat, dim=1)
     dcat = torch.gather(dcat, 1, o).contiguous()
     icat = torch.gather(icat, 1, o)
-    v, j = topk_rows(dcat, k, stream=stream)
+    v, j = topk_rows(dcat, k)
     return v, torch.gather(icat, 1, j.long())
 
 
@@ -84,6 +90,11 @@ def knn_rerank(Q: TrajSet, D: TrajSet, cand: torch.Tensor, k=10, measure="dtw", 
     """Exact top-k among candidate database indices cand [nq, c] (int64):
     (dist [nq, k], index [nq, k])."""
     m = measure_id(measure)
+    return on_stream(stream, (cand, Q.pts, Q.off, Q.lens, D.pts, D.off, D.lens), lambda: _knn_rerank(
+        Q, D, cand, k, m, eps, gpoint, exact, gather_lpt))
+
+
+def _knn_rerank(Q, D, cand, k, m, eps, gpoint, exact, gather_lpt):
     nq, c = cand.shape
     if Q.max_len <= MATRIX_QUERY_MAX:
         # each query's candidates in database-length order: the query is staged
@@ -93,7 +104,7 @@ def knn_rerank(Q: TrajSet, D: TrajSet, cand: torch.Tensor, k=10, measure="dtw", 
         dd = torch.empty((nq, c), dtype=torch.float32, device=Q.device)
         # longest queries first: their CTAs run longest, so the launch ends with short ones
         qo = torch.argsort(Q.lens, descending=True, stable=True).to(torch.int32) if gather_lpt else None
-        matrix_gather_raw(m, Q, D, cs, out=dd, eps=eps, gpoint=gpoint, exact=exact, stream=stream, q_order=qo)
+        matrix_gather_raw(m, Q, D, cs, out=dd, eps=eps, gpoint=gpoint, exact=exact, q_order=qo)
         cand = cs.long()
     else:  # queries too long for the matrix form: the paired kernel, in loop-shape order
         shift = D.pts.shape[0]
@@ -104,14 +115,14 @@ def knn_rerank(Q: TrajSet, D: TrajSet, cand: torch.Tensor, k=10, measure="dtw", 
         off_b, len_b = D.off[di], D.lens[di]
         dd = torch.empty(nq * c, dtype=torch.float32, device=Q.device)
         pairs_raw(m, pool, off_a, len_a, off_b, len_b, max(Q.max_len, D.max_len), out=dd, eps=eps,
-                  gpoint=shift_gpoint(gpoint, same_origin(Q, D)), exact=exact, stream=stream,
-                  order=shape_order(len_a, len_b, stream=stream))
+                  gpoint=shift_gpoint(gpoint, same_origin(Q, D)), exact=exact,
+                  order=shape_order(len_a, len_b))
         dd = dd.view(nq, c)
     # ties to the smaller database index, as in knn_exhaustive
     o = torch.argsort(cand, dim=1)
     dd = torch.gather(dd, 1, o).contiguous()
     ci = torch.gather(cand, 1, o)
-    v, j = topk_rows(dd, k, stream=stream)
+    v, j = topk_rows(dd, k)
     return v, torch.gather(ci, 1, j.long())
 
 
