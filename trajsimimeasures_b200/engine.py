@@ -365,7 +365,10 @@ MATRIX_QUERY_MAX = 1400  # longest query of the matrix forms (tsm_matrix_query_m
 def pair_order_dev(len_a: torch.Tensor, len_b: torch.Tensor, rows=DEFAULT_ROWS, stream=None) -> torch.Tensor:
     """pair_order on the device (tsm_pair_order): an int32 processing order for
     tsm_pairs, by classes of loop shapes (steps of 8 points, whatever rows),
-    the largest first."""
+    the largest first.  Lengths on the CPU: pair_order's order for `rows`."""
+    if not len_a.is_cuda:
+        return torch.from_numpy(pair_order(len_a.numpy(), len_b.numpy(), rows))
+
     def work():
         la, lb = len_a.to(torch.int32).contiguous(), len_b.to(torch.int32).contiguous()
         n = int(la.shape[0])
