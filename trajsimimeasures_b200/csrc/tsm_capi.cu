@@ -61,14 +61,19 @@ constexpr int kMaxLen = 32768;
 // non-empty pair runs one warp each on the wave kernels instead, with 4 rows
 // per lane unless rows_per_thread says otherwise.
 constexpr int kSmallBatchPerSm = 64;
-// Longest side of a pair in the two launches of the pruned Hausdorff pairs
-// kernel: 23 KB of shared memory per warp (eight warps per SM) and 181 KB (one).
-constexpr int kHausPrunedShort = 512;
+// Longest trajectory that the pruned Hausdorff kernels give to one warp (47 KB
+// of shared memory for a matrix CTA's eight, 93 KB for eight pairs); a longer one
+// is a CTA's.
+constexpr int kHausWarpLen = 256;
+// Longest side of a pair in the two launches of the pruned pairs kernel with a
+// CTA per pair: four and one of 8 warps fit an SM.
+constexpr int kHausPrunedMid = 1024;
 constexpr int kHausPrunedMax = 4096;
 static_assert(8 * tsm::haus_floats(kHausPrunedMax) <= 227 * 1024, "one staged pair fits a CTA");
-// Matrix launches of at most kHausThreadLen points on both sides and at least
-// kHausThreadPairs pairs (512 threads per SM) run one thread per pair.
-constexpr int kHausThreadLen = 64;
+// Matrix launches of at most kHausThreadLen points on both sides and, the
+// shorter these are, the fewer pairs (512 threads per SM at kHausThreadLen) run
+// one thread per pair; up to kHausThreadAlways points all do.
+constexpr int kHausThreadLen = 64, kHausThreadAlways = 12;
 constexpr int64_t kHausThreadPairs = 148 * 512;
 // Shared memory one CTA may use, leaving room for two CTAs per SM at cap 200.
 constexpr int kSmemPerCta = 113 * 1024;
@@ -273,37 +278,36 @@ int tsm_pairs(int measure, const float* pts, const int64_t* off_a, const int32_t
         int64_t warp_cells = small ? 0 : tsm::kHausWarpCells;
         void* args[] = {&p2, &off_a, &len_a, &off_b, &len_b, &order, &n, &ml, &warp_cells, &out};
         if ((int64_t)max_len * max_len <= warp_cells) return launch(fn, grid, dim3(threads), 0, args, s);
-        // longer pairs (small batch: every non-empty pair), one warp each: pruned up to kHausPrunedShort points
-        // with many warps per SM, pruned up to kHausPrunedMax with the few that then fit, unpruned above
-        const void* pfn = tsm_k::haus_pruned_pairs(exact);
-        int lo[2] = {0, kHausPrunedShort};
-        int cap[2] = {max_len < kHausPrunedShort ? max_len : kHausPrunedShort,
-                      max_len < kHausPrunedMax ? max_len : kHausPrunedMax};
+        // longer pairs (small batch: every non-empty pair): pruned, one warp each up to kHausWarpLen points, one CTA
+        // each up to kHausPrunedMax, unpruned above
+        const int top[3] = {kHausWarpLen, kHausPrunedMid, kHausPrunedMax};
+        int lo[3] = {0, kHausWarpLen, kHausPrunedMid}, cap[3];
+        for (int c = 0; c < 3; ++c) cap[c] = max_len < top[c] ? max_len : top[c];
         auto pruned = [&](int c, cudaStream_t st) {
-            const int pair_bytes = 8 * tsm::haus_floats(cap[c]);
-            int pw = 8;
-            while (pw > 1 && pw * pair_bytes > kSmemPerCta) pw >>= 1;
+            const void* pfn = tsm_k::haus_pruned_pairs(c > 0, exact);
+            const int pw = c > 0 ? 1 : 8, smem = pw * 8 * tsm::haus_floats(cap[c]);
             dim3 p_grid;
-            const int r = persistent_grid("tsm_pairs", pfn, 32 * pw, pw * pair_bytes, (n + pw - 1) / pw, p_grid, dev);
+            const int r = persistent_grid("tsm_pairs", pfn, 256, smem, (n + pw - 1) / pw, p_grid, dev);
             if (r != TSM_OK) return r;
             void* p_args[] = {&p2, &off_a, &len_a, &off_b, &len_b, &order, &n, &lo[c], &cap[c], &warp_cells, &out};
-            return launch(pfn, p_grid, dim3(32 * pw), pw * pair_bytes, p_args, st);
+            return launch(pfn, p_grid, dim3(256), smem, p_args, st);
         };
         auto main_side = [&](cudaStream_t st) {
             const int r = launch(fn, grid, dim3(threads), 0, args, st);
             return r != TSM_OK ? r : pruned(0, st);
         };
         auto long_side = [&](cudaStream_t st) {
-            const int r = pruned(1, st);
+            int r = max_len > kHausPrunedMid ? pruned(2, st) : TSM_OK;
+            if (r == TSM_OK) r = pruned(1, st);
             if (r != TSM_OK || max_len <= kHausPrunedMax) return r;
             const void* wfn = tsm_k::haus_wave(R, exact);
             dim3 w_grid;
             const int r2 = persistent_grid("tsm_pairs", wfn, threads, 0, (n + 3) / 4, w_grid, dev);
             if (r2 != TSM_OK) return r2;
-            void* w_args[] = {&p2, &off_a, &len_a, &off_b, &len_b, &order, &n, &ml, &cap[1], &warp_cells, &out};
+            void* w_args[] = {&p2, &off_a, &len_a, &off_b, &len_b, &order, &n, &ml, &cap[2], &warp_cells, &out};
             return launch(wfn, w_grid, dim3(threads), 0, w_args, st);
         };
-        if (max_len <= kHausPrunedShort) return main_side(s);
+        if (max_len <= kHausWarpLen) return main_side(s);
         // the long pairs on the side stream, overlapping the shorter ones
         return launch_with_side(main_side, long_side, s, dev);
     }
@@ -364,29 +368,48 @@ int matrix_launch(const char* who, int measure, const float* q_pts, const int64_
     if (measure == TSM_HAUSDORFF) {
         const void* fn = tsm_k::haus(true, R, exact);
         if (!fn) return fail(TSM_EINVAL, "%s: rows_per_thread must be 4, 8 or 16", who);
-        // One warp per pair with pruning, as many warps per CTA as fit (two CTAs per SM while they do), unless the
-        // trajectories are short and there are threads enough for a pair each.  Measured, 2000 x 2000 random walks,
-        // pruned / one thread per pair, ms: lengths 2..32 3.4 / 1.4, 2..64 4.7 / 4.2, 20..64 5.3 / 6.3, 2..96 5.7 /
-        // 8.7, 20..200 9.1 / 39.9; 1 x 2000 pairs of 20..200: 0.04 / 0.96.  (Points without any spatial order,
-        // where no box helps: 1000 x 1000 of 20..200 uniform random points 12.7 / 11.1.)
-        int dcap = d_max_len < 1 ? 1 : d_max_len;
-        const int64_t q_bytes = 4 * (int64_t)tsm::haus_floats(qcap), d_bytes = 4 * (int64_t)tsm::haus_floats(dcap);
-        int qb = sym == 2 ? 1 : 4, hw = 8;
-        while (hw > qb && qb * q_bytes + hw * d_bytes > kSmemPerCta) hw >>= 1;
-        if (qb * q_bytes + hw * d_bytes > kSmemPerCta) qb = 1;
-        while (hw > 1 && qb * q_bytes + hw * d_bytes > kSmemPerCta) hw >>= 1;
-        const bool by_thread = qcap <= kHausThreadLen && dcap <= kHausThreadLen && nq * nd >= kHausThreadPairs;
-        if (!by_thread && qb * q_bytes + hw * d_bytes <= kSmemPerCta) {
+        // One warp per pair with pruning (a CTA per pair with a long trajectory), unless the trajectories are short and
+        // there are threads enough for a pair each.  Measured, random walks, pruned / one thread per pair: 2000 x 2000
+        // of 2..32 points 3.4 / 1.4 ms, 2..64 4.7 / 4.2, 20..64 5.3 / 6.3, 2..96 5.7 / 8.7, 20..200 9.1 / 39.9; 100 x
+        // 100 of 2..32 points 38 / 50 us, 200 x 200 68 / 66, 270 x 270 97 / 86; 2..8 points 33 / 24, 56 / 27, 81 / 32.
+        // (Points without any spatial order, where no box helps: 1000 x 1000 of 20..200 13.0 / 11.5 ms, 500 x 1000 6.6
+        // / 6.1, 200 x 200 of 300..500 5.8 / 11.3.)
+        // Eight warps a CTA; four queries share a staged trajectory unless that leaves fewer than three CTAs on an SM
+        // and one query would leave more.  Where a CTA's warps would not fit twice on an SM, the long kernel: 1,000
+        // walks of 20..200 points and one of 2,500, all pairs, 4.5 ms, 26.9 with every warp's memory sized for that
+        // one (2 warps per SM), 194 unpruned; without any order 20.7, 132, 194.  300..500 points, 200 x 200: 0.68 ms
+        // by warps, 1.00 by CTAs.
+        const int hw = 8;
+        int dcap = d_max_len < 1 ? 1 : d_max_len, wcap = dcap;
+        const int64_t q_bytes = 4 * (int64_t)tsm::haus_floats(qcap);
+        int64_t d_bytes = hw * 4 * (int64_t)tsm::haus_floats(dcap);
+        auto queries = [&]() {
+            const int64_t four = kSmemMax / (4 * q_bytes + d_bytes + 1024), one = kSmemMax / (q_bytes + d_bytes + 1024);
+            return sym != 2 && four > 0 && four >= std::min(one, (int64_t)3) ? 4 : 1;
+        };
+        const bool longs = q_bytes + d_bytes > kSmemPerCta;
+        if (longs) {
+            wcap = dcap < kHausWarpLen ? dcap : kHausWarpLen;
+            d_bytes = 4 * std::max((int64_t)tsm::haus_floats(dcap), hw * (int64_t)tsm::haus_floats(wcap));
+        }
+        const int qb = queries();
+        const int64_t longer = std::max(qcap, dcap);
+        const bool by_thread = longer <= kHausThreadAlways ||
+                               (longer <= kHausThreadLen &&
+                                nq * nd * kHausThreadLen * kHausThreadLen >= kHausThreadPairs * longer * longer);
+        if (!by_thread && qb * q_bytes + d_bytes <= kSmemMax - 1024) {
             const int64_t qt = (nq + qb - 1) / qb;
             int per_cta = 64;  // database slots per CTA: fewer when that leaves SMs without a few CTAs each
             while (per_cta > hw && (nd + per_cta - 1) / per_cta * qt < 148 * 16) per_cta >>= 1;
             const int64_t chunks64 = (nd + per_cta - 1) / per_cta;
             if (chunks64 * qt > 0x7fffffffLL) return fail(TSM_EINVAL, "%s: grid too large", who);
             int chunks = (int)chunks64;
-            void* args[] = {&q2,   &q_off, &q_len,  &q_order, &nq,  &d2,   &d_off, &d_len, &d_order,
-                            &ndd,  &dtot,  &chunks, &per_cta, &sym, &qcap, &dcap,  &out,   &ld};
-            return launch(tsm_k::haus_pruned_matrix(qb, exact), dim3((unsigned)(chunks * qt)), dim3(32 * hw),
-                          (int)(qb * q_bytes + hw * d_bytes), args, s);
+            void* args[] = {&q2,   &q_off,  &q_len,   &q_order, &nq,   &d2,   &d_off, &d_len, &d_order, &ndd,
+                            &dtot, &chunks, &per_cta, &sym,     &qcap, &dcap, &out,   &ld};
+            void* l_args[] = {&q2,   &q_off,  &q_len,   &q_order, &nq,   &d2,   &d_off, &d_len, &d_order, &ndd,
+                              &dtot, &chunks, &per_cta, &sym,     &qcap, &wcap, &dcap,  &out,   &ld};
+            return launch(tsm_k::haus_pruned_matrix(qb, longs, exact), dim3((unsigned)(chunks * qt)), dim3(32 * hw),
+                          (int)(qb * q_bytes + d_bytes), longs ? l_args : args, s);
         }
         const int smem = ((qcap + 1) / 2) * 40;  // staged segment pairs
         if (smem > kSmemMax) return fail(TSM_ETOOLONG, "%s: query length %d too long", who, q_max_len);

@@ -34,8 +34,18 @@
 // points 55.3 -> 5.8 ms; 200,000 pairs of 20..200 points 6.7 -> 1.1 ms, 50,000
 // lognormal pairs (10..2000 points) 8.8 -> 0.64 ms.  64 registers (32 warps
 // per SM); 48 (40 warps) spill: 10.9 ms for the first case.  Finishing a group
-// with one lane per segment once few of its points count was slower (12.0).
+// with one lane per segment once few of its points count was slower (12.0), and
+// so was leaving out a group's tests after three that skipped nothing (2.46 ->
+// 2.87 ms for 1000 x 1000, and 13.1 -> 17.4 on points without any order).
+//
+// A pair with a long trajectory (22 bytes of shared memory a point) is a CTA's,
+// so that 8 to 24 warps work on an SM whatever the lengths; its warps take the
+// groups side by side and share the maximum, which skips a little less than one
+// warp after the other (1.00 ms for 200 x 200 of 300..500 points by CTAs, 0.68 by
+// warps, which still fit 16 times there).
 #pragma once
+
+#include <type_traits>
 
 #include "tsm_tile.cuh"
 
@@ -83,14 +93,31 @@ __device__ __forceinline__ float warp_min(float v) {
     return v;
 }
 
-// Stages n points by one warp (all lanes); the boxes include both end points
+// Who works on a pair: one warp (TEAM false) or all warps of the CTA.
+template <bool TEAM>
+struct HausGang {
+    static __device__ __forceinline__ int rank() { return TEAM ? threadIdx.x : threadIdx.x & 31; }
+    static __device__ __forceinline__ int size() { return TEAM ? blockDim.x : 32; }
+    static __device__ __forceinline__ void sync() {
+        if constexpr (TEAM) __syncthreads();
+        else __syncwarp();
+    }
+    static __device__ __forceinline__ bool all(bool v) {
+        if constexpr (TEAM) return __syncthreads_and(v);
+        else return __all_sync(0xffffffffu, v);
+    }
+};
+
+// Stages n points (all threads of the gang); the boxes include both end points
 // of every segment of their block.
-template <bool EXACT>
-__device__ __forceinline__ void haus_stage(HausTraj& t, const float2* __restrict__ p, int n, int lane) {
+template <bool EXACT, bool TEAM>
+__device__ __forceinline__ void haus_stage(HausTraj& t, const float2* __restrict__ p, int n) {
+    using G = HausGang<TEAM>;
+    const int rank = G::rank(), size = G::size(), lane = threadIdx.x & 31;
     t.n = n;
     bool fin = true;
     const int npair = (n + 1) >> 1;
-    for (int j = lane; j < npair; j += 32) {
+    for (int j = rank; j < npair; j += size) {
         const int k0 = 2 * j, k1 = min(k0 + 1, n - 1), k2 = min(k0 + 2, n - 1);
         const float2 v0 = __ldg(p + k0), v1 = __ldg(p + k1), v2 = __ldg(p + k2);
         SegPair g;
@@ -101,9 +128,15 @@ __device__ __forceinline__ void haus_stage(HausTraj& t, const float2* __restrict
         t.C[j] = g.ninv;
         fin = fin && isfinite(v0.x) && isfinite(v0.y) && isfinite(v1.x) && isfinite(v1.y);
     }
-    __syncwarp();
+    G::sync();
     float4 u = make_float4(CUDART_INF_F, -CUDART_INF_F, CUDART_INF_F, -CUDART_INF_F);
-    for (int b = lane; b < (n + kHausBlk - 1) / kHausBlk; b += 32) {
+    auto widen = [&](const float4& v) {
+        u.x = fminf(u.x, v.x);
+        u.y = fmaxf(u.y, v.y);
+        u.z = fminf(u.z, v.z);
+        u.w = fmaxf(u.w, v.w);
+    };
+    for (int b = rank; b < (n + kHausBlk - 1) / kHausBlk; b += size) {
         float4 v = make_float4(CUDART_INF_F, -CUDART_INF_F, CUDART_INF_F, -CUDART_INF_F);
 #pragma unroll
         for (int k = 0; k <= kHausBlk; k += 2) {  // vertices 8 b .. 8 b + 8, two per pair
@@ -117,13 +150,10 @@ __device__ __forceinline__ void haus_stage(HausTraj& t, const float2* __restrict
             v.w = max3f(v.w, -a.z, two ? -a.w : -a.z);
         }
         t.box[b] = v;
-        u.x = fminf(u.x, v.x);
-        u.y = fmaxf(u.y, v.y);
-        u.z = fminf(u.z, v.z);
-        u.w = fmaxf(u.w, v.w);
+        if (!TEAM) widen(v);
     }
-    __syncwarp();
-    for (int g = lane; g < (n + 31) >> 5; g += 32) {
+    G::sync();
+    for (int g = rank; g < (n + 31) >> 5; g += size) {
         float4 v = t.box[kHausGrp * g];
         for (int i = 1; i < kHausGrp; ++i) {
             const float4 w = t.box[min(kHausGrp * g + i, haus_blocks(n) - 1)];
@@ -131,12 +161,16 @@ __device__ __forceinline__ void haus_stage(HausTraj& t, const float2* __restrict
         }
         t.grp[g] = v;
     }
+    if constexpr (TEAM) {  // every warp makes the whole box
+        G::sync();
+        for (int g = lane; g < (n + 31) >> 5; g += 32) widen(t.grp[g]);
+    }
     u.x = warp_min(u.x);
     u.y = -warp_min(-u.y);
     u.z = warp_min(u.z);
     u.w = -warp_min(-u.w);
-    t.bb = __all_sync(0xffffffffu, fin) ? u : make_float4(-CUDART_INF_F, CUDART_INF_F, -CUDART_INF_F, CUDART_INF_F);
-    __syncwarp();
+    t.bb = G::all(fin) ? u : make_float4(-CUDART_INF_F, CUDART_INF_F, -CUDART_INF_F, CUDART_INF_F);
+    if (!TEAM) G::sync();
 }
 
 // Squared smallest and largest distance of two boxes (a point: lo = hi).
@@ -155,17 +189,23 @@ __device__ __forceinline__ float widen2(float d2, float delta) {
 }
 
 // max(m, max over the points of P of the min over the segments of T), by one
-// warp; m and the result are uniform.
-__device__ __forceinline__ float haus_directed(const HausTraj& P, const HausTraj& T, float m, float delta, int lane) {
+// warp (m and the result uniform), or the groups of P shared out to the warps of
+// a CTA (TEAM): a warp's result is then the largest that it or, as far as it has
+// seen, another one found, and *shared (a float's bits, not below m) the largest
+// of all once every warp is through.
+template <bool TEAM>
+__device__ __forceinline__ float haus_directed(const HausTraj& P, const HausTraj& T, float m, float delta, int lane,
+                                               int* shared) {
     constexpr unsigned kFull = 0xffffffffu;
     if (T.n < 2 || P.n <= 0) return m;
+    const int w0 = TEAM ? threadIdx.x >> 5 : 0, nw = TEAM ? blockDim.x >> 5 : 1;
     const int ngrp = (P.n + 31) >> 5, nblk = (T.n + kHausBlk - 1) / kHausBlk, npair = (T.n + 1) >> 1;
     for (int g0 = 0; g0 < ngrp; g0 += 32) {
         // lane l keeps the bound of group g0 + l (0: done; a bound is not, see delta) and the block it came from
         const int ng = min(32, ngrp - g0);
         uint32_t ub = 0;
         int ubb = 0;
-        for (int g = 0; g < ng; ++g) {
+        for (int g = w0; g < ng; g += nw) {
             const float4 gb = P.grp[g0 + g];
             float far = CUDART_INF_F;
             int fb = 0;
@@ -187,6 +227,10 @@ __device__ __forceinline__ float haus_directed(const HausTraj& P, const HausTraj
         for (;;) {
             // the remaining group with the largest bound (bounds are not negative: ordered like their bits)
             const uint32_t top = __reduce_max_sync(kFull, ub);
+            if constexpr (TEAM) {
+                const int seen = lane == 0 ? *reinterpret_cast<volatile int*>(shared) : 0;
+                m = fmaxf(m, __int_as_float(__shfl_sync(kFull, seen, 0)));
+            }
             if (__uint_as_float(top) <= m || top == 0) break;
             const int g = __ffs(__ballot_sync(kFull, ub == top)) - 1;
             const int first = __shfl_sync(kFull, ubb, g);
@@ -216,18 +260,23 @@ __device__ __forceinline__ float haus_directed(const HausTraj& P, const HausTraj
                     thr = (valid && best > m) ? widen2(best, delta) : -1.f;
                 }
             }
-            m = fmaxf(m, __uint_as_float(__reduce_max_sync(kFull, valid ? __float_as_uint(best) : 0u)));
+            const uint32_t top_min = __reduce_max_sync(kFull, valid ? __float_as_uint(best) : 0u);
+            if (TEAM && lane == 0 && __uint_as_float(top_min) > m) atomicMax(shared, (int)top_min);
+            m = fmaxf(m, __uint_as_float(top_min));
         }
     }
     return m;
 }
 
-// The Hausdorff distance of two staged trajectories.
-__device__ __forceinline__ float haus_pair(const HausTraj& a, const HausTraj& b, int lane) {
+// The squared Hausdorff distance of two staged trajectories.  TEAM: of the CTA's
+// pair, *shared 0 before; each warp's part of it, all in *shared once every warp
+// is through.
+template <bool TEAM>
+__device__ __forceinline__ float haus_pair(const HausTraj& a, const HausTraj& b, int lane, int* shared) {
     const float w = fmaxf(a.bb.y, b.bb.y) - fminf(a.bb.x, b.bb.x), h = fmaxf(a.bb.w, b.bb.w) - fminf(a.bb.z, b.bb.z);
     const float delta = fmaf(0x1p-19f, w + h, 0x1p-62f);
-    const float m = haus_directed(a, b, 0.f, delta, lane);
-    return __fsqrt_rn(haus_directed(b, a, m, delta, lane));
+    const float m = haus_directed<TEAM>(a, b, 0.f, delta, lane, shared);
+    return haus_directed<TEAM>(b, a, m, delta, lane, shared);
 }
 
 // Matrix kernel: CTA (t, chunk) stages the queries q_order[QB t ..] (QB of
@@ -261,7 +310,7 @@ __global__ void __launch_bounds__(256) hausdorff_pruned_matrix_kernel(
         if (n > q_cap) n = -1;
         if (n >= 0) {
             HausTraj q(smem + warp * haus_floats(q_cap), q_cap);
-            haus_stage<EXACT>(q, q_pts + q_off[qi], n, lane);
+            haus_stage<EXACT, false>(q, q_pts + q_off[qi], n);
             if (lane == 0) q_bb[warp] = q.bb;
         }
         if (lane == 0) {
@@ -277,7 +326,7 @@ __global__ void __launch_bounds__(256) hausdorff_pruned_matrix_kernel(
         const bool dbad = dj < 0 || dj >= d_total;
         int n = dbad ? -1 : d_len[dj];
         if (n > d_cap) n = -1;
-        if (n >= 0) haus_stage<EXACT>(d, d_pts + d_off[dj], n, lane);
+        if (n >= 0) haus_stage<EXACT, false>(d, d_pts + d_off[dj], n);
         for (int i = 0; i < QB; ++i) {
             if (qs0 + i >= nq || (sym == 1 && slot < qs0 + i)) break;
             float v = CUDART_NAN_F;
@@ -285,7 +334,7 @@ __global__ void __launch_bounds__(256) hausdorff_pruned_matrix_kernel(
                 HausTraj q(smem + i * haus_floats(q_cap), q_cap);
                 q.n = q_n[i];
                 q.bb = q_bb[i];
-                v = haus_pair(q, d, lane);
+                v = __fsqrt_rn(haus_pair<false>(q, d, lane, nullptr));
             }
             const int64_t qi = q_id[i];
             if (lane == 0) {
@@ -297,22 +346,133 @@ __global__ void __launch_bounds__(256) hausdorff_pruned_matrix_kernel(
     }
 }
 
+// The same for a database with long trajectories.  A slot of at most w_cap points
+// is one warp's as above; a longer one is the CTA's, staged over the warps' memory,
+// with the groups of its pairs shared out to the warps: one long trajectory does
+// not leave room for a few warps only.  (Short databases keep the kernel above:
+// in this one the CTA's part takes registers from the warps', 2000 x 2000 of
+// 20..200 points 5 % slower.)  Dynamic shared memory = QB * haus_floats(q cap) +
+// max(W * haus_floats(w cap), haus_floats(d cap)) floats, W >= QB, per_cta <= 64.
+template <int QB, bool EXACT>
+__global__ void __launch_bounds__(256, 3) hausdorff_long_matrix_kernel(
+    const float2* __restrict__ q_pts, const int64_t* __restrict__ q_off, const int32_t* __restrict__ q_len,
+    const int32_t* __restrict__ q_order, int64_t nq, const float2* __restrict__ d_pts,
+    const int64_t* __restrict__ d_off, const int32_t* __restrict__ d_len, const int32_t* __restrict__ d_order,
+    int64_t nd, int64_t d_total, int chunks, int per_cta, int sym, int q_cap, int w_cap, int d_cap,
+    float* __restrict__ out, int64_t ld) {
+    extern __shared__ float4 smem4[];
+    float* smem = reinterpret_cast<float*>(smem4);
+    __shared__ float4 q_bb[QB];
+    __shared__ int q_n[QB];  // -1: outside the set or a bad length
+    __shared__ int64_t q_id[QB];
+    __shared__ unsigned longs[2];  // bit s: slot s0 + s of the chunk is longer than w_cap
+    __shared__ int found[QB];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+    const int64_t qs0 = (int64_t)(blockIdx.x / chunks) * QB;
+    const int64_t s0 = (int64_t)(blockIdx.x % chunks) * per_cta;
+    const int64_t s1 = min(nd, s0 + per_cta);
+    if (sym == 1 && s1 <= qs0) return;
+    if (threadIdx.x < 2) longs[threadIdx.x] = 0;
+    auto stage_query = [&](int i, auto team) {
+        const int64_t qs = qs0 + i;
+        const int64_t qi = qs < nq ? (q_order ? (int64_t)q_order[qs] : qs) : 0;
+        int n = qs < nq ? q_len[qi] : -1;
+        if (n > q_cap) n = -1;
+        if (n >= 0) {
+            HausTraj q(smem + i * haus_floats(q_cap), q_cap);
+            haus_stage<EXACT, decltype(team)::value>(q, q_pts + q_off[qi], n);
+            if (lane == 0) q_bb[i] = q.bb;  // (TEAM: the same from every warp)
+        }
+        if (lane == 0) {
+            q_n[i] = n;
+            q_id[i] = qi;
+        }
+    };
+    if constexpr (QB == 1) stage_query(0, std::true_type{});  // (all warps on the one)
+    else if (warp < QB) stage_query(warp, std::false_type{});
+    __syncthreads();
+    float* area = smem + QB * haus_floats(q_cap);
+    // a slot's database index and length (-1: outside the set or a bad length)
+    auto slot_of = [&](int64_t slot, int64_t& dj) {
+        dj = d_order ? (int64_t)d_order[(sym == 2 ? q_id[0] * nd : 0) + slot] : slot;
+        const int n = dj < 0 || dj >= d_total ? -1 : d_len[dj];
+        return n > d_cap ? -1 : n;
+    };
+    // the pairs of a slot, staged as d (n >= 0)
+    auto pairs_of = [&](const HausTraj& d, int n, int64_t slot, int64_t dj, auto team) {
+        constexpr bool TEAM = decltype(team)::value;
+        for (int i = 0; i < QB; ++i) {
+            if (qs0 + i >= nq || (sym == 1 && slot < qs0 + i)) break;
+            float v = CUDART_NAN_F;
+            if (n >= 0 && q_n[i] >= 0) {
+                HausTraj q(smem + i * haus_floats(q_cap), q_cap);
+                q.n = q_n[i];
+                q.bb = q_bb[i];
+                v = haus_pair<TEAM>(q, d, lane, found + i);
+            }
+            if (TEAM) continue;
+            const int64_t qi = q_id[i];
+            if (lane == 0) {
+                v = __fsqrt_rn(v);
+                out[qi * ld + (sym == 2 ? slot : dj)] = v;
+                if (sym == 1 && dj != qi) out[dj * ld + qi] = v;
+            }
+        }
+    };
+    HausTraj d(area + warp * haus_floats(w_cap), w_cap);
+    for (int64_t slot = s0 + warp; slot < s1; slot += nwarp) {
+        if (sym == 1 && slot < qs0) continue;
+        int64_t dj;
+        const int n = slot_of(slot, dj);
+        if (n > w_cap) {
+            if (lane == 0) atomicOr(&longs[(slot - s0) >> 5], 1u << ((slot - s0) & 31));
+            continue;
+        }
+        if (n >= 0) haus_stage<EXACT, false>(d, d_pts + d_off[dj], n);
+        pairs_of(d, n, slot, dj, std::false_type{});
+        __syncwarp();  // the staged trajectory is free
+    }
+    __syncthreads();
+    HausTraj t(area, d_cap);
+    for (int h = 0; h < 2; ++h)
+        for (unsigned todo = longs[h]; todo; todo &= todo - 1) {
+            const int64_t slot = s0 + 32 * h + __ffs(todo) - 1;
+            int64_t dj;
+            const int n = slot_of(slot, dj);
+            if (threadIdx.x < QB) found[threadIdx.x] = 0;
+            haus_stage<EXACT, true>(t, d_pts + d_off[dj], n);
+            pairs_of(t, n, slot, dj, std::true_type{});
+            __syncthreads();  // every warp is through
+            if (threadIdx.x < QB) {
+                const int i = threadIdx.x;
+                if (qs0 + i < nq && !(sym == 1 && slot < qs0 + i)) {
+                    const float v = q_n[i] < 0 ? CUDART_NAN_F : __fsqrt_rn(__int_as_float(found[i]));
+                    const int64_t qi = q_id[i];
+                    out[qi * ld + (sym == 2 ? slot : dj)] = v;
+                    if (sym == 1 && dj != qi) out[dj * ld + qi] = v;
+                }
+            }
+        }
+}
+
 // Pairs kernel: the pairs of more than warp_cells point products whose longer
-// side is above min_side and at most cap points, one warp each (the others are
-// another launch's, hausdorff_pairs_kernel's or hausdorff_wave_kernel's).
-// Persistent, with the pair assignment of dp_wave_kernel.  Dynamic shared
-// memory = W * 2 * haus_floats(cap) floats.
-template <bool EXACT>
+// side is above min_side and at most cap points (the others are another launch's,
+// hausdorff_pairs_kernel's or hausdorff_wave_kernel's), one warp each or (TEAM)
+// one CTA each.  Persistent, with the pair assignment of dp_wave_kernel.  Dynamic
+// shared memory = 2 * haus_floats(cap) floats for each pair in work.
+template <bool TEAM, bool EXACT>
 __global__ void __launch_bounds__(256) hausdorff_pruned_pairs_kernel(
     const float2* __restrict__ pts, const int64_t* __restrict__ off_a, const int32_t* __restrict__ len_a,
     const int64_t* __restrict__ off_b, const int32_t* __restrict__ len_b, const int32_t* __restrict__ order,
     int64_t n, int min_side, int cap, int64_t warp_cells, float* __restrict__ out) {
     extern __shared__ float4 smem4[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ int found;
+    const int lane = threadIdx.x & 31, warp = TEAM ? 0 : threadIdx.x >> 5;
     float* smem = reinterpret_cast<float*>(smem4) + warp * 2 * haus_floats(cap);
     HausTraj a(smem, cap), b(smem + haus_floats(cap), cap);
-    const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
-    const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+    const int per = TEAM ? 1 : blockDim.x >> 5;
+    const int64_t gw = (int64_t)blockIdx.x * per + warp;
+    const int64_t nw = (int64_t)gridDim.x * per;
     for (int64_t i0 = 0; i0 * nw < n; i0 += 32) {
         const int64_t i = i0 + lane;
         const int64_t t = i * nw + ((i & 1) ? nw - 1 - gw : gw);
@@ -324,16 +484,22 @@ __global__ void __launch_bounds__(256) hausdorff_pruned_pairs_kernel(
             mine = na >= 0 && nb >= 0 && na <= cap && nb <= cap && max(na, nb) > min_side &&
                    (int64_t)na * nb > warp_cells;
         }
-        unsigned todo = __ballot_sync(0xffffffffu, mine);
+        unsigned todo = __ballot_sync(0xffffffffu, mine);  // (TEAM: the same in every warp)
         while (todo) {
             const int src = __ffs(todo) - 1;
             todo &= todo - 1;
             const int64_t kk = __shfl_sync(0xffffffffu, k, src);
-            haus_stage<EXACT>(a, pts + off_a[kk], len_a[kk], lane);
-            haus_stage<EXACT>(b, pts + off_b[kk], len_b[kk], lane);
-            const float v = haus_pair(a, b, lane);
-            if (lane == 0) out[kk] = v;
-            __syncwarp();
+            if (TEAM && threadIdx.x == 0) found = 0;
+            haus_stage<EXACT, TEAM>(a, pts + off_a[kk], len_a[kk]);
+            haus_stage<EXACT, TEAM>(b, pts + off_b[kk], len_b[kk]);
+            const float v = haus_pair<TEAM>(a, b, lane, &found);
+            HausGang<TEAM>::sync();
+            if (TEAM) {
+                if (threadIdx.x == 0) out[kk] = __fsqrt_rn(__int_as_float(found));
+                __syncthreads();  // (read before the next pair clears it)
+            } else if (lane == 0) {
+                out[kk] = __fsqrt_rn(v);
+            }
         }
     }
 }

@@ -31,21 +31,25 @@ const void* haus(bool matrix, int R, bool exact) {
 
 const void* haus_wave(int R, bool exact) { return exact ? haus_wave_of<true>(R) : haus_wave_of<false>(R); }
 
-const void* haus_pruned_pairs(bool exact) {
-    return exact ? (const void*)&tsm::hausdorff_pruned_pairs_kernel<true>
-                 : (const void*)&tsm::hausdorff_pruned_pairs_kernel<false>;
+const void* haus_pruned_pairs(bool team, bool exact) {
+    if (team)
+        return exact ? (const void*)&tsm::hausdorff_pruned_pairs_kernel<true, true>
+                     : (const void*)&tsm::hausdorff_pruned_pairs_kernel<true, false>;
+    return exact ? (const void*)&tsm::hausdorff_pruned_pairs_kernel<false, true>
+                 : (const void*)&tsm::hausdorff_pruned_pairs_kernel<false, false>;
 }
 
-const void* haus_pruned_matrix(int QB, bool exact) {
-    switch (QB) {
-        case 1:
-            return exact ? (const void*)&tsm::hausdorff_pruned_matrix_kernel<1, true>
-                         : (const void*)&tsm::hausdorff_pruned_matrix_kernel<1, false>;
-        case 4:
-            return exact ? (const void*)&tsm::hausdorff_pruned_matrix_kernel<4, true>
-                         : (const void*)&tsm::hausdorff_pruned_matrix_kernel<4, false>;
-        default: return nullptr;
-    }
+template <int QB>
+static const void* haus_pruned_matrix_of(bool longs, bool exact) {
+    if (longs)
+        return exact ? (const void*)&tsm::hausdorff_long_matrix_kernel<QB, true>
+                     : (const void*)&tsm::hausdorff_long_matrix_kernel<QB, false>;
+    return exact ? (const void*)&tsm::hausdorff_pruned_matrix_kernel<QB, true>
+                 : (const void*)&tsm::hausdorff_pruned_matrix_kernel<QB, false>;
+}
+
+const void* haus_pruned_matrix(int QB, bool longs, bool exact) {
+    return QB == 1 ? haus_pruned_matrix_of<1>(longs, exact) : haus_pruned_matrix_of<4>(longs, exact);
 }
 
 }  // namespace tsm_k

@@ -22,9 +22,10 @@ const void* bits_matrix(int measure);
 // hausdorff_matrix_kernel (matrix) or hausdorff_pairs_kernel, and hausdorff_wave_kernel <R, EXACT>
 const void* haus(bool matrix, int R, bool exact);
 const void* haus_wave(int R, bool exact);
-// hausdorff_pruned_matrix_kernel<QB, EXACT>, QB = 1 or 4, and hausdorff_pruned_pairs_kernel<EXACT>
-const void* haus_pruned_matrix(int QB, bool exact);
-const void* haus_pruned_pairs(bool exact);
+// hausdorff_pruned_matrix_kernel or (longs) hausdorff_long_matrix_kernel <QB, EXACT>, QB = 1 or 4, and
+// hausdorff_pruned_pairs_kernel<TEAM, EXACT>
+const void* haus_pruned_matrix(int QB, bool longs, bool exact);
+const void* haus_pruned_pairs(bool team, bool exact);
 // dp_sched_kernel<R, EXACT>
 const void* sched(int R, bool exact);
 
