@@ -29,7 +29,13 @@
 // their lanes instead of collected); 400 x 400 of 20..1000 points EDR 56 ->
 // 2.2; 200,000 EDR pairs of 20..200 points in any order 2.7 -> 0.29.  1000 x
 // 1000 of 20..200 points with everything within reach of everything, where no
-// test helps: EDR 3.71 -> 3.74, LCSS 3.35 -> 3.48.
+// test helps: EDR 3.71 -> 3.74, LCSS 3.35 -> 3.48 (600 x 600 1.68 -> 1.74 and
+// 1.51 -> 1.66, 200 x 200 0.46 -> 0.51 and 0.38 -> 0.48, where the launch is as long
+// as a lane's longest pairs; 1000 x 1000 of 2..20 points 0.095 -> 0.119 and 0.082 ->
+// 0.114).  Tried and slower: eight lanes per pair with four ballots a column (100 x
+// 100 as one warp per pair, 600 x 600 4.1 ms), loading a short word's rows only
+// (registers: 600 x 600 1.86), a second loop without tests for words near
+// everything, match masks by set instead of predicates (2.26).
 #pragma once
 
 #include "tsm_device.cuh"
@@ -73,10 +79,16 @@ __device__ __forceinline__ float4 warp_box(const float2* p, int n, int lane) {
                        ordered_float(__reduce_min_sync(0xffffffffu, ordered_int(b.z))),
                        ordered_float(__reduce_max_sync(0xffffffffu, ordered_int(b.w))));
 }
-// The boxes of the lanes' own trajectories (p, n; n <= 0: none), one after
-// the other by the whole warp (coalesced loads).  All 32 lanes call it.
+// The boxes of the lanes' own trajectories (p, n; n <= 0: none): one after the
+// other by the whole warp (coalesced loads, but a load's latency each) or, where
+// all are short, each by its lane.  All 32 lanes call it.
 __device__ __forceinline__ float4 lane_boxes(const float2* p, int n, int lane) {
     float4 mine = empty_box();
+    if (__reduce_max_sync(0xffffffffu, n) <= 32) {
+#pragma unroll 4
+        for (int i = 0; i < n; ++i) mine = box_add(mine, __ldg(p + i));
+        return mine;
+    }
     unsigned todo = __ballot_sync(0xffffffffu, n > 0);
     while (todo) {
         const int src = __ffs(todo) - 1;
@@ -245,16 +257,16 @@ struct BitsSmemCols {
 
 // Matrix kernel.  CTA (t, chunk) takes the queries q_order[QG t ..] (QG of
 // them, staged in shared memory with their boxes) and blockDim database slots,
-// one per thread, whose boxes it makes once for all QG queries.  The pairs
-// whose boxes are apart are written at once; the others are collected and then
-// taken 32 at a time, one per lane, or, when only a few are left over, one per
-// warp.  Query order, symmetric and gather modes as in dp_matrix_kernel
+// one per thread (FEW, for launches of few pairs: one per warp), whose boxes it
+// makes once for all QG queries.  The pairs whose boxes are apart are written at
+// once; the others are collected and then taken 32 at a time, one per lane, or,
+// when only a few are left over and always with FEW, one per warp.  Query order, symmetric and gather modes as in dp_matrix_kernel
 // (gather: QG = 1).  Dynamic shared memory = QG * q_cap float2 + (blockDim /
 // 32) * 32 * bits_words(q_cap) words.
 constexpr int kBitsQueries = 16;
 constexpr int kBitsThreads = 128;
 constexpr int kBitsWarpRest = 16;  // a rest of fewer pairs than this goes one per warp
-template <int M>
+template <int M, bool FEW>
 __global__ void __launch_bounds__(kBitsThreads) bits_matrix_kernel(
     const float2* __restrict__ q_pts, const int64_t* __restrict__ q_off, const int32_t* __restrict__ q_len,
     const int32_t* __restrict__ q_order, int64_t nq, const float2* __restrict__ d_pts,
@@ -273,8 +285,9 @@ __global__ void __launch_bounds__(kBitsThreads) bits_matrix_kernel(
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t* carry = reinterpret_cast<uint32_t*>(bits_smem + QG * q_cap) + warp * 32 * bits_words(q_cap);
     const int64_t qs0 = (int64_t)(blockIdx.x / chunks) * QG;
-    const int64_t s0 = (int64_t)(blockIdx.x % chunks) * kBitsThreads;
-    if (sym == 1 && s0 + kBitsThreads <= qs0) return;  // below the diagonal (uniform per CTA)
+    constexpr int kSlots = FEW ? kBitsThreads / 32 : kBitsThreads;
+    const int64_t s0 = (int64_t)(blockIdx.x % chunks) * kSlots;
+    if (sym == 1 && s0 + kSlots <= qs0) return;  // below the diagonal (uniform per CTA)
     const int ng = (int)min((int64_t)QG, nq - qs0);
     if (threadIdx.x == 0) n_todo = next = 0;
     for (int i = warp; i < ng; i += kBitsThreads / 32) {
@@ -292,7 +305,8 @@ __global__ void __launch_bounds__(kBitsThreads) bits_matrix_kernel(
         }
     }
     __syncthreads();
-    const int64_t slot = s0 + threadIdx.x;
+    auto slot_of = [&](int x) { return s0 + (FEW ? x >> 5 : x); };
+    const int64_t slot = FEW && lane > 0 ? nd : slot_of(threadIdx.x);  // (nd: none)
     int64_t dj = -1;
     int n = -1;
     const float2* dp = d_pts;
@@ -332,27 +346,27 @@ __global__ void __launch_bounds__(kBitsThreads) bits_matrix_kernel(
     }
     __syncthreads();
     const int all = n_todo;
-    const int full = (all + 32 - kBitsWarpRest) / 32;  // tasks of up to 32 pairs; the rest one by one
+    const int full = FEW ? 0 : (all + 32 - kBitsWarpRest) / 32;  // tasks of up to 32 pairs; the rest one by one
     const int tasks = full + max(0, all - 32 * full);
     for (;;) {
         int t = 0;
         if (lane == 0) t = atomicAdd(&next, 1);
         t = __shfl_sync(0xffffffffu, t, 0);
         if (t >= tasks) break;
-        if (t < full) {
+        if (!FEW && t < full) {
             const int k = 32 * t + lane;
             if (k < all) {
                 const int i = todo[k] / kBitsThreads, x = todo[k] % kBitsThreads;
                 const int c = bits_count<M>(d_ptr[x], d_n[x], BitsSmemCols{bits_smem + i * q_cap}, q_n[i], carry + lane,
                                             p.eps2, p.epsr, q_box[i]);
-                put(q_id[i], d_id[x], s0 + x, q_n[i], d_n[x], c);
+                put(q_id[i], d_id[x], slot_of(x), q_n[i], d_n[x], c);
             }
         } else {
             const int k = 32 * full + t - full;
             const int i = todo[k] / kBitsThreads, x = todo[k] % kBitsThreads;
             const int c = bits_count_warp<M>(d_ptr[x], d_n[x], bits_smem + i * q_cap, q_n[i], carry, p.eps2, p.epsr,
                                              q_box[i], lane);
-            if (lane == 0) put(q_id[i], d_id[x], s0 + x, q_n[i], d_n[x], c);
+            if (lane == 0) put(q_id[i], d_id[x], slot_of(x), q_n[i], d_n[x], c);
         }
         __syncwarp();
     }

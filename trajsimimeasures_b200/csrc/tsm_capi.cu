@@ -49,6 +49,10 @@ static_assert(tsm::kHeavyRows >= kTileCap, "a tile-heavy pair must have a side l
 // Matrix mode keeps the query as the tile kernel's columns: its boundary
 // rows (32 per warp) and staged columns must fit one CTA's shared memory.
 constexpr int kMatrixQueryMax = 1400;
+// EDR and LCSS matrices of at most kBitsFew pairs (kBitsFewShort where no trajectory is longer than kBitsShort)
+// take one warp per pair (see matrix_launch).
+constexpr int kBitsShort = 64;
+constexpr int64_t kBitsFew = 148 * 100, kBitsFewShort = 148 * 20;
 // Longest query of the matrix kernel with one lane per pair (see matrix_launch).
 constexpr int kMatrixLaneMax = 96;
 // Longest trajectory accepted by the paired kernels: the wave kernel keeps 4
@@ -425,17 +429,26 @@ int matrix_launch(const char* who, int measure, const float* q_pts, const int64_
         return fail(TSM_ETOOLONG, "%s: q_max_len %d > %d (use the pairs form)", who, q_max_len, kMatrixQueryMax);
     if (R != 4 && R != 8 && R != 16) return fail(TSM_EINVAL, "%s: rows_per_thread must be 4, 8 or 16", who);
     if (measure == TSM_EDR || measure == TSM_LCSS) {
+        // One warp per pair while there are so few pairs that one lane per pair would leave most of the GPU idle (and
+        // the launch as long as its longest pair by one lane).  Measured, every point near every other, one warp / one
+        // lane, us: EDR of 20..200 points 30 x 30 75 / 356, 100 x 100 219 / 346, 120 x 120 290 / 340, 160 x 160 465 /
+        // 374; LCSS 53 / 337, 143 / 326, 187 / 320, 434 / 370; 2..20 points, 50 x 50 26 / 27, 120 x 120 43 / 27; 40 x
+        // 40 of 1000..1400 points 3.6 / 13.7 ms.
+        const int threads = tsm::kBitsThreads, carry_bytes = threads * tsm::bits_words(qcap) * 4;
+        const int64_t pairs = sym == 1 ? nq * (nq + 1) / 2 : nq * nd;
+        const bool few = pairs <= (std::max(qcap, (int)d_max_len) <= kBitsShort ? kBitsFewShort : kBitsFew);
+        const int slots = few ? threads / 32 : threads;
+        int chunks = (int)((nd + slots - 1) / slots);
         // queries per CTA: as many as share the database boxes within half an SM's shared memory, fewer when
         // that leaves SMs without a few CTAs each
-        const int threads = tsm::kBitsThreads, carry_bytes = threads * tsm::bits_words(qcap) * 4;
-        int chunks = (int)((nd + threads - 1) / threads);
-        int qg = sym == 2 ? 1 : tsm::kBitsQueries;
+        int qg = sym == 2 || few ? 1 : tsm::kBitsQueries;
         while (qg > 1 && (qg * qcap * 8 + carry_bytes > kSmemPerCta || (nq + qg - 1) / qg * chunks < 148 * 8)) qg >>= 1;
         const int64_t ctas = (nq + qg - 1) / qg * chunks;
         if (ctas > 0x7fffffffLL) return fail(TSM_EINVAL, "%s: grid too large", who);
         void* args[] = {&q2,   &q_off,  &q_len, &q_order, &nq,   &d2,  &d_off,      &d_len, &d_order, &ndd,
                         &dtot, &chunks, &qg,    &sym,     &qcap, &dml, (void*)&kp, &out,   &ld,      &out_counts};
-        return launch(tsm_k::bits_matrix(measure), dim3((unsigned)ctas), dim3(threads), qg * qcap * 8 + carry_bytes, args, s);
+        return launch(tsm_k::bits_matrix(measure, few), dim3((unsigned)ctas), dim3(threads), qg * qcap * 8 + carry_bytes,
+                      args, s);
     }
     const void* fn = tsm_k::dp_matrix(measure, R, exact);
     // Two lanes per pair; one lane per pair where the query is short.  Measured, 2000 x 2000 random walks, two / one,

@@ -16,8 +16,12 @@ const void* dp_matrix(int measure, int R, bool exact) {
     TSM_DP_MATRIX_TABLE(tsm::dp_matrix_kernel, true, measure, R)
 }
 
-const void* bits_matrix(int measure) {
-    return measure == TSM_EDR ? (const void*)&tsm::bits_matrix_kernel<tsm::EDR> : (const void*)&tsm::bits_matrix_kernel<tsm::LCSS>;
+const void* bits_matrix(int measure, bool few) {
+    if (few)
+        return measure == TSM_EDR ? (const void*)&tsm::bits_matrix_kernel<tsm::EDR, true>
+                                  : (const void*)&tsm::bits_matrix_kernel<tsm::LCSS, true>;
+    return measure == TSM_EDR ? (const void*)&tsm::bits_matrix_kernel<tsm::EDR, false>
+                              : (const void*)&tsm::bits_matrix_kernel<tsm::LCSS, false>;
 }
 
 }  // namespace tsm_k

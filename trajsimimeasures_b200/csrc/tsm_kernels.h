@@ -17,8 +17,8 @@ const void* dp_wave(int measure, int R, bool exact);
 // dp_matrix_lane_kernel<M, 8, EXACT>, M = TSM_DTW or TSM_DFRECHET
 const void* dp_matrix_lane(int measure, bool exact);
 const void* dp_matrix_lane_fast(int measure);
-// bits_matrix_kernel<M>, M = TSM_EDR or TSM_LCSS
-const void* bits_matrix(int measure);
+// bits_matrix_kernel<M, FEW>, M = TSM_EDR or TSM_LCSS
+const void* bits_matrix(int measure, bool few);
 // hausdorff_matrix_kernel (matrix) or hausdorff_pairs_kernel, and hausdorff_wave_kernel <R, EXACT>
 const void* haus(bool matrix, int R, bool exact);
 const void* haus_wave(int R, bool exact);
