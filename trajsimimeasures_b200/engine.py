@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import math
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -368,23 +369,33 @@ def pair_order_dev(len_a: torch.Tensor, len_b: torch.Tensor, rows=DEFAULT_ROWS, 
     the largest first.  Lengths on the CPU: pair_order's order for `rows`."""
     if not len_a.is_cuda:
         return torch.from_numpy(pair_order(len_a.numpy(), len_b.numpy(), rows))
+    if stream is not None:
+        return on_stream(stream, (len_a, len_b), lambda: (pair_order_dev(len_a, len_b, rows),))[0]
+    la, lb = len_a.to(torch.int32).contiguous(), len_b.to(torch.int32).contiguous()
+    n = int(la.shape[0])
+    lib = _lib.load()
+    order = torch.empty(n, dtype=torch.int32, device=la.device)
+    ws = torch.empty(lib.tsm_pair_order_workspace_bytes() // 4, dtype=torch.int32, device=la.device)
+    _lib.check(lib.tsm_pair_order(_ptr(la), _ptr(lb), n, _ptr(order), _ptr(ws), _stream_ptr(None)), "tsm_pair_order")
+    return order
 
-    def work():
-        la, lb = len_a.to(torch.int32).contiguous(), len_b.to(torch.int32).contiguous()
-        n = int(la.shape[0])
-        lib = _lib.load()
-        order = torch.empty(n, dtype=torch.int32, device=la.device)
-        ws = torch.empty(lib.tsm_pair_order_workspace_bytes() // 4, dtype=torch.int32, device=la.device)
-        _lib.check(lib.tsm_pair_order(_ptr(la), _ptr(lb), n, _ptr(order), _ptr(ws), _stream_ptr(None)), "tsm_pair_order")
-        return (order,)
-    return on_stream(stream, (len_a, len_b), work)[0]
+
+# A batch without an order is sorted by loop shape from (pairs per SM, cells) on,
+# cells counted as pairs times the square of the set's longest trajectory.  With fewer
+# pairs a launch lasts as long as its longest pair whatever the order; with fewer
+# cells the sort (25 us) costs more than it saves.  Measured without / with it, us:
+# DTW of 20..200 points 29,601 pairs 508 / 477, 100,000 1,487 / 742, of 2..64
+# points 29,601 107 / 114, 40,000 127 / 118, of 2..20 200,000 82 / 94; Frechet of
+# 20..200 29,601 450 / 482, of 2..64 40,000 109 / 114, 60,000 129 / 118; ERP of 2..64
+# 40,000 148 / 134; Hausdorff 261 / 220.  (All of one length, 200 points: 40,000 DTW
+# pairs 909 / 935.)  EDR and LCSS never: 200,000 pairs 0.29 / 0.27 ms, less than the
+# sort takes.
+ORDER_FROM = {_lib.DTW: (200, 1.5e8), _lib.ERP: (200, 1.5e8), _lib.DFRECHET: (250, 2e8), _lib.HAUSDORFF: (200, 1.5e8)}
 
 
-# Pairs per SM from which a batch without an order is worth sorting by loop
-# shape: below, a launch lasts as long as its longest pair whatever the order
-# (12,000 DTW pairs of 20..200 points 450 us unsorted, 496 with the sort; 30,000
-# 578 and 561; 100,000 1,487 and 742).
-ORDER_PAIRS_PER_SM = 200
+def _worth_sorting(m, n, max_len, device) -> bool:
+    per_sm, cells = ORDER_FROM.get(m, (0, math.inf))
+    return n * max_len * max_len >= cells and n > per_sm * _sm_count(device)
 
 
 @functools.lru_cache(maxsize=None)
@@ -434,7 +445,14 @@ def matrix(measure, q: TrajSet, d: TrajSet, *, eps=0.0, gpoint=(0.0, 0.0), exact
     return out, counts
 
 
-def _pairs_in_set(m, s, idx_a, idx_b, order, with_counts, **kw):
+def pairs_in_set(measure, s: TrajSet, idx_a, idx_b, *, eps=0.0, gpoint=(0.0, 0.0), exact=False, rows=0,
+                 stream=None, order=None, with_counts=None):
+    """Pairs (idx_a[k], idx_b[k]) of one device set -> (out float32 [n], counts)."""
+    if stream is not None:  # (an order formed while the lengths still change would not be a permutation)
+        return on_stream(stream, (idx_a, idx_b, order, s.pts, s.off, s.lens), lambda: pairs_in_set(
+            measure, s, idx_a, idx_b, eps=eps, gpoint=gpoint, exact=exact, rows=rows, order=order,
+            with_counts=with_counts))
+    m = measure_id(measure)
     ia = torch.as_tensor(idx_a, device=s.device).long()
     ib = torch.as_tensor(idx_b, device=s.device).long()
     off_a, len_a = s.off[ia], s.lens[ia]
@@ -443,19 +461,8 @@ def _pairs_in_set(m, s, idx_a, idx_b, order, with_counts, **kw):
     out = torch.empty(n, dtype=torch.float32, device=s.device)
     want = (m in (_lib.EDR, _lib.LCSS)) if with_counts is None else with_counts
     counts = torch.empty(n, dtype=torch.int32, device=s.device) if want else None
-    if order is None and m not in (_lib.EDR, _lib.LCSS) and \
-            n > ORDER_PAIRS_PER_SM * _sm_count(s.device):
-        # lanes of a warp that take unequal pairs wait for the longest (EDR and LCSS: 0.29 -> 0.27 ms for 200,000 pairs,
-        # less than the sort takes)
-        order = pair_order_dev(len_a, len_b)
-    pairs_raw(m, s.pts, off_a, len_a, off_b, len_b, s.max_len, out=out, counts=counts, order=order, **kw)
+    if order is None and _worth_sorting(m, n, s.max_len, s.device):
+        order = pair_order_dev(len_a, len_b)  # lanes of a warp that take unequal pairs wait for the longest
+    pairs_raw(m, s.pts, off_a, len_a, off_b, len_b, s.max_len, out=out, counts=counts, order=order,
+              eps=eps, gpoint=shift_gpoint(gpoint, s.origin), exact=exact, rows=rows)
     return out, counts
-
-
-def pairs_in_set(measure, s: TrajSet, idx_a, idx_b, *, eps=0.0, gpoint=(0.0, 0.0), exact=False, rows=0,
-                 stream=None, order=None, with_counts=None):
-    """Pairs (idx_a[k], idx_b[k]) of one device set -> (out float32 [n], counts)."""
-    # (on_stream: an order formed while the lengths still change would not be a permutation)
-    return on_stream(stream, (idx_a, idx_b, order, s.pts, s.off, s.lens), lambda: _pairs_in_set(
-        measure_id(measure), s, idx_a, idx_b, order, with_counts, eps=eps, gpoint=shift_gpoint(gpoint, s.origin),
-        exact=exact, rows=rows))
