@@ -247,10 +247,13 @@ __device__ __forceinline__ float dp_pair(const float2* __restrict__ rowp, int nr
 //
 // Measured on B200, all-pairs 2000 x 2000 of 20..200 points, ms, against one
 // lane per pair (two, for ERP four, blocks of 8 rows a lane), same bits: DTW 15.2
-// -> 13.9, ERP 18.1 -> 17.1, Frechet 12.3 -> 11.6.  R = 16: 14.0, 17.3 (3 CTAs'
-// registers; 18.3 and 20.7 in 168 and 128), 11.5; R = 4: 16.9, 19.7, 14.1.  The
+// -> 13.9, ERP 18.1 -> 17.1, Frechet 12.3 -> 11.6; R = 4: 16.9, 19.7, 14.1.  The
 // launch bound of 4 CTAs gives ptxas the registers that the shared memory allows
-// (without it DTW 14.1, ERP 19.9; with 6 CTAs 16.6, 20.0, 12.6).  Tried on one
+// (without it DTW 14.1, ERP 19.9; with 6 CTAs 16.6, 20.0, 12.6).  R = 16 has none
+// (with 4 ERP spills): 1000 x 1000 DTW 3.81 ms, ERP 4.69, Frechet 3.14 (4.22, 5.71,
+// 3.33 with it; one lane per pair 4.22, 5.23, 3.49).  Scalar instead of f32x2
+// differences, 2 % faster for Frechet with one lane per pair: 3.39 for 3.17 with two.
+// Tried on one
 // lane per pair, slower, same bits: the square roots one column ahead of the
 // recurrence (DTW 15.2 -> 16.0, ERP 18.1 -> 19.8), the lower block first (25 %),
 // the squared distances of two rows packed in f32x2 (19.0, 20.5, Frechet 15.6:
@@ -434,7 +437,7 @@ __global__ void __launch_bounds__(128) dp_pairs_kernel(
 // Dynamic shared memory = cap + 3 float4 columns + W * duo_ring(cap) floats.
 
 template <int M, int R, bool EXACT>
-__global__ void __launch_bounds__(128, 4) dp_matrix_kernel(
+__global__ void __launch_bounds__(128, R == 16 ? 1 : 4) dp_matrix_kernel(
     const float2* __restrict__ q_pts, const int64_t* __restrict__ q_off, const int32_t* __restrict__ q_len,
     const int32_t* __restrict__ q_order, const float2* __restrict__ d_pts, const int64_t* __restrict__ d_off,
     const int32_t* __restrict__ d_len, const int32_t* __restrict__ d_order, int64_t nd, int64_t d_total, int chunks,
