@@ -232,18 +232,22 @@ int tsm_pairs_sched_noalloc(const float* pts, const int64_t* off_a, const int32_
 /* Packs a batch of padded HOST arrays for tsm_pairs (the stacking and upload of
  * core/dtw.py:61-72): the len1[k] valid points of trajectory k of t1, then those
  * of t2, to pts (float32 x, y) back to back; off_a / off_b / len_a / len_b as
- * tsm_pairs takes them.  t1 / t2: float64 (is_f64) or float32, coordinates of a
+ * tsm_pairs takes them.  t1 / t2: of one type (TSM_F32 ..), coordinates of a
  * point adjacent, byte strides between trajectories and points.  origin_mode:
  * TSM_ORIGIN_NONE rounds to float32; TSM_ORIGIN_PER_PAIR first subtracts, in
  * FP64, the pair's first point (of t1, else t2, rounded to float32; 0 when not
  * finite); TSM_ORIGIN_ONE subtracts origin[2].  max_points: capacity of pts (the
  * sum of the lengths).  All pointers are HOST memory; no CUDA call.  May use
  * threads of its own, joined before it returns. */
+#define TSM_F32 0
+#define TSM_F64 1
+#define TSM_I32 2
+#define TSM_I64 3
 #define TSM_ORIGIN_NONE 0
 #define TSM_ORIGIN_PER_PAIR 1
 #define TSM_ORIGIN_ONE 2
 int tsm_pack_pairs(const void* t1, int64_t traj_stride1, int64_t pt_stride1, const int64_t* len1, const void* t2,
-                   int64_t traj_stride2, int64_t pt_stride2, const int64_t* len2, int64_t n, int32_t is_f64,
+                   int64_t traj_stride2, int64_t pt_stride2, const int64_t* len2, int64_t n, int32_t type,
                    int32_t origin_mode, const double* origin, int64_t* off_a, int64_t* off_b, int32_t* len_a,
                    int32_t* len_b, float* pts, int64_t max_points);
 /* Processing order for tsm_pairs: order[0 .. n_pairs - 1] = the pair indices,

@@ -187,10 +187,13 @@ def release_staging():
     _tls.pinned = None
 
 
+_PACK_TYPES = {np.dtype(np.float32): 0, np.dtype(np.float64): 1, np.dtype(np.int32): 2, np.dtype(np.int64): 3}
+
+
 def _packable(a):
-    """Whether tsm_pack_pairs reads the array as it is: float64 or float32 in
+    """Whether tsm_pack_pairs reads the array as it is: of one of its types, in
     native byte order, aligned, the two coordinates of a point adjacent."""
-    return a.dtype in (np.dtype(np.float64), np.dtype(np.float32)) and a.flags.aligned and a.strides[2] == a.itemsize
+    return a.dtype in _PACK_TYPES and a.flags.aligned and a.strides[2] == a.itemsize
 
 
 def _stage_padded(a1, a2, la, lb, order, dev, origin=None):
@@ -216,7 +219,7 @@ def _stage_padded(a1, a2, la, lb, order, dev, origin=None):
     o = None if own or origin is None else np.ascontiguousarray(origin, dtype=np.float64)
     l1, l2 = np.ascontiguousarray(la, dtype=np.int64), np.ascontiguousarray(lb, dtype=np.int64)
     rc = _lib.load().tsm_pack_pairs(a1.ctypes.data, a1.strides[0], a1.strides[1], l1.ctypes.data, a2.ctypes.data,
-                                    a2.strides[0], a2.strides[1], l2.ctypes.data, n, int(a1.dtype == np.float64),
+                                    a2.strides[0], a2.strides[1], l2.ctypes.data, n, _PACK_TYPES[a1.dtype],
                                     1 if own else 0 if o is None else 2, None if o is None else o.ctypes.data,
                                     off.ctypes.data, off[n:].ctypes.data, ints.ctypes.data, ints[n:].ctypes.data,
                                     host.ctypes.data + pts_at, P)

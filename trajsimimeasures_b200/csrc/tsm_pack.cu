@@ -7,6 +7,8 @@
 // GB/s, for 20,000 pairs).  Measured on the host of a B200, pairs of 20..200
 // float64 points padded to 200: 512 of them 197 us as one array operation over
 // the padded width per side, 113 us here; 64 of them 8 us.
+#include <emmintrin.h>
+
 #include <cmath>
 #include <cstring>
 #include <thread>
@@ -46,6 +48,14 @@ void pack_rows(const Side& s, int64_t k0, int64_t k1, const double* origin, bool
             continue;
         }
         const double ox = origin[per_pair ? 2 * k : 0], oy = origin[per_pair ? 2 * k + 1 : 1];
+        if (std::is_same<T, double>::value) {  // a point's two coordinates at a time, whatever lies between points
+            const __m128d o2 = _mm_set_pd(oy, ox);
+            for (int64_t i = 0; i < n; ++i) {
+                const __m128d v = _mm_loadu_pd(reinterpret_cast<const double*>(p + i * s.pt));
+                _mm_storel_pi(reinterpret_cast<__m64*>(d + 2 * i), _mm_cvtpd_ps(_mm_sub_pd(v, o2)));
+            }
+            continue;
+        }
         if (s.pt == 2 * (int64_t)sizeof(T)) {  // contiguous points
             const T* q = reinterpret_cast<const T*>(p);
             for (int64_t i = 0; i < n; ++i) {
@@ -65,8 +75,8 @@ void pack_rows(const Side& s, int64_t k0, int64_t k1, const double* origin, bool
 template <class T>
 void first_point(const Side& s, int64_t k, double* o) {
     const T* q = reinterpret_cast<const T*>(s.base + k * s.traj);
-    o[0] = (double)(float)q[0];
-    o[1] = (double)(float)q[1];
+    o[0] = (double)(float)(double)q[0];
+    o[1] = (double)(float)(double)q[1];
 }
 
 template <class T>
@@ -93,8 +103,13 @@ void pack_all(const Side& a, const Side& b, int64_t n, int mode, const double* o
     // 262,144 / of 524,288 / of 98,304 points (float64 pairs of 20..200): 1,000
     // pairs 0.49 ms / - / - / 0.54, 4,096 (0.9 million points) 1.34 / 1.20 / - /
     // 1.54 (float32 1.11 / 1.21 / - / 1.74), 6,000 (float32) 1.55 / 1.87 / 1.48,
-    // 20,000 12.5 / 5.1 / 5.0.
-    int64_t nt = total / 524288;
+    // 20,000 12.5 / 5.1 / 5.0.  Points that are not back to back (a slice of wider
+    // rows) are bound by one core's loads sooner: 40 bytes apart, 1,500 pairs 0.83 ms
+    // in one thread, 0.73 in threads of 131,072, 4,096 1.96 / 1.31.  (Array operations
+    // over the padded width, in a pool that is always there: 0.62 and 1.32; 1,000
+    // pairs 0.50, here in one thread 0.62.)
+    const bool dense = a.pt == 2 * (int64_t)sizeof(T) && b.pt == a.pt;
+    int64_t nt = total / (dense ? 524288 : 131072);
     const int64_t hw = (int64_t)std::thread::hardware_concurrency();
     if (nt > 8) nt = 8;
     if (nt > hw) nt = hw;
@@ -119,7 +134,7 @@ void pack_all(const Side& a, const Side& b, int64_t n, int mode, const double* o
 extern "C" {
 
 int tsm_pack_pairs(const void* t1, int64_t traj_stride1, int64_t pt_stride1, const int64_t* len1, const void* t2,
-                   int64_t traj_stride2, int64_t pt_stride2, const int64_t* len2, int64_t n, int32_t is_f64,
+                   int64_t traj_stride2, int64_t pt_stride2, const int64_t* len2, int64_t n, int32_t type,
                    int32_t origin_mode, const double* origin, int64_t* off_a, int64_t* off_b, int32_t* len_a,
                    int32_t* len_b, float* pts, int64_t max_points) {
     if (n < 0) return tsm_internal_fail(TSM_EINVAL, "tsm_pack_pairs: n < 0");
@@ -128,6 +143,7 @@ int tsm_pack_pairs(const void* t1, int64_t traj_stride1, int64_t pt_stride1, con
         return tsm_internal_fail(TSM_EINVAL, "tsm_pack_pairs: null pointer");
     if (origin_mode < TSM_ORIGIN_NONE || origin_mode > TSM_ORIGIN_ONE || (origin_mode == TSM_ORIGIN_ONE && !origin))
         return tsm_internal_fail(TSM_EINVAL, "tsm_pack_pairs: bad origin");
+    if (type < TSM_F32 || type > TSM_I64) return tsm_internal_fail(TSM_EINVAL, "tsm_pack_pairs: unknown type");
     try {
         int64_t at = 0;
         for (int side = 0; side < 2; ++side) {
@@ -144,8 +160,12 @@ int tsm_pack_pairs(const void* t1, int64_t traj_stride1, int64_t pt_stride1, con
         }
         const Side a{static_cast<const unsigned char*>(t1), traj_stride1, pt_stride1, len1, off_a, len_a};
         const Side b{static_cast<const unsigned char*>(t2), traj_stride2, pt_stride2, len2, off_b, len_b};
-        if (is_f64) pack_all<double>(a, b, n, origin_mode, origin, pts, at);
-        else pack_all<float>(a, b, n, origin_mode, origin, pts, at);
+        switch (type) {
+            case TSM_F32: pack_all<float>(a, b, n, origin_mode, origin, pts, at); break;
+            case TSM_F64: pack_all<double>(a, b, n, origin_mode, origin, pts, at); break;
+            case TSM_I32: pack_all<int32_t>(a, b, n, origin_mode, origin, pts, at); break;
+            default: pack_all<int64_t>(a, b, n, origin_mode, origin, pts, at);
+        }
     } catch (...) {
         return tsm_internal_fail(TSM_EINVAL, "tsm_pack_pairs: out of memory");
     }
