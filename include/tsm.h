@@ -102,8 +102,7 @@ int32_t tsm_matrix_query_max(void);
  *   out     float32 [n_pairs]
  *   out_counts int32 [n_pairs] or NULL: EDR/LCSS edit/match counts before
  *           normalisation (ignored for other measures)
- * When max_len exceeds 256 (Hausdorff: when max_len^2 exceeds 2^17), the
- * long pairs' kernel runs on a stream of the
+ * When max_len exceeds 256, the long pairs' kernels run on a stream of the
  * calling thread forked from `stream` (an event record / wait on each side;
  * the side stream and its two events are created once per thread and
  * device).  `stream` waits for it before the call returns, so later work on
@@ -252,7 +251,8 @@ int tsm_pack_pairs(const void* t1, int64_t traj_stride1, int64_t pt_stride1, con
                    int32_t* len_b, float* pts, int64_t max_points);
 /* Processing order for tsm_pairs: order[0 .. n_pairs - 1] = the pair indices,
  * grouped by the shape of their DP (steps of 8 points on both sides up to 256,
- * of an eighth of an octave above), the largest first; inside a group in any order.
+ * of an eighth of an octave above, lengths from 3,584 in one), the largest first;
+ * inside a group in any order.
  * The reference processes a batch in its given order (core/dtw.py:69-72);
  * results do not depend on it.  len_a / len_b int32 [n_pairs] (any values),
  * order int32 [n_pairs], workspace tsm_pair_order_workspace_bytes() bytes, all

@@ -62,9 +62,11 @@ __device__ __forceinline__ float d2f(float ax, float ay, float bx, float by) {
 // difference c + nr = -(r - c) is exactly the negated scalar difference
 // (round-to-nearest is symmetric) and the squares do not see the sign, so
 // the value is bit-identical to d2f(r.x, r.y, c.x, c.y).  The difference is
-// one f32x2 add: it costs what two scalar adds do but one instruction less, and
-// measured (same inputs, same outputs) 5-15 % faster in the paired kernels, and
-// 4 to 6 % in the matrix kernels.
+// one f32x2 add: it costs what two scalar adds do but one instruction less.
+// Measured (same inputs, same outputs), scalar / f32x2: matrices of 1000 x 1000,
+// 20..200 points, DTW 3.92 / 3.80 ms, ERP 4.90 / 4.67, Frechet 3.39 / 3.18, EDR with
+// all near (600 x 600) 1.83 / 1.75; 200,000 sorted pairs DTW 0.95 / 0.95, ERP 1.18 /
+// 1.15, but Frechet 0.80 / 0.87.
 __device__ __forceinline__ float d2nr(float2 nr, float2 c) {
     const float2 d = __fadd2_rn(nr, c);
     return __fmaf_rn(d.y, d.y, __fmul_rn(d.x, d.x));

@@ -252,7 +252,7 @@ __global__ void enc_adam(float* __restrict__ p, const float* __restrict__ g, flo
 // and 32 of a half's 64 units, with the biases in FP32, h in FP32 registers and
 // written back to shared memory as BF16.  The a_t part comes from
 // enc_conv_fwd_tc as one 16 KB BF16 image per step already in the operand
-// layout, bulk-copied two buffers ahead.  a_t and h_t enter the products as BF16
+// layout, bulk-copied a step ahead into the other of two buffers.  a_t and h_t enter the products as BF16
 // (the training kernels multiply FP32 a and h by the BF16 weights) and the
 // gates use the hardware tanh, so the embeddings agree with the training
 // forward to BF16 rounding of the activations.
@@ -872,8 +872,8 @@ int tsm_enc_train_status(void* workspace, int32_t* status, void* stream) {
     if (*status == 0) return TSM_OK;
     if ((rc = enc_check(cudaMemset(workspace, 0, 4), "tsm_enc_train_status: clear"))) return rc;
     char b[256];
-    snprintf(b, sizeof(b), "tsm_enc_loss_grad: a tensor-core wait ran out (status %d%s); "
-             "the gradients of the calls since the last check are incomplete", *status,
+    snprintf(b, sizeof(b), "training kernels: a tensor-core or copy wait ran out (status %d%s); "
+             "results of the tsm_enc_loss_grad and tsm_enc_forward calls since the last check are incomplete", *status,
              (*status & 128) ? ": tensor memory not freed, reset the device" : "");
     return tsm_internal_fail(TSM_ETIMEOUT, b);
 }

@@ -2,8 +2,8 @@
 // pairs by the shape of their DP (rows = the longer side, columns = the
 // shorter), the largest first, so that the lanes of a warp run loops of
 // near-equal length.  64 classes a side: steps of 8 points up to 256, then
-// eighths of an octave up to 4,096 (longer ones share the last); pairs of a
-// class in any order.
+// eighths of an octave (lengths from 3,584 share the last); pairs of a class in
+// any order.
 //
 // Bound by launches and by the latency of its atomics, not by its 12 bytes a
 // pair.  A call with 100,000 pairs of 20..200 points and this order takes 742 us

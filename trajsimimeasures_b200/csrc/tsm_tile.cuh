@@ -424,8 +424,9 @@ __global__ void __launch_bounds__(128) dp_pairs_kernel(
 }
 
 // Matrix mode -----------------------------------------------------------------
-// grid.x = nq * chunks; CTA (s, chunk) computes out[i, d_order[chunk*blockDim + t]]
-// for the query i = q_order[s] (i = s without an order).
+// grid.x = nq * chunks; CTA (s, chunk) computes out[i, d_order[chunk * S + t]], t <
+// S = blockDim / 2 (two lanes a slot; dp_matrix_lane_kernel: blockDim), for the
+// query i = q_order[s] (i = s without an order).
 // Symmetric mode (sym == 1; the query set is the database set and q_order ==
 // d_order): only the slots at or after the query's own sorted position s are
 // computed (the upper triangle in sorted order), and each value is written to
@@ -756,7 +757,7 @@ __global__ void __launch_bounds__(128) hausdorff_matrix_kernel(
 }
 
 // Pairs mode: a pair with more than kHausWarpCells point products (na * nb)
-// runs one warp per pair (hausdorff_pruned_pairs_kernel, or above
+// runs one warp or one CTA per pair (hausdorff_pruned_pairs_kernel, or above
 // kHausPrunedMax points hausdorff_wave_kernel): below that line one thread
 // per pair costs less than staging a pair (see matrix_launch for both sides).
 constexpr int64_t kHausWarpCells = 2048;

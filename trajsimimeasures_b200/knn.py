@@ -127,9 +127,9 @@ def _knn_rerank(Q, D, cand, k, m, eps, gpoint, exact, gather_lpt):
 
 
 def shape_order(len_a: torch.Tensor, len_b: torch.Tensor, rows=DEFAULT_ROWS, stream=None) -> torch.Tensor:
-    """engine.pair_order on the device: the pairs ordered by (row blocks,
-    columns) of their DP, the largest first, so a warp's 32 lanes run loops of
-    equal trip counts (int32 processing order for tsm_pairs)."""
+    """engine.pair_order_dev: an int32 processing order for tsm_pairs by classes of
+    loop shapes, the largest first, so that a warp's 32 lanes run loops of
+    near-equal trip counts (lengths on the CPU: engine.pair_order's for `rows`)."""
     return pair_order_dev(len_a, len_b, rows, stream)
 
 

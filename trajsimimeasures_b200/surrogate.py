@@ -136,8 +136,8 @@ class Encoder:
 
     def check_training(self, stream=None):
         """Raises TsmError if a bounded wait of a training kernel ran out in a
-        loss_grad call since the last check (the gradients of those calls are
-        incomplete).  Synchronises the stream; fit() calls
+        loss_grad call or an embed call without tensor_cores since the last check
+        (their results are incomplete).  Synchronises the stream; fit() calls
         it once per epoch."""
         if self._ws is None:
             return
