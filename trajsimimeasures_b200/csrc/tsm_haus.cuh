@@ -31,8 +31,8 @@
 // where 8 need 16, and 16 evaluate 6.7 blocks of twice the size.  Measured on
 // B200, unpruned -> pruned, bit for bit the same: 2000 x 2000 of 20..200
 // points 39.9 -> 9.1 ms, 1200 x 1500 18.5 -> 4.2 ms, 600 x 600 of 20..700
-// points 55.3 -> 5.8 ms; 200,000 pairs of 20..200 points 6.7 -> 1.1 ms, 50,000
-// lognormal pairs (10..2000 points) 8.8 -> 0.64 ms.  64 registers (32 warps
+// points 55.3 -> 6.2 ms; 200,000 pairs of 20..200 points 6.7 -> 0.94 ms, 50,000
+// lognormal pairs (10..2000 points) 8.8 -> 0.59 ms.  64 registers (32 warps
 // per SM); 48 (40 warps) spill: 10.9 ms for the first case.  Finishing a group
 // with one lane per segment once few of its points count was slower (12.0), and
 // so was leaving out a group's tests after three that skipped nothing (2.46 ->
@@ -42,7 +42,10 @@
 // so that 8 to 24 warps work on an SM whatever the lengths; its warps take the
 // groups side by side and share the maximum, which skips a little less than one
 // warp after the other (1.00 ms for 200 x 200 of 300..500 points by CTAs, 0.68 by
-// warps, which still fit 16 times there).
+// warps, which still fit 16 times there).  From 256 points on (320, 384, 512): 600 x
+// 600 of 20..700 points 6.3 ms (6.1, 7.2, 6.2; 5.7 by eight warps an SM), 1,000 of
+// 20..200 and one of 1,000 3.2 (4.1, 4.1, 4.1; 7.2), 100 x 100 of 800..1000 0.48
+// (0.60, 0.60, 0.60; 0.90).
 #pragma once
 
 #include <type_traits>

@@ -21,14 +21,14 @@
 // Blocks take trajectories of similar length (a counting sort by length), so
 // few of a block's 16 rows idle, and time steps are stored compactly.
 //
-// What bounds it: the chain of steps.  A forward step (1.55 us) is 24 MMAs (M =
+// What bounds it: the chain of steps.  A forward step (1.75 us) is 24 MMAs (M =
 // 128, N = 48, K = 16, about 40 cycles each) on the previous step's result, a
-// commit, the tensor-memory loads (370 cycles), the gate math (900) and the
+// commit, the tensor-memory loads (370 cycles), the gate math (1,300) and the
 // operand stores (110); the input products of the next step run under the gate
 // math.  A backward step (1.7 us) has 24 MMAs on the chain and 24 (dA) beside it.
 // 48 KB leave and 40 KB enter the SM a step, all by bulk copies off the chain.
-// Measured, 1,024 pairs of 20..200 points (128 blocks): forward 309 us, backward
-// 347 us.  With the weights in shared memory (64 cycles an MMA: bound by reading
+// Measured, 1,024 pairs of 20..200 points (128 blocks): forward 350 us, backward
+// 350 us.  With the weights in shared memory (64 cycles an MMA: bound by reading
 // A; 128 for the 64-row dA), eight values a thread and every value stored and
 // loaded by the epilogue: about 560 us each.
 #include <cstdio>
