@@ -18,10 +18,10 @@
 // the bounds are compared with a margin delta above the rounding error of an
 // evaluation.  With M the extent of the two trajectories' common bounding box
 // and u = 2^-24, an evaluated foot offset differs from the offset to a point
-// of the segment by at most 3 u M per coordinate; delta = 2^-19 M + 2^-62 is 7
-// times the resulting length, plus what underflow can take: the approximate
+// of the segment by at most 3 u M per coordinate; delta = max(2^-19 M, 2^-62) is 7
+// times the resulting length, and twice what underflow can take: the approximate
 // square root of a bound flushes squared distances below 2^-126 (lengths below
-// 2^-63) to 0, and a widened bound stays a normal number (2^-124 at least).
+// 2^-63) to 0.  A widened bound stays a normal number (2^-124 at least).
 // Non-finite coordinates set delta to infinity, which turns every skip off.
 //
 // What bounds it: issue, and the latency of its warp votes and reductions.  On
@@ -277,7 +277,7 @@ __device__ __forceinline__ float haus_directed(const HausTraj& P, const HausTraj
 template <bool TEAM>
 __device__ __forceinline__ float haus_pair(const HausTraj& a, const HausTraj& b, int lane, int* shared) {
     const float w = fmaxf(a.bb.y, b.bb.y) - fminf(a.bb.x, b.bb.x), h = fmaxf(a.bb.w, b.bb.w) - fminf(a.bb.z, b.bb.z);
-    const float delta = fmaf(0x1p-19f, w + h, 0x1p-62f);
+    const float delta = fmaxf(0x1p-19f * (w + h), 0x1p-62f);
     const float m = haus_directed<TEAM>(a, b, 0.f, delta, lane, shared);
     return haus_directed<TEAM>(b, a, m, delta, lane, shared);
 }
